@@ -62,6 +62,7 @@ struct ColonyDev {
   const int32_t *nn;
   const int16_t *nn16;  // n x 32 candidate ids (-1 padded) when k <= 32, else null
   const float *eta_nn;
+  int32_t *prior_set;  // non-zero: eta_nn carries a learned prior (differs from eta's entries)
   float *tau_nn;
   float *choice_nn;
   int32_t *tours;

@@ -37,6 +37,9 @@ cudaError_t launch_gather_nn_f32(const float *src, int n, int ld, const int32_t 
 cudaError_t launch_greedy_tau0(const ColonyDev &c, int tau0_mode, float tau0_value,
                                cudaStream_t s);
 cudaError_t launch_init_colony(const ColonyDev &c, cudaStream_t s);
+// Sets *c.prior_set to whether the candidate heuristic differs from the
+// gathered plain heuristic (a learned prior is installed).
+cudaError_t launch_prior_set(const ColonyDev &c, cudaStream_t s);
 
 // ---- iteration ----
 size_t construct_smem_bytes(int n, int K, int ants_per_block);
@@ -86,47 +89,17 @@ cudaError_t launch_construct_direct(const ColonyDev &c, int grid, int warps, cud
 cudaError_t query_construct_cluster(const ColonyDev &c, int warps, int cs, int *max_clusters);
 cudaError_t launch_construct_cluster(const ColonyDev &c, int grid, int warps, int cs,
                                      cudaStream_t s);
-// Long candidate rows (k > 32, full rows included; n <= kRowsMaxCities): a
-// CTA holds A <= kRowsMaxAnts ants of one instance, one scan warp per ant and
-// one chain warp (k_construct_rows.cu).  Each ant has a region of
-// rows_ant_bytes in shared memory (rows_layout): two buffers of compacted
-// weights and int16 ids (S = rows_slots(K) entries each), the running sums at
-// every 32nd entry, the tabu bits and a visited byte per city.  The scan
-// warps read the rows themselves from L2.
-// The last 32 slots of each buffer are per-lane sinks for the stores of
-// dropped entries (past any chain length).  With aging,
-// launch_construct_rows runs the aging plan first (two launches).
+// Long candidate rows (k > 32, full rows included; n <= kRowsMaxCities): one
+// warp per ant, at most kRowsMaxAnts a CTA (k_construct_rows.cu).  With
+// aging, launch_construct_rows runs the aging plan first (two launches).
 constexpr int kRowsMaxCities = 8192;
 constexpr int kRowsMaxAnts = 11;
-__host__ __device__ inline int rows_slots(int K) { return (K + 31) / 32 * 32 + 32; }
-struct RowsLayout {
-  int S;
-  size_t id_off, bend_off, tw_off, tb_off, bytes;
-};
-__host__ __device__ inline RowsLayout rows_layout(int n, int K) {
-  RowsLayout L;
-  L.S = rows_slots(K);
-  L.id_off = (size_t)L.S * 8;
-  L.bend_off = (size_t)L.S * 12;
-  L.tw_off = L.bend_off + ((size_t)L.S / 32 * 4 + 15) / 16 * 16;
-  L.tb_off = L.tw_off + (size_t)(((n + 31) / 32 + 3) / 4) * 16;
-  L.bytes = L.tb_off + (size_t)(n + 15) / 16 * 16;
-  return L;
-}
-__host__ __device__ inline size_t rows_ant_bytes(int n, int K) {
-  const size_t b = rows_layout(n, K).bytes;
-  return (b + 127) / 128 * 128 + 16;  // consecutive regions start four banks apart
-}
-cudaError_t configure_construct_rows(size_t smem);
 cudaError_t launch_construct_rows(const ColonyDev &c, int grid, int ants, cudaStream_t s);
-// max_ldk: the largest candidate-row pitch of the batch (every instance's
-// layout fits in rows_ant_bytes(max_n, max_ldk), as K <= ldk).
-size_t batch_rows_smem_bytes(int max_n, int max_ldk, int ants);
-cudaError_t configure_batch_construct_rows(size_t smem);
-int batch_rows_blocks_per_sm(int ants, size_t smem, bool aging);
+// max_n: the batch's largest instance (it picks the visited mask's size).
+int batch_rows_blocks_per_sm(int ants, int max_n, bool aging);
 cudaError_t launch_batch_construct_rows(const ColonyDev *descs, const int4 *items, int num_items,
-                                        int *queue_head, int grid, int ants, int max_n,
-                                        int max_ldk, bool aging, cudaStream_t s);
+                                        int *queue_head, int grid, int ants, int max_n, bool aging,
+                                        cudaStream_t s);
 cudaError_t launch_nn_to_i16(const int32_t *nn, int n, int K, int ldk, int16_t *nn16,
                              cudaStream_t s);
 cudaError_t launch_epilogue(const ColonyDev &c, cudaStream_t s);

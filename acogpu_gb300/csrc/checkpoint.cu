@@ -195,6 +195,7 @@ int aco_colony_load(aco_colony *c, const char *path) {
   if (e == cudaSuccess) e = h2d(c, c->len, len, 1, m, m);
   if (e == cudaSuccess) e = h2d(c, c->tours, tours, m, n, c->ld);
   if (e == cudaSuccess) e = h2d(c, c->newlen, newlen, 1, m, m);
+  if (e == cudaSuccess) e = launch_prior_set(colony_dev(c), c->stream);
   // choice, choice_nn, tau_nn and the row means from the restored tau/eta_nn
   if (e == cudaSuccess)
     e = launch_pheromone_rows(colony_dev(c), false, false, false, c->stream);

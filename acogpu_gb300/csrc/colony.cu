@@ -119,6 +119,7 @@ ColonyDev make_dev(const aco_colony *c) {
   d.succT = c->succT; d.predT = c->predT; d.gbtour = c->gbtour;
   d.age = c->age; d.perf = c->perf; d.valid = c->valid; d.mean = c->mean;
   d.dep_col = c->dep_col; d.dep_delta = c->dep_delta; d.plan = c->plan; d.st = c->st;
+  d.prior_set = c->prior_set;
   d.nn2 = c->nn2; d.t2v = c->t2v; d.mout = c->mout; d.t2 = c->t2;
   d.rho = c->p.rho; d.alpha = c->p.alpha; d.use_alpha = c->p.use_alpha;
   d.aging = c->p.aging; d.min_ret = c->p.min_retirement_age;
@@ -209,6 +210,7 @@ int allocate(aco_colony *c) {
   a.add(&c->plan, m + 2);
   a.add(&c->dep_col, m + 1);
   a.add(&c->dep_delta, m + 1);
+  a.add(&c->prior_set, 1);
   a.add(&c->st, 1);
   if ((s = a.commit(c))) return s;
   ACO_CUDA(c, cudaMemsetAsync(c->tours, 0, m * ld * 4, c->stream), "memset tours");
@@ -314,9 +316,7 @@ cudaError_t launch_construction(aco_colony *c, const ColonyDev &d) {
 // else the direct kernel (the same step loop on rows read from L2); otherwise,
 // and in ACO_CONSTRUCT_GLOBAL mode, the general global-memory kernel.  The
 // k <= 32 kernels put one ant per warp.  For k > 32 (mode AUTO or ROWS) the
-// long-row kernel: A ants a CTA (a scan warp each, plus the chain warp), one
-// CTA per SM, the ants spread evenly over the SMs (each ant's steps are a
-// latency-bound chain of float adds).
+// long-row kernel: one warp per ant, the ants spread evenly over the SMs.
 int plan_construction(aco_colony *c) {
   c->staged = false;
   c->direct = false;
@@ -326,16 +326,11 @@ int plan_construction(aco_colony *c) {
   const int sms = c->num_sms > 0 ? c->num_sms : 1;
   if (c->nn16 && c->n <= kRowsMaxCities && c->K > 32 &&
       (mode == ACO_CONSTRUCT_ROWS || mode == ACO_CONSTRUCT_AUTO)) {
-    const size_t per_ant = rows_ant_bytes(c->n, c->K);
-    const size_t avail = (size_t)c->max_smem_optin - 1024;  // static shared memory
     int ants = c->tune_warps > 0 ? c->tune_warps : (c->m + sms - 1) / sms;
     ants = std::max(1, std::min(ants, kRowsMaxAnts));
-    ants = std::min<int>(ants, (int)(avail / per_ant));
-    if (ants < 1) return fail(c, ACO_ERR_UNSUPPORTED, "a long row does not fit in shared memory");
-    ACO_CUDA(c, configure_construct_rows((size_t)ants * per_ant), "configure row construct");
     c->rows = true;
     c->staged_warps = ants;
-    c->staged_grid = std::min(sms, (c->m + ants - 1) / ants);
+    c->staged_grid = (c->m + ants - 1) / ants;
     return ACO_OK;
   }
   if (c->K > 32 || !c->nn16 || mode == ACO_CONSTRUCT_GLOBAL) return ACO_OK;
@@ -610,6 +605,7 @@ int init_rest(aco_colony *c) {
   }
   ACO_CUDA(c, launch_gather_nn_f32(c->eta, n, c->ld, c->nn, c->K, c->ldk, c->eta_nn, c->stream),
            "eta_nn");
+  ACO_CUDA(c, cudaMemsetAsync(c->prior_set, 0, sizeof(int32_t), c->stream), "memset prior");
   if (c->nn16) ACO_CUDA(c, launch_nn_to_i16(c->nn, n, c->K, c->ldk, c->nn16, c->stream), "nn16");
 
   const ColonyDev d = make_dev(c);
@@ -1012,7 +1008,7 @@ struct aco_batch {
   size_t region_bytes = 0;  // shared region of the construction launch
   int staged_count = 0;     // instances built from a staged table
   bool rows = false;        // construction by the long-row batch kernel (every k > 32)
-  int min_k = 1 << 30, max_ldk_rows = 0;
+  int min_k = 1 << 30;
   bool initialized = false;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
@@ -1093,11 +1089,9 @@ int batch_build_items(aco_batch *b) {
   }
   // The launch shape first: the grid decides how many items make whole waves.
   if (b->rows) {
-    const size_t smem = batch_rows_smem_bytes(b->max_n, b->max_ldk_rows, b->apb);
-    if (b->apb > kRowsMaxAnts || smem + 1024 > (size_t)b->max_smem_optin)
-      return bfail(b, ACO_ERR_UNSUPPORTED, "too many ants per CTA for the long rows' buffers");
-    ACO_BCUDA(b, configure_batch_construct_rows(smem), "configure batch row construct");
-    b->grid = b->num_sms * batch_rows_blocks_per_sm(b->apb, smem, b->p.aging != 0);
+    if (b->apb > kRowsMaxAnts)
+      return bfail(b, ACO_ERR_UNSUPPORTED, "too many ants per CTA for the long-row kernel");
+    b->grid = b->num_sms * batch_rows_blocks_per_sm(b->apb, b->max_n, b->p.aging != 0);
   } else {
     const size_t smem = batch_construct_smem_bytes(b->region_bytes, b->apb);
     ACO_BCUDA(b, configure_batch_construct(smem), "configure batch construct");
@@ -1109,18 +1103,19 @@ int batch_build_items(aco_batch *b) {
   // tour).  When every instance has the same n and m the items take equally
   // long, and their count is raised to whole waves of the grid (at most apb
   // and at least one ant an item): the last wave then runs as many items as
-  // the others, each a little lighter, instead of leaving CTAs idle.
+  // the others, each a little lighter, instead of leaving CTAs idle.  The
+  // long-row kernel's warps take single ants.
   const size_t ni = b->cols.size();
   std::vector<int> parts(ni);
   bool uniform = true;
   long total = 0;
   for (size_t i = 0; i < ni; i++) {
     const aco_colony *c = b->cols[i];
-    parts[i] = (c->m + b->apb - 1) / b->apb;
+    parts[i] = b->rows ? c->m : (c->m + b->apb - 1) / b->apb;
     total += parts[i];
     uniform = uniform && c->n == b->cols[0]->n && c->m == b->cols[0]->m;
   }
-  if (uniform && b->grid > 0 && total % b->grid != 0) {
+  if (uniform && !b->rows && b->grid > 0 && total % b->grid != 0) {
     const long target = (total + b->grid - 1) / b->grid * b->grid;
     for (size_t i = 0; i < ni; i++) {
       const long want = target / (long)ni + ((long)i < target % (long)ni ? 1 : 0);
@@ -1157,8 +1152,8 @@ int batch_enqueue(aco_batch *b, bool construct, bool epilogue, bool rows, bool u
     }
     if (b->rows)
       ACO_BCUDA(b, launch_batch_construct_rows(b->d_descs, b->d_items, b->num_items, b->d_queue,
-                                               b->grid, b->apb, b->max_n, b->max_ldk_rows,
-                                               b->p.aging != 0, b->stream),
+                                               b->grid, b->apb, b->max_n, b->p.aging != 0,
+                                               b->stream),
                 "batch row construct");
     else
       ACO_BCUDA(b, launch_batch_construct(b->d_descs, b->d_items, b->num_items, b->d_queue,
@@ -1261,25 +1256,16 @@ int aco_batch_create(const aco_params *params, int32_t count, const int32_t *siz
     b->max_n = std::max(b->max_n, c->n);
     b->max_k = std::max(b->max_k, c->K);
     b->min_k = std::min(b->min_k, c->K);
-    b->max_ldk_rows = std::max(b->max_ldk_rows, c->ldk);
     if (c->K <= 32) b->sp = std::max(b->sp, c->ldk);
     b->max_ld = std::max(b->max_ld, c->ld);
     b->total_rows += n;
   }
   if (b->sp == 0) b->sp = 32;
   // Candidate rows longer than 32 in every instance (full rows included):
-  // the long-row batch kernel, when every instance has int16 ids and one
-  // ant's buffers fit.
-  b->rows = b->min_k > 32 && params->construct_mode != ACO_CONSTRUCT_GLOBAL &&
-            batch_rows_smem_bytes(b->max_n, b->max_ldk_rows, 1) + 1024 <=
-                (size_t)b->max_smem_optin;
+  // the long-row batch kernel, when every instance has int16 ids.
+  b->rows = b->min_k > 32 && params->construct_mode != ACO_CONSTRUCT_GLOBAL;
   for (aco_colony *c : b->cols)
     if (!c->nn16) b->rows = false;
-  if (b->rows) b->apb = kRowsMaxAnts;  // as many ants a CTA as the registers allow
-  while (b->rows && b->apb > 1 &&
-         batch_rows_smem_bytes(b->max_n, b->max_ldk_rows, b->apb) + 1024 >
-             (size_t)b->max_smem_optin)
-    b->apb--;
   *out = b;
   return ACO_OK;
 }
@@ -1512,7 +1498,7 @@ int aco_batch_autotune(aco_batch *b, aco_tuning *out) {
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   // Ants per CTA: warps of the k <= 32 kernels (launch-bounded to 512
-  // threads); ants (scan warps, plus the chain warp) of the long-row kernel.
+  // threads); ants (one a warp) of the long-row kernel.
   const int apbs_short[6] = {1, 2, 4, 8, 16, kBatchMaxWarps};
   const int apbs_rows[6] = {2, 4, 6, 8, 11, 11};
   const int *apbs = b->rows ? apbs_rows : apbs_short;
@@ -1520,7 +1506,7 @@ int aco_batch_autotune(aco_batch *b, aco_tuning *out) {
   int best_apb = b->apb;
   for (int ai = 0; ai < 6; ai++) {
     const int apb = apbs[ai];
-    const size_t need = b->rows ? batch_rows_smem_bytes(b->max_n, b->max_ldk_rows, apb) + 1024
+    const size_t need = b->rows ? 0
                                 : batch_construct_smem_bytes(
                                       batch_plan_region(b, apb, nullptr, nullptr), apb);
     if (need > (size_t)b->max_smem_optin || (b->rows && apb > kRowsMaxAnts)) continue;

@@ -393,9 +393,32 @@ cudaError_t launch_gather_nn_f32(const float *src, int n, int ld, const int32_t 
   return cudaGetLastError();
 }
 
+// Whether the candidate heuristic is anything but the plain heuristic in
+// candidate order (bit for bit): full rows are summed from the plain choice
+// matrix only while the two agree.  Run after whatever rewrites eta_nn.
+__global__ void k_prior_set(ColonyDev c) {
+  const int64_t total = (int64_t)c.n * c.K;
+  bool differs = false;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t j = t / c.K;
+    const int r = (int)(t % c.K);
+    const float plain = c.eta[j * c.ld + c.nn[j * c.ldk + r]];
+    differs |= __float_as_uint(c.eta_nn[j * c.ldk + r]) != __float_as_uint(plain);
+  }
+  if (__any_sync(kFull, differs) && (threadIdx.x & 31) == 0) *c.prior_set = 1;
+}
+
+cudaError_t launch_prior_set(const ColonyDev &c, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(c.prior_set, 0, sizeof(int32_t), s);
+  if (e != cudaSuccess) return e;
+  k_prior_set<<<608, 256, 0, s>>>(c);
+  return cudaGetLastError();
+}
+
 // int16 copy of the candidate rows (same pitch; entries past the K
 // candidates of a row are -1).  The staged kernel keeps the k <= 32 table in
-// shared memory; the long-row kernel copies one row at a time by TMA.
+// shared memory; the long-row kernel reads rows from L2.
 __global__ void k_nn_to_i16(const int32_t *__restrict__ nn, int n, int K, int ldk,
                             int16_t *__restrict__ nn16) {
   const int64_t total = (int64_t)n * ldk;

@@ -5,6 +5,7 @@ colony, rows longer than one scan round (n > 1024), candidate lists of
 weights), ants that blend their fitness after convergence, and batches whose
 instances differ in size."""
 import os
+import tempfile
 
 import numpy as np
 import pytest
@@ -12,6 +13,7 @@ import pytest
 import oracle
 import acogpu_gb300 as aco
 from acogpu_gb300 import _abi, instances
+from acogpu_gb300.prior import EdgePrior, candidate_heuristic
 from helpers import assert_same_state, bits, instance
 
 pytestmark = pytest.mark.gpu
@@ -122,3 +124,70 @@ def test_batch_of_long_rows_of_uneven_size():
     for q in ports:
         q.close()
     b.close()
+
+
+@pytest.mark.parametrize("n,k", [(33, 0), (64, 0), (127, 0), (128, 0), (129, 0), (1023, 0),
+                                 (1024, 0), (1025, 0), (2051, 0), (300, 33), (300, 127),
+                                 (300, 128), (300, 129), (1100, 1099), (4100, 40)])
+@pytest.mark.parametrize("aging", [0, 1])
+def test_row_edges_match_the_port(n, k, aging):
+    """Row lengths around a lane's four entries, a chunk (128) and a round
+    (1024), full rows and candidate lists; bit for bit."""
+    _, _, d = instance(n, 400 + n + k, kind="clustered" if n % 2 else "uniform")
+    more = dict(nn_order=_abi.ACO_NN_STABLE, heuristic=_abi.ACO_HEURISTIC_DEVICE,
+                fallback=_abi.ACO_FALLBACK_BEST, tau0_mode=_abi.ACO_TAU0_DORIGO) if k else {}
+    p = _abi.default_params(num_ants=60 if n < 1000 else 24, aging=aging, cand_k=k, rho=0.2,
+                            beta=2.0, seed=n + k, **more)
+    run_vs_port(d, p, 3 if n < 1000 else 2, f"n={n} k={k}")
+
+
+@pytest.mark.parametrize("n,k", [(90, 0), (200, 70)])
+def test_long_rows_with_a_prior_match_the_port(n, k):
+    """A learned prior on long rows: the candidate heuristic is no longer the
+    plain one, so full rows are summed in row order; a checkpoint of the colony
+    continues the same way, and initialising drops the prior again."""
+    x, y, d = instance(n, 500 + n)
+    p = _abi.default_params(num_ants=40, cand_k=k, rho=0.2, beta=2.0, seed=9,
+                            fallback=_abi.ACO_FALLBACK_BEST if k else _abi.ACO_FALLBACK_REFERENCE)
+    g = aco.Colony(coords=(x, y), params=p, num_ants=40)
+    g.initialize()
+    g.run(1)
+    pr = EdgePrior(seed=5)
+    g.initialize()
+    pr.apply(g, floor=0.05)
+    q = oracle.Port(p, d, threads=THREADS)
+    q.initialize()
+    q.set_candidate_heuristic(candidate_heuristic(g))
+    for it in range(3):
+        g.constructSolution()
+        q.iterate()
+        assert_same_state(g, q, ctx=f"prior iteration {it}")
+    with tempfile.TemporaryDirectory() as tmp:
+        g.save(os.path.join(tmp, "c"))
+        h = aco.Colony(coords=(x, y), params=p, num_ants=40)
+        h.initialize()
+        h.load(os.path.join(tmp, "c"))
+    q.iterate()
+    for col in (g, h):
+        col.constructSolution()
+        assert_same_state(col, q, ctx="after the checkpoint")
+    g.initialize()
+    q2 = oracle.Port(p, d, threads=THREADS)
+    q2.initialize()
+    for it in range(2):
+        g.constructSolution()
+        q2.iterate()
+        assert_same_state(g, q2, ctx=f"plain again {it}")
+    for col in (g, h, q, q2):
+        col.close()
+    pr.close()
+
+
+@pytest.mark.parametrize("side,aging", [(8, 0), (20, 1), (34, 0)])
+def test_lattice_rows_match_the_port(side, aging):
+    """Cities on an integer lattice: few distinct distances, so weights repeat,
+    running sums fall halfway between floats and thresholds land on them."""
+    x, y = np.meshgrid(np.arange(side, dtype=np.float32), np.arange(side, dtype=np.float32))
+    d = instances.euc2d_distances(x.ravel(), y.ravel())
+    p = _abi.default_params(num_ants=40, aging=aging, cand_k=0, rho=0.5, beta=2.0, seed=side)
+    run_vs_port(d, p, 4, f"lattice {side}")
