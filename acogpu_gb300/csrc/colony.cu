@@ -1266,6 +1266,14 @@ int aco_batch_create(const aco_params *params, int32_t count, const int32_t *siz
   b->rows = b->min_k > 32 && params->construct_mode != ACO_CONSTRUCT_GLOBAL;
   for (aco_colony *c : b->cols)
     if (!c->nn16) b->rows = false;
+  // Ants per CTA until tuned: the ants spread over the SMs, at most what the
+  // kernel's registers allow (20 warps, one CTA an SM; the long-row kernel
+  // keeps four CTAs of 8 warps an SM).  512 instances of 50 to 2000 cities:
+  // construction 55.5 ms at the former 8 ants a CTA, 30 at 20.
+  int64_t ants = 0;
+  for (aco_colony *c : b->cols) ants += c->m;
+  b->apb = (int)std::min<int64_t>(b->rows ? 8 : kBatchMaxWarps,
+                                  std::max<int64_t>(1, (ants + b->num_sms - 1) / b->num_sms));
   *out = b;
   return ACO_OK;
 }
