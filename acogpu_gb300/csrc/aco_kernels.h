@@ -53,8 +53,6 @@ constexpr int kStagedMaxWarps = 16;
 // Warps (ants) per CTA of the batch kernel: 20 fit the register file
 // without spilling (launch bound 640 threads, at most 102 registers).
 constexpr int kBatchMaxWarps = 20;
-// Launches of at most this many warps per CTA may hold 255 registers a thread.
-constexpr int kWideFallbackWarps = 8;
 // Pitch of the candidate rows (nn, eta_nn, tau_nn, choice_nn, nn16) for
 // k <= 32: the staged step folds pitch/4 groups of four weights, and the
 // pitch takes one of four values so the fold length is a template constant.
@@ -73,7 +71,7 @@ __host__ __device__ inline StagedLayout staged_layout(int n, int ld, int sp, boo
   L.table = L.mean_off + (aging ? (size_t)ld * 4 : 0);
   return L;
 }
-size_t construct_staged_smem_bytes(int n, int ld, int sp, bool aging, int warps);
+size_t construct_staged_smem_bytes(int n, int ld, int sp, bool aging);
 cudaError_t configure_construct_staged(size_t smem);
 cudaError_t launch_construct_staged(const ColonyDev &c, const int16_t *nn16, int grid, int warps,
                                     cudaStream_t s);
@@ -114,7 +112,7 @@ cudaError_t launch_batch_pheromone_rows(const ColonyDev *descs, const int2 *rowm
 // the per-warp tabu lists of an L2-row item.
 size_t batch_staged_table_bytes(int n, int ld, int sp, bool aging);
 size_t batch_region_bytes(int max_n, int max_k, int warps, size_t max_table);
-size_t batch_construct_smem_bytes(size_t region_bytes, int warps);
+size_t batch_construct_smem_bytes(size_t region_bytes);
 cudaError_t configure_batch_construct(size_t smem);
 int batch_construct_blocks_per_sm(int warps, size_t smem, bool multi, int sp, bool aging);
 // sp: the pitch of the staged items (every staged item's ldk equals it).

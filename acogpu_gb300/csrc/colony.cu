@@ -352,7 +352,7 @@ int plan_construction(aco_colony *c) {
   }
   if (c->n <= 2048 && (mode == ACO_CONSTRUCT_AUTO || mode == ACO_CONSTRUCT_STAGED)) {
     const size_t smem =
-        construct_staged_smem_bytes(c->n, c->ld, c->ldk, c->p.aging != 0, c->staged_warps);
+        construct_staged_smem_bytes(c->n, c->ld, c->ldk, c->p.aging != 0);
     if (smem <= (size_t)c->max_smem_optin) {
       ACO_CUDA(c, configure_construct_staged(smem), "configure staged construct");
       c->staged = true;
@@ -1054,7 +1054,7 @@ size_t batch_plan_region(const aco_batch *b, int apb, std::vector<char> *staged,
   const bool aging = b->p.aging != 0;
   // static shared memory of the kernel (descriptor, item, flags) plus slack
   const size_t fixed = sizeof(ColonyDev) + 256;
-  const size_t avail = (size_t)b->max_smem_optin - batch_construct_smem_bytes(0, apb) - fixed;
+  const size_t avail = (size_t)b->max_smem_optin - batch_construct_smem_bytes(0) - fixed;
   size_t max_table = 0;
   int cnt = 0;
   if (staged) staged->assign(b->cols.size(), 0);
@@ -1093,7 +1093,7 @@ int batch_build_items(aco_batch *b) {
       return bfail(b, ACO_ERR_UNSUPPORTED, "too many ants per CTA for the long-row kernel");
     b->grid = b->num_sms * batch_rows_blocks_per_sm(b->apb, b->max_n, b->p.aging != 0);
   } else {
-    const size_t smem = batch_construct_smem_bytes(b->region_bytes, b->apb);
+    const size_t smem = batch_construct_smem_bytes(b->region_bytes);
     ACO_BCUDA(b, configure_batch_construct(smem), "configure batch construct");
     b->grid = b->num_sms * batch_construct_blocks_per_sm(b->apb, smem, b->max_k > 32, b->sp,
                                                          b->p.aging != 0);
@@ -1516,7 +1516,7 @@ int aco_batch_autotune(aco_batch *b, aco_tuning *out) {
     const int apb = apbs[ai];
     const size_t need = b->rows ? 0
                                 : batch_construct_smem_bytes(
-                                      batch_plan_region(b, apb, nullptr, nullptr), apb);
+                                      batch_plan_region(b, apb, nullptr, nullptr));
     if (need > (size_t)b->max_smem_optin || (b->rows && apb > kRowsMaxAnts)) continue;
     b->apb = apb;
     if (int s = batch_build_items(b)) return s;

@@ -115,7 +115,7 @@ cudaError_t launch_batch_aging_plan(const ColonyDev *descs, int count, cudaStrea
 // ids and FP32 choice values at pitch 4G -- into shared memory with TMA bulk
 // copies once per launch, so a construction step touches only shared memory.
 // One CTA per SM; its warps loop over ants.  Shared-memory layout: the table
-// of staged_layout, then per warp 32 f32, then the mbarrier.
+// of staged_layout, then the mbarrier.
 //
 // Without aging every CTA stages the table and its warps build tours.  With
 // aging the ants' roles come from k_aging_plan: CTA b < B takes blend ant b
@@ -136,8 +136,7 @@ __global__ void __launch_bounds__(kStagedMaxWarps * 32)
   float *scw = reinterpret_cast<float *>(smem_staged);
   int16_t *sids = reinterpret_cast<int16_t *>(smem_staged + L.ids_off);
   float *smean = reinterpret_cast<float *>(smem_staged + L.mean_off);
-  float *wbuf = reinterpret_cast<float *>(smem_staged + L.table) + (size_t)warp * 32;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smem_staged + L.table + (size_t)warps * 128);
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem_staged + L.table);
   __shared__ int flag;
   const TableRows<SP> rows{sids, scw, smean};
 
@@ -221,8 +220,7 @@ __global__ void __launch_bounds__(kStagedMaxWarps * 32)
         a.blend = true;
         a.ratio = ratio;
         a.meanc = 0.0f;
-        staged_ant_body<TW, G, false, true, TableRows<SP>, 4, false, TIER>(c, k, iter, wbuf, rows,
-                                                                          a, lane);
+        staged_ant_body<TW, G, false, TableRows<SP>, TIER>(c, k, iter, nullptr, rows, a, lane);
       }
       __syncthreads();
     }
@@ -244,8 +242,7 @@ __global__ void __launch_bounds__(kStagedMaxWarps * 32)
   const int others = c.m - B;
   for (int i = ((int)blockIdx.x - base) + P * warp; i < others; i += P * warps) {
     if (!AGING) {
-      construct_ant_staged<false, TW, G, TableRows<SP>, 4, false, TIER>(c, i, iter, wbuf, rows,
-                                                                         lane);
+      construct_ant_staged<false, TW, G, TableRows<SP>, TIER>(c, i, iter, nullptr, rows, lane);
       continue;
     }
     const int k = plan_list[B + i];
@@ -258,22 +255,20 @@ __global__ void __launch_bounds__(kStagedMaxWarps * 32)
     a.blend = false;
     a.ratio = 0.0f;
     a.meanc = 0.0f;
-    staged_ant_body<TW, G, false, false, TableRows<SP>, 4, false, TIER>(c, k, iter, wbuf, rows, a,
-                                                                       lane);
+    staged_ant_body<TW, G, false, TableRows<SP>, TIER>(c, k, iter, nullptr, rows, a, lane);
   }
 }
 
 // k <= 32 with a candidate table too large for shared memory (e.g. n = 4096,
 // k = 32: 768 KB): the staged step loop reading its rows straight from L2
-// (the same pitch-`4G` choice values and int16 ids), the tabu list in
-// registers (TW words per lane, n <= 1024 * TW).
+// (the same pitch-`4G` choice values and int16 ids; n <= 1024 * TW).
 template <bool AGING, int TW, int G>
 __global__ void __launch_bounds__(kStagedMaxWarps * 32) k_construct_direct(ColonyDev c) {
-  __shared__ __align__(16) float wb[kStagedMaxWarps * 32];
+  __shared__ uint32_t words[TW > 2 ? kStagedMaxWarps : 1][TW > 2 ? TW * 32 : 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const uint32_t iter = c.st->iteration;
   for (int k = blockIdx.x * warps + warp; k < c.m; k += gridDim.x * warps)
-    construct_ant_staged<AGING, TW, G>(c, k, iter, wb + warp * 32,
+    construct_ant_staged<AGING, TW, G>(c, k, iter, words[TW > 2 ? warp : 0],
                                        TableRows<4 * G>{c.nn16, c.choice_nn, c.mean}, lane);
 }
 
@@ -314,8 +309,8 @@ size_t construct_smem_bytes(int n, int K, int ants_per_block) {
   return (size_t)ants_per_block * per_warp * 4;
 }
 
-size_t construct_staged_smem_bytes(int n, int ld, int sp, bool aging, int warps) {
-  return staged_layout(n, ld, sp, aging).table + (size_t)warps * 128 + 16;
+size_t construct_staged_smem_bytes(int n, int ld, int sp, bool aging) {
+  return staged_layout(n, ld, sp, aging).table + 16;
 }
 
 cudaError_t configure_construct(size_t smem) {
@@ -405,7 +400,7 @@ cudaError_t launch_construct(const ColonyDev &c, int apb, cudaStream_t s) {
 cudaError_t launch_construct_staged(const ColonyDev &c, const int16_t *nn16, int grid, int warps,
                                     cudaStream_t s) {
   if (c.n > 2048 || c.K > 32 || c.ldk != staged_pitch(c.K)) return cudaErrorInvalidValue;
-  const size_t smem = construct_staged_smem_bytes(c.n, c.ld, c.ldk, c.aging, warps);
+  const size_t smem = construct_staged_smem_bytes(c.n, c.ld, c.ldk, c.aging);
   switch (c.ldk) {
     case 16: return staged_launch<4>(c, nn16, grid, warps, smem, s);
     case 20: return staged_launch<5>(c, nn16, grid, warps, smem, s);

@@ -21,7 +21,7 @@ namespace aco {
 // single-colony kernel.  Other items with the same pitch (n <= 2048) run that
 // step loop on rows read from L2; the rest use the general kernel with the
 // tabu list in the region.  Shared layout:
-//   [region: table, or per-warp tabu lists][per warp: 32 f32][mbarrier]
+//   [region: table, or per-warp tabu lists][mbarrier]
 template <bool MULTI, bool AGING, int G>
 __global__ void __launch_bounds__(kBatchMaxWarps * 32) k_batch_construct(const ColonyDev *__restrict__ descs,
                                                          const int4 *__restrict__ items,
@@ -31,13 +31,12 @@ __global__ void __launch_bounds__(kBatchMaxWarps * 32) k_batch_construct(const C
   extern __shared__ __align__(128) unsigned char smem_bc[];
   __shared__ ColonyDev s_desc;
   __shared__ int s_item, s_ok;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t *tabu = reinterpret_cast<uint32_t *>(smem_bc) +
                    (size_t)warp * (words + 32 + (MULTI ? max_chunks : 0));
   float *wbuf = reinterpret_cast<float *>(tabu + words);
   float *cend = wbuf + 32;
-  float *swbuf = reinterpret_cast<float *>(smem_bc + region_bytes) + (size_t)warp * 32;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smem_bc + region_bytes + (size_t)warps * 128);
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem_bc + region_bytes);
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     fence_barrier_init();
@@ -86,17 +85,17 @@ __global__ void __launch_bounds__(kBatchMaxWarps * 32) k_batch_construct(const C
       if (!s_ok) break;
       if (warp < w.z) {
         if (n <= 1024)
-          construct_ant_staged<AGING, 1, G, TableRows<4 * G>, 4, true>(
-              c, w.y + warp, c.st->iteration, swbuf, TableRows<4 * G>{sids, scw, smean}, lane);
+          construct_ant_staged<AGING, 1, G, TableRows<4 * G>>(
+              c, w.y + warp, c.st->iteration, nullptr, TableRows<4 * G>{sids, scw, smean}, lane);
         else
-          construct_ant_staged<AGING, 2, G, TableRows<4 * G>, 4, true>(
-              c, w.y + warp, c.st->iteration, swbuf, TableRows<4 * G>{sids, scw, smean}, lane);
+          construct_ant_staged<AGING, 2, G, TableRows<4 * G>>(
+              c, w.y + warp, c.st->iteration, nullptr, TableRows<4 * G>{sids, scw, smean}, lane);
       }
     } else if (!MULTI && c.nn16 && c.ldk == 4 * G && c.n <= 2048) {
       // Too large to stage: the same step loop on rows read from L2.
       if (warp < w.z)
-        construct_ant_staged<AGING, 2, G, TableRows<4 * G>, 4, true>(
-            c, w.y + warp, c.st->iteration, swbuf,
+        construct_ant_staged<AGING, 2, G, TableRows<4 * G>>(
+            c, w.y + warp, c.st->iteration, nullptr,
             TableRows<4 * G>{c.nn16, c.choice_nn, c.mean}, lane);
     } else if (warp < w.z) {
       construct_ant<MULTI, AGING, false>(c, w.y + warp, c.st->iteration, tabu, cend, wbuf,
@@ -116,9 +115,7 @@ size_t batch_region_bytes(int max_n, int max_k, int warps, size_t max_table) {
   return ((tabu > max_table ? tabu : max_table) + 127) / 128 * 128;
 }
 
-size_t batch_construct_smem_bytes(size_t region_bytes, int warps) {
-  return region_bytes + (size_t)warps * 128 + 16;
-}
+size_t batch_construct_smem_bytes(size_t region_bytes) { return region_bytes + 16; }
 
 size_t batch_staged_table_bytes(int n, int ld, int sp, bool aging) {
   return staged_layout(n, ld, sp, aging).table;
@@ -181,7 +178,7 @@ cudaError_t launch_batch_construct(const ColonyDev *descs, const int4 *items, in
                                    size_t region_bytes, int sp, bool aging, cudaStream_t s) {
   const int words = (max_n + 31) / 32;
   const int chunks = (max_k + 31) / 32;
-  const size_t smem = batch_construct_smem_bytes(region_bytes, warps);
+  const size_t smem = batch_construct_smem_bytes(region_bytes);
   const uint32_t rb = (uint32_t)region_bytes;
   if (max_k > 32)
     return aging ? batch_launch<true, true, 8>(descs, items, num_items, queue_head, grid, warps,

@@ -14,10 +14,7 @@ namespace aco {
 // keeps each slice alive until the whole cluster is done.  Every thread
 // reaches both barriers on every path (a copy that timed out only records
 // the error, and the ants run only when every rank staged its slice).  All
-// CTAs share all ants.  Launches of at most kWideFallbackWarps warps use the
-// FB = 16 instantiation (255 registers a thread: the fallback's full-row scan
-// keeps 16 row chunks in flight); the fallback is a called function here
-// (ClusterRows::kOutlineFallback), which keeps the step loop small.
+// CTAs share all ants.
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -37,8 +34,8 @@ __device__ __forceinline__ void cluster_barrier() {
           : "memory");
 }
 
-template <bool AGING, int TW, int G, int FB>
-__global__ void __launch_bounds__((FB > 4 ? kWideFallbackWarps : kStagedMaxWarps) * 32)
+template <bool AGING, int TW, int G>
+__global__ void __launch_bounds__(kStagedMaxWarps * 32)
     k_construct_cluster(ColonyDev c) {
   extern __shared__ __align__(128) unsigned char smem_cl[];
   constexpr int SP = 4 * G;
@@ -47,8 +44,8 @@ __global__ void __launch_bounds__((FB > 4 ? kWideFallbackWarps : kStagedMaxWarps
   float *scw = reinterpret_cast<float *>(smem_cl);
   int16_t *sids = reinterpret_cast<int16_t *>(smem_cl + L.ids_off);
   float *smean = reinterpret_cast<float *>(smem_cl + L.mean_off);
-  float *wbuf = reinterpret_cast<float *>(smem_cl + L.table) + (size_t)warp * 32;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smem_cl + L.table + (size_t)warps * 128);
+  uint32_t *words = reinterpret_cast<uint32_t *>(smem_cl + L.table) + (size_t)warp * TW * 32;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem_cl + L.table + (size_t)warps * TW * 128);
   __shared__ int flag, all_ok;
 
   const int r0 = (int)cluster_rank() * kClusterRows;
@@ -98,26 +95,28 @@ __global__ void __launch_bounds__((FB > 4 ? kWideFallbackWarps : kStagedMaxWarps
     const ClusterRows<SP> rows{smem_u32(sids), smem_u32(scw), smem_u32(smean)};
     const uint32_t iter = c.st->iteration;
     for (int k = blockIdx.x * warps + warp; k < c.m; k += gridDim.x * warps)
-      construct_ant_staged<AGING, TW, G, ClusterRows<SP>, FB>(c, k, iter, wbuf, rows, lane);
+      construct_ant_staged<AGING, TW, G, ClusterRows<SP>>(c, k, iter, words, rows, lane);
   }
   __syncthreads();
   cluster_barrier();  // no slice is released while another CTA may read it
 }
 
-size_t construct_cluster_smem_bytes(int sp, bool aging, int warps) {
-  return staged_layout(kClusterRows, kClusterRows, sp, aging).table + (size_t)warps * 128 + 16;
+// The slice's table, the tabu words of every warp (used above TW = 2), the
+// mbarrier.
+size_t construct_cluster_smem_bytes(int sp, bool aging, int warps, int tw) {
+  return staged_layout(kClusterRows, kClusterRows, sp, aging).table + (size_t)warps * tw * 128 + 16;
 }
 
 namespace {
-template <bool AGING, int TW, int G, int FB>
+template <bool AGING, int TW, int G>
 cudaError_t cluster_launch_t(const ColonyDev &c, int grid, int warps, int cs, cudaStream_t s,
                              int *max_clusters) {
-  const size_t smem = construct_cluster_smem_bytes(4 * G, AGING, warps);
+  const size_t smem = construct_cluster_smem_bytes(4 * G, AGING, warps, TW);
   if (max_clusters) {
     // the query, at planning time, opens the kernel to any warp count, so a
     // launch (possibly under stream capture) sets no attribute
-    const size_t most = construct_cluster_smem_bytes(4 * G, AGING, kStagedMaxWarps);
-    cudaError_t e = cudaFuncSetAttribute(k_construct_cluster<AGING, TW, G, FB>,
+    const size_t most = construct_cluster_smem_bytes(4 * G, AGING, kStagedMaxWarps, TW);
+    cudaError_t e = cudaFuncSetAttribute(k_construct_cluster<AGING, TW, G>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e != cudaSuccess) return e;
   }
@@ -134,20 +133,15 @@ cudaError_t cluster_launch_t(const ColonyDev &c, int grid, int warps, int cs, cu
   cfg.attrs = at;
   cfg.numAttrs = 1;
   if (max_clusters)
-    return cudaOccupancyMaxActiveClusters(max_clusters, k_construct_cluster<AGING, TW, G, FB>, &cfg);
-  return cudaLaunchKernelEx(&cfg, k_construct_cluster<AGING, TW, G, FB>, c);
+    return cudaOccupancyMaxActiveClusters(max_clusters, k_construct_cluster<AGING, TW, G>, &cfg);
+  return cudaLaunchKernelEx(&cfg, k_construct_cluster<AGING, TW, G>, c);
 }
 template <bool AGING, int G>
 cudaError_t cluster_launch_tw(const ColonyDev &c, int grid, int warps, int cs, cudaStream_t s,
                               int *max_clusters) {
-  // n > 2048 with few ants per CTA: the fallback scan with 16 chunks in flight
-  const bool wide = warps <= kWideFallbackWarps;
-  if (c.n <= 2048) return cluster_launch_t<AGING, 2, G, 4>(c, grid, warps, cs, s, max_clusters);
-  if (c.n <= 4096)
-    return wide ? cluster_launch_t<AGING, 4, G, 16>(c, grid, warps, cs, s, max_clusters)
-                : cluster_launch_t<AGING, 4, G, 4>(c, grid, warps, cs, s, max_clusters);
-  return wide ? cluster_launch_t<AGING, 8, G, 16>(c, grid, warps, cs, s, max_clusters)
-              : cluster_launch_t<AGING, 8, G, 4>(c, grid, warps, cs, s, max_clusters);
+  if (c.n <= 2048) return cluster_launch_t<AGING, 2, G>(c, grid, warps, cs, s, max_clusters);
+  if (c.n <= 4096) return cluster_launch_t<AGING, 4, G>(c, grid, warps, cs, s, max_clusters);
+  return cluster_launch_t<AGING, 8, G>(c, grid, warps, cs, s, max_clusters);
 }
 template <int G>
 cudaError_t cluster_launch_g(const ColonyDev &c, int grid, int warps, int cs, cudaStream_t s,
@@ -172,13 +166,8 @@ cudaError_t cluster_dispatch(const ColonyDev &c, int grid, int warps, int cs, cu
 
 cudaError_t query_construct_cluster(const ColonyDev &c, int warps, int cs, int *max_clusters) {
   *max_clusters = 0;
-  // Both fallback widths (the query also opens each kernel's shared memory):
-  // the launch picks one by its final warp count.
-  int wide = 0, narrow = 0;
-  cudaError_t e = cluster_dispatch(c, cs, kWideFallbackWarps, cs, nullptr, &wide);
-  if (e == cudaSuccess) e = cluster_dispatch(c, cs, kStagedMaxWarps, cs, nullptr, &narrow);
-  if (e == cudaSuccess) *max_clusters = warps <= kWideFallbackWarps ? wide : narrow;
-  return e;
+  // The query also opens the kernel's shared memory.
+  return cluster_dispatch(c, cs, warps, cs, nullptr, max_clusters);
 }
 
 cudaError_t launch_construct_cluster(const ColonyDev &c, int grid, int warps, int cs,

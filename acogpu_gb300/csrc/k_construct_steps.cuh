@@ -16,10 +16,10 @@
 //    src/Colony.cu:814; partial_sum += ..., :840); rows longer than 32 keep
 //    the prefix at each chunk end and redo only the chunk of the crossing;
 //  * staged_steps (k <= 32; the staged, cluster, direct and batch kernels):
-//    the tabu list in registers, lane r holding candidate r of the current
-//    row, every lane's prefix formed by masked FMAs (see staged_steps), the
-//    rows read through a policy (TableRows: shared or global memory;
-//    ClusterRows: distributed shared memory of a thread-block cluster).
+//    lane r holding candidate r of the current row, the pick settled by
+//    bounded sums (see staged_steps), the rows read through a policy
+//    (TableRows: shared or global memory; ClusterRows: distributed shared
+//    memory of a thread-block cluster).
 //
 // In both, the crossing `first i with partial_sum > u * sum` is a ballot;
 // when the roulette cannot pick (sum <= 0, or no crossing) the fallback is
@@ -322,14 +322,12 @@ __device__ void construct_ant(const ColonyDev &c, int k, uint32_t iter, uint32_t
 // Staged construction step, specialised for the short critical path of one
 // ant: candidate rows in shared memory, the tabu bitmask in registers (lane
 // l owns the 32-city words l, l+32, ...; a lookup is one __shfl_sync and the
-// owner lane sets the bit), the non-zero weights compacted into a
-// zero-padded 32-float buffer and folded in lane order from broadcast
-// 16-byte reads.
+// owner lane sets the bit).
 // TW words per lane cover 1024*TW cities: word w of the tabu list is held
 // by lane w % 32 as its register w / 32.  A city past the list (a padding id)
 // reads as unvisited.
 template <int TW>
-__device__ __forceinline__ bool reg_visited(const uint32_t (&tw)[TW], int city) {
+__device__ __forceinline__ uint32_t reg_word(const uint32_t (&tw)[TW], int city) {
   const int word = city >> 5;
   uint32_t v = __shfl_sync(kFull, tw[0], word & 31);
 #pragma unroll
@@ -338,7 +336,7 @@ __device__ __forceinline__ bool reg_visited(const uint32_t (&tw)[TW], int city) 
     v = (word >> 5) == t ? x : v;
   }
   if (TW > 1 && (word >> 5) >= TW) v = 0u;
-  return (v >> (city & 31)) & 1u;
+  return v;
 }
 
 // Every register is updated (with the bit or with 0), so the compiler never
@@ -365,130 +363,121 @@ __device__ __forceinline__ uint32_t tw_pick(const uint32_t (&tw)[TW], int t) {
   return v;
 }
 
-// Largest choice value among unvisited cities (register tabu version).  The
-// plain rule issues the row loads FB 128-city chunks at a time, so a scan of
-// n cities waits for ceil(n / (128 FB)) L2 round trips, not one per chunk
-// (FB = 16 holds 64 registers of loads: kernels launched for at most
-// kWideFallbackWarps warps).  Inlined: the tabu words must stay in registers
-// (a call would take the array's address and move it to local memory).
-// WIDE: the blend scan also issues its loads two chunks at a time (more
-// registers; used where the kernel has them to spare).
-template <int TW, bool WIDE, int FB = 4>
-__device__ __forceinline__ int fallback_best_reg(const ColonyDev &c, int cur,
-                                                 const uint32_t (&tw)[TW], const AntCtx &a,
-                                                 int lane) {
+// The tabu list of the step loop: in registers for up to 2048 cities, else as
+// TW * 32 words of shared memory (TW shuffles and selects a lookup cost more
+// there than one load).
+template <int TW>
+struct StepTabu {
+  static constexpr bool kShared = TW > 2;
+  uint32_t tw[kShared ? 1 : TW];
+  uint32_t *words;
+  __device__ __forceinline__ void clear(int lane) {
+    if constexpr (kShared) {
+#pragma unroll
+      for (int t = 0; t < TW; t++) words[t * 32 + lane] = 0u;
+      __syncwarp();
+    } else {
+#pragma unroll
+      for (int t = 0; t < TW; t++) tw[t] = 0u;
+    }
+  }
+  // Every lane takes part; an id past the list (the -1 of a row's padding)
+  // gives either answer, its weight is 0.
+  __device__ __forceinline__ bool visited(int id) const {
+    uint32_t v;
+    if constexpr (kShared) v = words[(id >> 5) & (TW * 32 - 1)];
+    else v = reg_word(tw, id & 0xffff);
+    return (v >> (id & 31)) & 1u;
+  }
+  __device__ __forceinline__ void mark(int city, int lane) {
+    if constexpr (kShared) {
+      if (lane == 0) words[city >> 5] |= 1u << (city & 31);
+      __syncwarp();
+    } else {
+      reg_mark(tw, city, lane);
+    }
+  }
+  // The words as registers (the fallback's layout).
+  __device__ __forceinline__ void words_of(uint32_t (&out)[TW], int lane) const {
+#pragma unroll
+    for (int t = 0; t < TW; t++) {
+      if constexpr (kShared) out[t] = words[t * 32 + lane];
+      else out[t] = tw[t];
+    }
+  }
+};
+
+// x plus the values of the lanes before it, up to lane - 2 o + 1, in its
+// segment of W lanes: one level of an inclusive scan.
+template <int W>
+__device__ __forceinline__ float scan_level(float x, int o) {
+  asm("{\n\t.reg .f32 y;\n\t.reg .pred p;\n\t"
+      "shfl.sync.up.b32 y|p, %0, %1, %2, 0xffffffff;\n\t"
+      "@p add.f32 %0, %0, y;\n\t}"
+      : "+f"(x)
+      : "r"(o), "n"((32 - W) << 8));
+  return x;
+}
+
+// The best-choice fallback over the whole row: the unvisited city with the
+// largest choice value (a blending ant: its blended weight), lowest index on
+// ties, -1 if there is none.  Weights are non-negative, so their bits order
+// like they do, and a visited city's are masked to 0: a lane keeps the
+// largest of its cities chunk by chunk (128 cities, four a lane, the chunk's
+// four values kept with it), one warp maximum gives the value and one warp
+// minimum the lowest city that has it.  Four chunks are loaded ahead of the
+// four being compared: about 24 lines of a warp are in flight at once (a
+// seventh 512-byte load waits for the first to return), so more would not
+// help.  A row whose largest value is 0 or NaN goes to fallback_rest, which
+// tells an unvisited zero from a visited city and skips NaNs.
+template <int TW>
+struct TwPack {
+  uint32_t w[TW];
+};
+
+// One lane's four weights at cities j4 .. j4 + 3 (j4 < n: inside the row's
+// pitch; padding has eta 0, so weight 0).
+__device__ __forceinline__ uint4 fallback_load(const ColonyDev &c, size_t row, int j4,
+                                               const AntCtx &a) {
+  uint4 q = make_uint4(0u, 0u, 0u, 0u);
+  if (j4 >= c.n) return q;
+  if (!a.blend) return __ldcg(reinterpret_cast<const uint4 *>(c.choice + row + j4));
+  const float4 t = __ldcg(reinterpret_cast<const float4 *>(c.tau + row + j4));
+  const float4 e = __ldg(reinterpret_cast<const float4 *>(c.eta + row + j4));
+  q.x = __float_as_uint(blend_fitness(t.x, e.x, a.meanc, a.ratio, c.use_alpha, c.alpha));
+  q.y = __float_as_uint(blend_fitness(t.y, e.y, a.meanc, a.ratio, c.use_alpha, c.alpha));
+  q.z = __float_as_uint(blend_fitness(t.z, e.z, a.meanc, a.ratio, c.use_alpha, c.alpha));
+  q.w = __float_as_uint(blend_fitness(t.w, e.w, a.meanc, a.ratio, c.use_alpha, c.alpha));
+  return q;
+}
+
+// The tabu word that holds cities j4 .. j4 + 3 (j4 a multiple of four, lane
+// l's at 128 t + 4 l), shifted so that they are its low bits.
+template <int TW>
+__device__ __forceinline__ uint32_t fallback_bits(const TwPack<TW> &p, int t, int lane) {
+  const uint32_t v = __shfl_sync(kFull, tw_pick(p.w, t >> 3), (t * 4 + (lane >> 3)) & 31);
+  return v >> ((lane * 4) & 31);
+}
+
+template <int TW>
+__device__ __noinline__ int fallback_rest(const ColonyDev &c, int cur, TwPack<TW> p, AntCtx a,
+                                          int lane) {
   float bw = -1.0f;
   int bj = -1;
-  const float *crow = c.choice + (size_t)cur * c.ld;
-  const float *trow = c.tau + (size_t)cur * c.ld;
-  const float *erow = c.eta + (size_t)cur * c.ld;
-  if (!a.blend) {
-    // Four independent running maxima, one per float4 component (each sees
-    // its cities in increasing order, so a strict > keeps the lowest index
-    // of a tie), merged below; visited and out-of-range cities enter as -1,
-    // below every weight, so the scan has no branch.
-    float cw[4] = {-1.0f, -1.0f, -1.0f, -1.0f};
-    int cj[4] = {-1, -1, -1, -1};
+  const size_t row = (size_t)cur * c.ld;
+#pragma unroll 1
+  for (int t = 0; t * 128 < c.n; t++) {
+    const int j4 = t * 128 + lane * 4;
+    const uint32_t b = fallback_bits(p, t, lane);
+    const uint4 q = fallback_load(c, row, j4, a);
+    const float v[4] = {__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z),
+                        __uint_as_float(q.w)};
 #pragma unroll
-    for (int t0 = 0; t0 < 8 * TW; t0 += FB) {  // n <= 1024 * TW
-      if (t0 * 128 >= c.n) continue;  // (not break: the loop stays fully unrolled)
-      float4 q[FB];
-#pragma unroll
-      for (int t = 0; t < FB; t++) {
-        const int j4 = (t0 + t) * 128 + lane * 4;  // j4 < n implies j4 + 3 < ld (ld % 32 == 0)
-        q[t] = j4 < c.n ? __ldcg(reinterpret_cast<const float4 *>(crow + j4))
-                        : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r = 0; r < 4; r++)
+      if (!((b >> r) & 1u) && j4 + r < c.n && v[r] > bw) {
+        bw = v[r];
+        bj = j4 + r;
       }
-#pragma unroll
-      for (int t = 0; t < FB; t++) {
-        const int j4 = (t0 + t) * 128 + lane * 4;
-        const uint32_t v =
-            __shfl_sync(kFull, tw_pick(tw, (t0 + t) >> 3), ((t0 + t) * 4 + (lane >> 3)) & 31);
-        const int left = c.n - j4;  // cities of this float4 inside the instance
-        const uint32_t in = left >= 4 ? 0xfu : (left > 0 ? (1u << left) - 1u : 0u);
-        const uint32_t open = ~(v >> (j4 & 31)) & in;
-        const float qq[4] = {q[t].x, q[t].y, q[t].z, q[t].w};
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-          const float x = (open >> r) & 1u ? qq[r] : -1.0f;
-          const bool up = x > cw[r];
-          cw[r] = up ? x : cw[r];
-          cj[r] = up ? j4 + r : cj[r];
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const bool take = cj[r] >= 0 && (bj < 0 || cw[r] > bw || (cw[r] == bw && cj[r] < bj));
-      bw = take ? cw[r] : bw;
-      bj = take ? cj[r] : bj;
-    }
-  } else if (WIDE) {  // aging blend (young ants after convergence): tau and
-                      // eta rows, four 128-city chunks at a time, the same
-                      // four branch-free running maxima
-    float cw[4] = {-1.0f, -1.0f, -1.0f, -1.0f};
-    int cj[4] = {-1, -1, -1, -1};
-#pragma unroll
-    for (int t0 = 0; t0 < 8 * TW; t0 += 4) {  // n <= 1024 * TW
-      if (t0 * 128 >= c.n) continue;
-      float4 tq[4], eq[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const int j4 = (t0 + t) * 128 + lane * 4;
-        const bool in = j4 < c.n;
-        tq[t] = in ? __ldcg(reinterpret_cast<const float4 *>(trow + j4))
-                   : make_float4(0.f, 0.f, 0.f, 0.f);
-        eq[t] = in ? __ldg(reinterpret_cast<const float4 *>(erow + j4))
-                   : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const int j4 = (t0 + t) * 128 + lane * 4;
-        const uint32_t v =
-            __shfl_sync(kFull, tw_pick(tw, (t0 + t) >> 3), ((t0 + t) * 4 + (lane >> 3)) & 31);
-        const int left = c.n - j4;
-        const uint32_t in = left >= 4 ? 0xfu : (left > 0 ? (1u << left) - 1u : 0u);
-        const uint32_t open = ~(v >> (j4 & 31)) & in;
-        const float ta[4] = {tq[t].x, tq[t].y, tq[t].z, tq[t].w};
-        const float ea[4] = {eq[t].x, eq[t].y, eq[t].z, eq[t].w};
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-          const float q = blend_fitness(ta[r], ea[r], a.meanc, a.ratio, c.use_alpha, c.alpha);
-          const float x = (open >> r) & 1u ? q : -1.0f;
-          const bool up = x > cw[r];
-          cw[r] = up ? x : cw[r];
-          cj[r] = up ? j4 + r : cj[r];
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const bool take = cj[r] >= 0 && (bj < 0 || cw[r] > bw || (cw[r] == bw && cj[r] < bj));
-      bw = take ? cw[r] : bw;
-      bj = take ? cj[r] : bj;
-    }
-  } else {  // aging blend, one 128-city chunk per round trip
-    for (int base = 0; base < c.n; base += 128) {
-      const int j4 = base + lane * 4;
-      const int word = j4 >> 5;  // register word >> 5 (uniform), lane word & 31
-      const uint32_t v = __shfl_sync(kFull, tw_pick(tw, word >> 5), word & 31);
-      if (j4 >= c.n) continue;
-      const uint32_t bits = (v >> (j4 & 31)) & 0xfu;
-      if (bits == 0xfu) continue;
-      const float4 t = *reinterpret_cast<const float4 *>(trow + j4);
-      const float4 e = *reinterpret_cast<const float4 *>(erow + j4);
-      const float q[4] = {blend_fitness(t.x, e.x, a.meanc, a.ratio, c.use_alpha, c.alpha),
-                          blend_fitness(t.y, e.y, a.meanc, a.ratio, c.use_alpha, c.alpha),
-                          blend_fitness(t.z, e.z, a.meanc, a.ratio, c.use_alpha, c.alpha),
-                          blend_fitness(t.w, e.w, a.meanc, a.ratio, c.use_alpha, c.alpha)};
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        if (!((bits >> r) & 1u) && j4 + r < c.n && q[r] > bw) {
-          bw = q[r];
-          bj = j4 + r;
-        }
-      }
-    }
   }
   for (int o = 16; o; o >>= 1) {
     const float ow = __shfl_xor_sync(kFull, bw, o);
@@ -499,6 +488,43 @@ __device__ __forceinline__ int fallback_best_reg(const ColonyDev &c, int cur,
     }
   }
   return bj;
+}
+
+template <int TW>
+__device__ __forceinline__ int fallback_scan(const ColonyDev &c, int cur, const TwPack<TW> &p,
+                                             const AntCtx &a, int lane) {
+  constexpr int GR = TW > 2 ? 8 : 4;  // chunks loaded ahead
+  const size_t row = (size_t)cur * c.ld;
+  unsigned best = 0u;
+  int bt = 0;
+  uint4 bq = make_uint4(0u, 0u, 0u, 0u), q[GR], nx[GR];
+#pragma unroll
+  for (int t = 0; t < GR; t++) q[t] = fallback_load(c, row, t * 128 + lane * 4, a);
+#pragma unroll 1
+  for (int t0 = 0; t0 * 128 < c.n; t0 += GR) {
+#pragma unroll
+    for (int t = 0; t < GR; t++) nx[t] = fallback_load(c, row, (t0 + GR + t) * 128 + lane * 4, a);
+    unsigned m[GR];
+#pragma unroll
+    for (int t = 0; t < GR; t++) {
+      const uint32_t b = fallback_bits(p, t0 + t, lane);
+      uint4 &v = q[t];
+      v.x &= ~(uint32_t)((int32_t)(b << 31) >> 31);
+      v.y &= ~(uint32_t)((int32_t)(b << 30) >> 31);
+      v.z &= ~(uint32_t)((int32_t)(b << 29) >> 31);
+      v.w &= ~(uint32_t)((int32_t)(b << 28) >> 31);
+      m[t] = max(max(v.x, v.y), max(v.z, v.w));
+    }
+#pragma unroll
+    for (int t = 0; t < GR; t++)
+      if (m[t] > best) { best = m[t]; bt = t0 + t; bq = q[t]; }
+#pragma unroll
+    for (int t = 0; t < GR; t++) q[t] = nx[t];
+  }
+  const unsigned m = __reduce_max_sync(kFull, best);
+  if (m == 0u || m > 0x7f800000u) return fallback_rest<TW>(c, cur, p, a, lane);
+  const int r = bq.x == m ? 0 : bq.y == m ? 1 : bq.z == m ? 2 : 3;
+  return (int)__reduce_min_sync(kFull, best == m ? (unsigned)(bt * 128 + lane * 4 + r) : ~0u);
 }
 
 // The fallback's second tier: the largest plain choice value among the
@@ -514,8 +540,7 @@ __device__ __forceinline__ int fallback_best_reg(const ColonyDev &c, int cur,
 // candidate table (which may carry a learned prior).
 template <int TW>
 __device__ __forceinline__ int fallback_tier2(const ColonyDev &c, int cur,
-                                              const uint32_t (&tw)[TW], int id, bool vis,
-                                              int lane) {
+                                              const TwPack<TW> &p, int id, bool vis, int lane) {
   constexpr int Q = kTier2 / 32;
   const size_t base = (size_t)cur * kTier2;
   const bool own = lane < c.K && (unsigned)id < (unsigned)c.n && !vis;
@@ -539,40 +564,29 @@ __device__ __forceinline__ int fallback_tier2(const ColonyDev &c, int cur,
 #pragma unroll
   for (int q = 0; q < Q; q++) {
     const int city = (unsigned)id2[q] < (unsigned)c.n ? id2[q] : -1;
-    const bool seen = reg_visited(tw, city < 0 ? 0 : city);  // every lane takes part
+    const int at = city < 0 ? 0 : city;
+    const bool seen = (reg_word(p.w, at) >> (at & 31)) & 1u;  // every lane takes part
     if (city >= 0 && !seen && (v2[q] > bw || (v2[q] == bw && city < bj))) {
       bw = v2[q];
       bj = city;
     }
   }
-  for (int o = 16; o; o >>= 1) {
-    const float ow = __shfl_xor_sync(kFull, bw, o);
-    const int oj = __shfl_xor_sync(kFull, bj, o);
-    if (oj >= 0 && (bj < 0 || ow > bw || (ow == bw && oj < bj))) {
-      bw = ow;
-      bj = oj;
-    }
-  }
-  return bj >= 0 && bw > mo ? bj : -1;
+  // Values are at least 0 where a city was found, so their bits order like
+  // they do; a NaN is never kept above.
+  const unsigned bits = bj >= 0 ? __float_as_uint(bw) + 1u : 0u;
+  const unsigned m = __reduce_max_sync(kFull, bits);
+  const unsigned j = __reduce_min_sync(kFull, m != 0u && bits == m ? (unsigned)bj : ~0u);
+  return m != 0u && __uint_as_float(m - 1u) > mo ? (int)j : -1;
 }
 
-// The whole fallback as a called function (the tabu words by value, so they
-// stay in registers): the step loop that calls it is smaller and needs fewer
-// registers.  Used where that measured faster (the cluster kernel at n =
-// 4096: 1.56 -> 1.52 ms), not in the staged kernel (0.334 -> 0.343 ms).
+// The whole best-choice fallback, as a called function (the tabu words by
+// value, so they stay in registers): its code stays out of the step loop.
 template <int TW>
-struct TwPack {
-  uint32_t w[TW];
-};
-template <int TW, bool WIDE, int FB>
-__device__ __noinline__ int fallback_outline(const ColonyDev &c, int cur, TwPack<TW> p, AntCtx a,
-                                             int lane, int id, bool vis, bool tier_ok) {
-  uint32_t tw[TW];
-#pragma unroll
-  for (int t = 0; t < TW; t++) tw[t] = p.w[t];
+__device__ __noinline__ int fallback_best(const ColonyDev &c, int cur, TwPack<TW> p, AntCtx a,
+                                          int lane, int id, bool vis, bool tier_ok) {
   int next = -1;
-  if (tier_ok && c.t2 > 0) next = fallback_tier2<TW>(c, cur, tw, id, vis, lane);
-  if (next < 0) next = fallback_best_reg<TW, WIDE, FB>(c, cur, tw, a, lane);
+  if (tier_ok && c.t2 > 0) next = fallback_tier2<TW>(c, cur, p, id, vis, lane);
+  if (next < 0) next = fallback_scan<TW>(c, cur, p, a, lane);
   return next;
 }
 
@@ -582,7 +596,6 @@ __device__ __noinline__ int fallback_outline(const ColonyDev &c, int cur, TwPack
 // at the same shared-memory offsets in every CTA), through DSMEM.
 template <int SP>
 struct TableRows {
-  static constexpr bool kOutlineFallback = false;
   const int16_t *ids;
   const float *w;
   const float *mean;
@@ -595,7 +608,6 @@ constexpr int kClusterRows = 1024;  // rows in each CTA's slice
 
 template <int SP>
 struct ClusterRows {
-  static constexpr bool kOutlineFallback = true;
   uint32_t ids, w, mean;  // shared::cta addresses of the slice arrays
   __device__ __forceinline__ static uint32_t owner_addr(uint32_t local, int cur) {
     uint32_t r;
@@ -627,51 +639,59 @@ struct ClusterRows {
 
 // The step loop of one ant; BLEND (the aging fitness blend, fixed for the
 // ant's whole tour) is a template parameter so the loop carries no per-step
-// test of it.  Rows of the staged table are padded to 32 entries with id -1
-// and weight 0, so every lane loads unconditionally.
+// test of it.  Rows are padded to the pitch with id -1 and weight 0, so every
+// lane inside it loads unconditionally.
 //
-// One step, with no data-dependent branch on the common path:
+// The reference adds the row's weights in order, visited ones as 0, into S and
+// picks the first candidate whose running sum exceeds fl(u * S)
+// (src/Colony.cu:801-846).  Sequential float sums of at most 32 non-negative
+// terms lie within 31 * 2^-24 (relative) of the true sums, so sums formed in
+// any other order settle the pick unless the threshold is that close to a
+// running sum.  One step, with no data-dependent branch on the common path:
 //  * lane r holds candidate r: its id and its weight, zeroed when the city is
-//    visited (one __shfl_sync of the owner's tabu word);
-//  * the 32 weights go through a per-warp shared buffer and every lane reads
-//    all of them back with broadcast 16-byte loads;
-//  * lane l forms the reference's sequential prefix s_l = (..(w_0 + w_1) +
-//    ..) + w_l as acc = fma(w_e, incl_e, acc) over e = 0..31 with incl_e = 1
-//    for e <= l and 0 after: w*1 + acc rounds exactly like the reference's
-//    float add, and w*0 + acc = acc, so every lane runs the same 32 FMAs
-//    (zero weights change no non-negative float sum, as in the reference,
-//    which adds them too); each lane also adds all 32 for the full sum S;
-//  * the pick is the first candidate with !(s <= u*S) (src/Colony.cu:833-846):
-//    prefixes never decrease, so the crossing lanes form a suffix of the warp
-//    and the first of them is a ballot + ffs; the crossing candidate always
-//    has a non-zero weight.  No crossing (S = 0, or u*S rounding up to S)
-//    takes the fallback, as the reference does.  An infinite weight (two
-//    cities at distance 0) turns the masked product inf*0 into a NaN prefix
-//    in the lanes before it, where the reference has a finite one, so the
+//    visited;
+//  * a scan within groups of eight lanes (three shuffles), then the groups'
+//    totals in every lane (independent shuffles): the prefix at each lane and
+//    S', within 6 * 2^-24 of the true sums.  Seven independent shuffles in
+//    the place of the three were slower (their selects: 321 us an iteration's
+//    construction at n = m = 1000 against 268), as were the weights through
+//    shared memory and packed FMA chains a lane (310);
+//  * hi, lo = u S' (1 +- E) +- 1e-37, E = 1.02 * 94 * 2^-24 covering both
+//    errors of both sums and the roundings of the bounds (the 1e-37 where
+//    they are not relative any more).  If the first prefix past lo is also
+//    past hi, the reference's sums pass its threshold at that candidate: a
+//    warp minimum of (lane, city) keys finds it and hands over the city;
+//  * otherwise -- a prefix in the window (about 1e-4 of the steps), a sum that
+//    is or may become infinite or NaN, no candidate left -- the reference's
+//    own sums decide: its prefix
+//    at lane l as acc = fma(w_e, incl_e, acc) in order (w*1 + acc rounds like
+//    its float add, w*0 + acc = acc), the pick a ballot + ffs.  An infinite
+//    weight (two cities at distance 0) turns a masked product into a NaN in
+//    the lanes before it, where the reference has a finite prefix, so the
 //    test is written acc > rnd || rnd is NaN: the same as !(s <= rnd) for
-//    every prefix the reference forms (its prefixes are NaN only when a
-//    weight is, and then S and rnd are NaN too), false for the masks' NaNs.
-//    With S = +inf this gives the reference's walk: past the row into the
-//    fallback for rnd = +inf, candidate 0 for rnd = NaN (u = 0).
-// The next row is loaded before the (rare) fallback test resolves.  The
-// uniforms of 32 consecutive steps are computed one per lane and broadcast;
-// the tour positions of the current 32-step block stay in one register per
-// lane and are stored together.
-template <int TW, bool BLEND, int G, bool WIDE, class ROWS, int FB = 4, bool LEAN = false,
-          bool TIER = true>
-__device__ __forceinline__ int staged_steps(const ColonyDev &c, int k, uint32_t akey, int start,
-                                            uint32_t (&tw)[TW], float *wbuf, const ROWS &rows,
-                                            AntCtx a, int lane, int64_t &fallbacks) {
-  constexpr int SP = 4 * G;  // row pitch of the staged table
+//    every prefix the reference forms, false for the masks' NaNs.  With S =
+//    +inf this gives the reference's walk: past the row into the fallback for
+//    rnd = +inf, candidate 0 for rnd = NaN.  No crossing (S = 0, or u*S
+//    rounding up to S) takes the fallback, as the reference does.
+// The next row is loaded before the rare cases resolve.  The uniforms of 32
+// consecutive steps are computed one per lane and broadcast; the tour
+// positions of the current 32-step block stay in one register per lane and
+// are stored together.
+template <int TW, bool BLEND, int G, class ROWS, bool TIER>
+__device__ __forceinline__ void staged_steps(const ColonyDev &c, int k, uint32_t akey, int start,
+                                             StepTabu<TW> &tabu, const ROWS &rows, AntCtx a,
+                                             int lane, int64_t &fallbacks) {
+  constexpr int SP = 4 * G;           // row pitch of the staged table
+  constexpr int NG = (SP + 7) / 8;    // groups of eight lanes that hold candidates
+  constexpr float E = 94 * 6.08e-8f;  // 1.02 * 94 * 2^-24
   const int n = c.n;
   int32_t *trow = c.tours + (size_t)k * c.ld;
-  const float4 *wbuf4 = reinterpret_cast<const float4 *>(wbuf);
-  float incl[SP];
-#pragma unroll
-  for (int e = 0; e < SP; e++) incl[e] = e <= lane ? 1.0f : 0.0f;
-  // Lanes past the pitch repeat the last entry: their prefix equals the full
-  // sum, so they are never the first crossing.
-  const int lr = lane < SP ? lane : SP - 1;
+  // Lanes past the pitch hold no candidate: they read the last entry and
+  // carry weight 0, so they are never the first past the threshold.
+  const bool in_row = lane < SP;
+  const int lr = in_row ? lane : SP - 1;
+  const bool g1 = lane >= 8, g2 = lane >= 16, g3 = lane >= 24;
+  const unsigned lane_key = (unsigned)lane << 16;
   int cur = start;
   int id = rows.id(cur, lr);
   float wraw = BLEND ? 0.0f : rows.weight(cur, lr);
@@ -683,6 +703,7 @@ __device__ __forceinline__ int staged_steps(const ColonyDev &c, int k, uint32_t 
 #pragma unroll 1
     for (int x = xb == 0 ? 1 : xb; x < xe; x++) {
       const float u = __shfl_sync(kFull, ublk, x & 31);
+      const float uhi = u * (1.0f + E), ulo = u * (1.0f - E);
       float w = wraw;
       if (BLEND) {
         a.meanc = rows.row_mean(cur);  // every lane: the fallback scan uses it too
@@ -692,63 +713,62 @@ __device__ __forceinline__ int staged_steps(const ColonyDev &c, int k, uint32_t 
                        : 0.0f;
       }
       // Padding entries (id -1) carry weight 0, so their tabu lookup result
-      // is irrelevant; every lane must take part in the shuffle.
-      const bool vis = reg_visited(tw, id & 0xffff);
-      if (vis) w = 0.0f;
-      wbuf[lane] = w;
-      __syncwarp();
-      // Two independent chains: this lane's prefix and the full sum S (the
-      // second fills the first's latency gaps and saves a broadcast).  LEAN
-      // (launches with many warps a scheduler, bound by issue rather than by
-      // one ant's latency): S is lane 31's prefix -- the same adds in the
-      // same order -- broadcast, for 4G fewer instructions a step.
-      float acc = 0.0f, sum = 0.0f;
-#pragma unroll
-      for (int g = 0; g < G; g++) {
-        const float4 p = wbuf4[g];
-        acc = __fmaf_rn(p.x, incl[4 * g + 0], acc);
-        if constexpr (!LEAN) sum = __fadd_rn(sum, p.x);
-        acc = __fmaf_rn(p.y, incl[4 * g + 1], acc);
-        if constexpr (!LEAN) sum = __fadd_rn(sum, p.y);
-        acc = __fmaf_rn(p.z, incl[4 * g + 2], acc);
-        if constexpr (!LEAN) sum = __fadd_rn(sum, p.z);
-        acc = __fmaf_rn(p.w, incl[4 * g + 3], acc);
-        if constexpr (!LEAN) sum = __fadd_rn(sum, p.w);
-      }
-      if constexpr (LEAN) sum = __shfl_sync(kFull, acc, 31);
-      const float rnd = __fmul_rn(u, sum);
-      // The reference's !(s <= rnd), with the mask's NaNs (inf*0) left out.
-      const unsigned hit = __ballot_sync(kFull, acc > rnd || rnd != rnd);
-      int next = __shfl_sync(kFull, id, (__ffs(hit) - 1) & 31);
-      // The next row, loaded before the fallback test resolves (an in-range
-      // stand-in keeps the loads inside the table) and reloaded if the
-      // fallback picks the city.
-      const int nx = (unsigned)next < (unsigned)n ? next : 0;
+      // is irrelevant; every lane must take part in it.
+      const bool vis = tabu.visited(id);
+      if (vis || !in_row) w = 0.0f;
+      float p = scan_level<8>(w, 1);
+      p = scan_level<8>(p, 2);
+      p = scan_level<8>(p, 4);
+      const float T0 = __shfl_sync(kFull, p, 7), T1 = __shfl_sync(kFull, p, 15);
+      float T2 = 0.0f, T3 = 0.0f;
+      if (NG > 2) T2 = __shfl_sync(kFull, p, 23);
+      if (NG > 3) T3 = __shfl_sync(kFull, p, 31);
+      float S = T0 + T1;
+      if (NG > 3) S += T2 + T3;
+      else if (NG > 2) S += T2;
+      if (g1) p += T0;
+      if (g2) p += T1;
+      if (NG > 3 && g3) p += T2;
+      const float hi = __fmaf_rn(uhi, S, 1e-37f), lo = __fmaf_rn(ulo, S, -1e-37f);
+      // The first lane past lo; its city, or 0xffff (as when there is no such
+      // lane) if it is inside the window.
+      const unsigned city = p > hi ? (unsigned)(id & 0xffff) : 0xffffu;
+      const unsigned key = p > lo ? lane_key | city : ~0u;
+      int next = (int)(__reduce_min_sync(kFull, key) & 0xffffu);
+      // The next row, loaded before the rare cases resolve (an in-range
+      // stand-in keeps the loads inside the table) and reloaded after them.
+      const int nx = min(next, n - 1);
       int id_next = rows.id(nx, lr);
       float w_next = BLEND ? 0.0f : rows.weight(nx, lr);
-      if (hit == 0u || (unsigned)next >= (unsigned)n) {
-        if (hit != 0u) {  // a candidate id outside the instance: recorded, not used
-          ok = false;
-        } else if (c.fallback == ACO_FALLBACK_BEST) {
-          if (!BLEND && a.blend) a.meanc = rows.row_mean(cur);  // pre-blended table
-          next = -1;
-          if constexpr (ROWS::kOutlineFallback) {
-            TwPack<TW> pk;
-#pragma unroll
-            for (int t = 0; t < TW; t++) pk.w[t] = tw[t];
-            next = fallback_outline<TW, WIDE, FB>(c, cur, pk, a, lane, id, vis,
-                                                  TIER && !BLEND && !a.blend);
-          } else {
-            if (TIER && !BLEND && !a.blend && c.t2 > 0)
-              next = fallback_tier2<TW>(c, cur, tw, id, vis, lane);
-            if (next < 0) next = fallback_best_reg<TW, WIDE, FB>(c, cur, tw, a, lane);
+      if (next >= n || !(S <= 3e38f)) {
+        unsigned hit = 0u;
+        if (S != 0.0f) {  // the reference's own sums (header)
+          float ra = 0.0f, rs = 0.0f;
+#pragma unroll 4
+          for (int e = 0; e < SP; e++) {
+            const float we = __shfl_sync(kFull, w, e);
+            ra = __fmaf_rn(we, e <= lane ? 1.0f : 0.0f, ra);
+            rs = __fadd_rn(rs, we);
           }
-        } else {  // select_local_best on a full row of at most 32 cities (k == n)
-          const unsigned um = __ballot_sync(kFull, lane < c.K && id >= 0 && !vis);
-          next = um ? __shfl_sync(kFull, id, 31 - __clz(um)) : -1;
+          const float rnd = __fmul_rn(u, rs);
+          hit = __ballot_sync(kFull, ra > rnd || rnd != rnd);
+          next = __shfl_sync(kFull, id, (__ffs(hit) - 1) & 31);
         }
-        fallbacks += hit == 0u;
-        if (next < 0 || next >= n) ok = false;  // no unvisited city, or a bad id
+        if (hit != 0u) {
+          if ((unsigned)next >= (unsigned)n) ok = false;  // recorded, not used
+        } else {
+          fallbacks++;
+          if (c.fallback == ACO_FALLBACK_BEST) {
+            if (!BLEND && a.blend) a.meanc = rows.row_mean(cur);  // pre-blended table
+            TwPack<TW> pk;
+            tabu.words_of(pk.w, lane);
+            next = fallback_best<TW>(c, cur, pk, a, lane, id, vis, TIER && !BLEND && !a.blend);
+          } else {  // select_local_best on a full row of at most 32 cities (k == n)
+            const unsigned um = __ballot_sync(kFull, lane < c.K && id >= 0 && !vis);
+            next = um ? __shfl_sync(kFull, id, 31 - __clz(um)) : -1;
+          }
+          if (next < 0 || next >= n) ok = false;  // no unvisited city, or a bad id
+        }
         if (!ok) {
           if (lane == 0) atomicOr(&c.st->error, kErrCheck);
           break;
@@ -756,7 +776,7 @@ __device__ __forceinline__ int staged_steps(const ColonyDev &c, int k, uint32_t 
         id_next = rows.id(next, lr);
         w_next = BLEND ? 0.0f : rows.weight(next, lr);
       }
-      reg_mark(tw, next, lane);
+      tabu.mark(next, lane);
       tpos = lane == (x & 31) ? next : tpos;
       cur = next;
       id = id_next;
@@ -764,22 +784,20 @@ __device__ __forceinline__ int staged_steps(const ColonyDev &c, int k, uint32_t 
     }
     if (xb + lane < xe) trow[xb + lane] = tpos;
   }
-  return cur;
 }
 
 // The tour of one valid ant once its blend context is known: placement,
 // the step loop (BLEND: the aging fitness blend of every candidate per step;
 // otherwise the weights come blended, or plain, from the table), then the
 // integer length and the transposed successor/predecessor lists.
-template <int TW, int G, bool BLEND, bool WIDE, class ROWS, int FB = 4, bool LEAN = false,
-          bool TIER = true>
-__device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, float *wbuf,
+template <int TW, int G, bool BLEND, class ROWS, bool TIER = true>
+__device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, uint32_t *words,
                                 const ROWS &rows, AntCtx a, int lane) {
   const int n = c.n;
   int32_t *trow = c.tours + (size_t)k * c.ld;
-  uint32_t tw[TW];
-#pragma unroll
-  for (int t = 0; t < TW; t++) tw[t] = 0u;
+  StepTabu<TW> tabu;
+  tabu.words = words;
+  tabu.clear(lane);
 
   // initTour placement (src/Colony.cu:518-520)
   const uint32_t akey = aco_ant_key(c.seed, iter, (uint32_t)k);
@@ -788,11 +806,10 @@ __device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, float 
     if (lane == 0) atomicOr(&c.st->error, kErrCheck);
     start = n - 1;
   }
-  reg_mark(tw, start, lane);
+  tabu.mark(start, lane);
 
   int64_t fallbacks = 0;
-  staged_steps<TW, BLEND, G, WIDE, ROWS, FB, LEAN, TIER>(c, k, akey, start, tw, wbuf, rows, a, lane,
-                                             fallbacks);
+  staged_steps<TW, BLEND, G, ROWS, TIER>(c, k, akey, start, tabu, rows, a, lane, fallbacks);
   __syncwarp();
   // Tour length (order-free integer sum) and the transposed successor /
   // predecessor of every city for the row-owned deposit, one edge per lane;
@@ -823,8 +840,8 @@ __device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, float 
 // One ant with its aging step: updateAntAges (src/Colony.cu:353-364), the
 // cleared tour of an invalid ant (src/Colony.cu:507-510) and the blend
 // decision of compute_fittness (inc/Colony.cuh:21-30).
-template <bool AGING, int TW, int G, class ROWS, int FB = 4, bool LEAN = false, bool TIER = true>
-__device__ void construct_ant_staged(const ColonyDev &c, int k, uint32_t iter, float *wbuf,
+template <bool AGING, int TW, int G, class ROWS, bool TIER = true>
+__device__ void construct_ant_staged(const ColonyDev &c, int k, uint32_t iter, uint32_t *words,
                                      const ROWS &rows, int lane) {
   AntCtx a;
   a.blend = false;
@@ -846,9 +863,9 @@ __device__ void construct_ant_staged(const ColonyDev &c, int k, uint32_t iter, f
     if (a.blend) a.ratio = __fdiv_rn(__int2float_rn(age), __int2float_rn(c.min_ret));
   }
   if (AGING && a.blend)
-    staged_ant_body<TW, G, true, false, ROWS, FB, LEAN, TIER>(c, k, iter, wbuf, rows, a, lane);
+    staged_ant_body<TW, G, true, ROWS, TIER>(c, k, iter, words, rows, a, lane);
   else
-    staged_ant_body<TW, G, false, false, ROWS, FB, LEAN, TIER>(c, k, iter, wbuf, rows, a, lane);
+    staged_ant_body<TW, G, false, ROWS, TIER>(c, k, iter, words, rows, a, lane);
 }
 
 }  // namespace aco

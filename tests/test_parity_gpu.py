@@ -9,7 +9,7 @@ import pytest
 
 import oracle
 import acogpu_gb300 as aco
-from acogpu_gb300 import _abi
+from acogpu_gb300 import _abi, instances
 from helpers import assert_same_state, bits, instance, is_permutation_rows, params, tour_lengths
 
 pytestmark = pytest.mark.gpu
@@ -405,3 +405,48 @@ def test_errors_are_reported_not_fatal():
     g.initialize()
     g.constructSolution()
     g.synchronize()
+
+
+@pytest.mark.parametrize("k", [1, 7, 8, 9, 15, 16, 17, 23, 24, 25, 31, 32])
+@pytest.mark.parametrize("mode", [_abi.ACO_CONSTRUCT_STAGED, _abi.ACO_CONSTRUCT_CLUSTER,
+                                  _abi.ACO_CONSTRUCT_DIRECT])
+def test_step_group_edges_match_oracle(k, mode):
+    """Candidate lists around the eight-lane groups of the step's scan, on every
+    kernel that shares the step loop; a lattice, so that weights repeat and
+    thresholds land on running sums, and few candidates, so that many steps
+    fall back."""
+    side = 14
+    x, y = np.meshgrid(np.arange(side, dtype=np.float32), np.arange(side, dtype=np.float32))
+    d = instances.euc2d_distances(x.ravel(), y.ravel())
+    p = params(num_ants=40, beta=2.0, rho=0.2, cand_k=k, seed=k + mode, **FAST_MODE)
+    p.construct_mode = mode
+    g = aco.Colony(d, params=p, num_ants=40)
+    g.initialize()
+    p.construct_mode = _abi.ACO_CONSTRUCT_AUTO
+    q = oracle.Port(p, d, threads=8)
+    q.initialize()
+    for it in range(3):
+        g.constructSolution()
+        q.iterate()
+        assert_same_state(g, q, ctx=f"k={k} mode={mode} iteration {it}")
+    g.close()
+    q.close()
+
+
+@pytest.mark.parametrize("n", [127, 128, 129, 511, 513, 1024, 1025, 2047, 2049, 4097])
+def test_fallback_scan_edges_match_oracle(n):
+    """The best-choice fallback's scan around its chunks and groups (rank-based
+    system: no second tier), three candidates so that most steps fall back."""
+    x, y, d = instance(n, 900 + n)
+    p = params(num_ants=12, variant=_abi.ACO_RANK_BASED, rank_w=4, beta=2.0, rho=0.2, cand_k=3,
+               seed=n, **FAST_MODE)
+    g = aco.Colony(d, params=p, num_ants=12)
+    g.initialize()
+    q = oracle.Port(p, d, threads=8)
+    q.initialize()
+    for it in range(2):
+        g.constructSolution()
+        q.iterate()
+        assert_same_state(g, q, ctx=f"n={n} iteration {it}")
+    g.close()
+    q.close()
