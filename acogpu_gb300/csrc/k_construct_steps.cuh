@@ -425,10 +425,9 @@ __device__ __forceinline__ float scan_level(float x, int o) {
 // like they do, and a visited city's are masked to 0: a lane keeps the
 // largest of its cities chunk by chunk (128 cities, four a lane, the chunk's
 // four values kept with it), one warp maximum gives the value and one warp
-// minimum the lowest city that has it.  Four chunks are loaded ahead of the
-// four being compared: about 24 lines of a warp are in flight at once (a
-// seventh 512-byte load waits for the first to return), so more would not
-// help.  A row whose largest value is 0 or NaN goes to fallback_rest, which
+// minimum the lowest city that has it.  A group of chunks is loaded ahead of
+// the one being compared: four (n <= 2048; the whole row at n = 1000 takes two
+// groups) or eight (n = 4096: construction 1436 us with four, 1374 with eight).  A row whose largest value is 0 or NaN goes to fallback_rest, which
 // tells an unvisited zero from a visited city and skips NaNs.
 template <int TW>
 struct TwPack {
@@ -490,25 +489,51 @@ __device__ __noinline__ int fallback_rest(const ColonyDev &c, int cur, TwPack<TW
   return bj;
 }
 
-template <int TW>
+// The raw loads of GR chunks from chunk t0 on: choice values, or for a
+// blending ant (BL) tau and eta, blended when they are used -- every load of
+// a group is issued before any is waited for.
+template <bool BL, int GR>
+__device__ __forceinline__ void fallback_group(const ColonyDev &c, size_t row, int t0, int lane,
+                                               uint4 (&q)[GR], uint4 (&e)[GR]) {
+#pragma unroll
+  for (int t = 0; t < GR; t++) {
+    const int j4 = (t0 + t) * 128 + lane * 4;
+    const bool in = j4 < c.n;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    q[t] = in ? __ldcg(reinterpret_cast<const uint4 *>((BL ? c.tau : c.choice) + row + j4)) : zero;
+    if (BL) e[t] = in ? __ldg(reinterpret_cast<const uint4 *>(c.eta + row + j4)) : zero;
+  }
+}
+
+__device__ __forceinline__ uint32_t blend_bits(const ColonyDev &c, uint32_t t, uint32_t e,
+                                               const AntCtx &a) {
+  return __float_as_uint(blend_fitness(__uint_as_float(t), __uint_as_float(e), a.meanc, a.ratio,
+                                       c.use_alpha, c.alpha));
+}
+
+template <int TW, bool BL>
 __device__ __forceinline__ int fallback_scan(const ColonyDev &c, int cur, const TwPack<TW> &p,
                                              const AntCtx &a, int lane) {
-  constexpr int GR = TW > 2 ? 8 : 4;  // chunks loaded ahead
+  constexpr int GR = TW > 2 && !BL ? 8 : 4;  // chunks a group; the next one loaded ahead
   const size_t row = (size_t)cur * c.ld;
   unsigned best = 0u;
   int bt = 0;
-  uint4 bq = make_uint4(0u, 0u, 0u, 0u), q[GR], nx[GR];
-#pragma unroll
-  for (int t = 0; t < GR; t++) q[t] = fallback_load(c, row, t * 128 + lane * 4, a);
+  uint4 bq = make_uint4(0u, 0u, 0u, 0u), q[GR], e[GR], nq[GR], ne[GR];
+  fallback_group<BL, GR>(c, row, 0, lane, q, e);
 #pragma unroll 1
   for (int t0 = 0; t0 * 128 < c.n; t0 += GR) {
-#pragma unroll
-    for (int t = 0; t < GR; t++) nx[t] = fallback_load(c, row, (t0 + GR + t) * 128 + lane * 4, a);
+    fallback_group<BL, GR>(c, row, t0 + GR, lane, nq, ne);
     unsigned m[GR];
 #pragma unroll
     for (int t = 0; t < GR; t++) {
       const uint32_t b = fallback_bits(p, t0 + t, lane);
       uint4 &v = q[t];
+      if (BL) {
+        v.x = blend_bits(c, v.x, e[t].x, a);
+        v.y = blend_bits(c, v.y, e[t].y, a);
+        v.z = blend_bits(c, v.z, e[t].z, a);
+        v.w = blend_bits(c, v.w, e[t].w, a);
+      }
       v.x &= ~(uint32_t)((int32_t)(b << 31) >> 31);
       v.y &= ~(uint32_t)((int32_t)(b << 30) >> 31);
       v.z &= ~(uint32_t)((int32_t)(b << 29) >> 31);
@@ -517,9 +542,16 @@ __device__ __forceinline__ int fallback_scan(const ColonyDev &c, int cur, const 
     }
 #pragma unroll
     for (int t = 0; t < GR; t++)
-      if (m[t] > best) { best = m[t]; bt = t0 + t; bq = q[t]; }
+      if (m[t] > best) {
+        best = m[t];
+        bt = t0 + t;
+        bq = q[t];
+      }
 #pragma unroll
-    for (int t = 0; t < GR; t++) q[t] = nx[t];
+    for (int t = 0; t < GR; t++) {
+      q[t] = nq[t];
+      e[t] = ne[t];
+    }
   }
   const unsigned m = __reduce_max_sync(kFull, best);
   if (m == 0u || m > 0x7f800000u) return fallback_rest<TW>(c, cur, p, a, lane);
@@ -586,7 +618,9 @@ __device__ __noinline__ int fallback_best(const ColonyDev &c, int cur, TwPack<TW
                                           int lane, int id, bool vis, bool tier_ok) {
   int next = -1;
   if (tier_ok && c.t2 > 0) next = fallback_tier2<TW>(c, cur, p, id, vis, lane);
-  if (next < 0) next = fallback_scan<TW>(c, cur, p, a, lane);
+  if (next < 0)
+    next = a.blend ? fallback_scan<TW, true>(c, cur, p, a, lane)
+                   : fallback_scan<TW, false>(c, cur, p, a, lane);
   return next;
 }
 
