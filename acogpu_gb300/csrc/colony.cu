@@ -411,6 +411,7 @@ int enqueue_iteration(aco_colony *c) {
 int read_matrix_f32(aco_colony *c, const float *src, int cols, int ldsrc, float *out) {
   if (!out) return fail(c, ACO_ERR_INVALID_ARGUMENT, "null output");
   if (!c->initialized) return fail(c, ACO_ERR_NOT_INITIALIZED, "colony not initialized");
+  prefault(out, (size_t)c->n * cols * 4);
   ACO_CUDA(c, cudaMemcpy2DAsync(out, (size_t)cols * 4, src, (size_t)ldsrc * 4, (size_t)cols * 4,
                                 c->n, cudaMemcpyDeviceToHost, c->stream),
            "read matrix");
@@ -836,6 +837,7 @@ const char *aco_colony_name(const aco_colony *c) {
 int aco_colony_get_best_tour(aco_colony *c, int32_t *out) {
   if (!c || !out) return ACO_ERR_INVALID_ARGUMENT;
   if (!c->initialized) return fail(c, ACO_ERR_NOT_INITIALIZED, "colony not initialized");
+  prefault(out, (size_t)c->n * 4);
   ACO_CUDA(c, cudaMemcpyAsync(out, c->gbtour, (size_t)c->n * 4, cudaMemcpyDeviceToHost, c->stream),
            "read best tour");
   ACO_CUDA(c, cudaStreamSynchronize(c->stream), "synchronize");
@@ -881,6 +883,7 @@ int aco_colony_read_candidate_heuristic(aco_colony *c, float *out) {
 
 int aco_colony_read_distances(aco_colony *c, int32_t *out) {
   if (!c || !out) return ACO_ERR_INVALID_ARGUMENT;
+  prefault(out, (size_t)c->n * c->n * 4);
   ACO_CUDA(c, cudaMemcpy2DAsync(out, (size_t)c->n * 4, c->dist, (size_t)c->ld * 4,
                                 (size_t)c->n * 4, c->n, cudaMemcpyDeviceToHost, c->stream),
            "read distances");
@@ -891,6 +894,7 @@ int aco_colony_read_distances(aco_colony *c, int32_t *out) {
 int aco_colony_read_tours(aco_colony *c, int32_t *out) {
   if (!c || !out) return ACO_ERR_INVALID_ARGUMENT;
   if (!c->initialized) return fail(c, ACO_ERR_NOT_INITIALIZED, "colony not initialized");
+  prefault(out, (size_t)c->m * c->n * 4);
   ACO_CUDA(c, cudaMemcpy2DAsync(out, (size_t)c->n * 4, c->tours, (size_t)c->ld * 4,
                                 (size_t)c->n * 4, c->m, cudaMemcpyDeviceToHost, c->stream),
            "read tours");
@@ -901,6 +905,7 @@ int aco_colony_read_tours(aco_colony *c, int32_t *out) {
 int aco_colony_read_tour_lengths(aco_colony *c, int64_t *out) {
   if (!c || !out) return ACO_ERR_INVALID_ARGUMENT;
   if (!c->initialized) return fail(c, ACO_ERR_NOT_INITIALIZED, "colony not initialized");
+  prefault(out, (size_t)c->m * 8);
   ACO_CUDA(c, cudaMemcpyAsync(out, c->len, (size_t)c->m * 8, cudaMemcpyDeviceToHost, c->stream),
            "read lengths");
   ACO_CUDA(c, cudaStreamSynchronize(c->stream), "synchronize");

@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <string>
 #include <vector>
@@ -63,6 +65,26 @@ struct aco_colony {
   bool state_fresh = false;
   std::string err;
 };
+
+// Maps the pages of a host buffer that a device-to-host copy is about to
+// fill.  A caller's fresh buffer has no pages yet, and on this machine the
+// copy then takes a fault from the GPU's side for each of them, about 70 us a
+// 64 KB page: 64 MB (the pheromone at n = 4096) took 58.6 ms to read, and 2.3
+// ms with the pages populated first; 2.4 MB 2.7 and 0.11 ms.  Buffers below
+// 128 KB mostly come from a heap that is mapped already (malloc maps larger
+// ones afresh), and the call costs about 3 us.  The buffer's contents do not
+// change; where the kernel cannot populate (EINVAL, or memory that is not the
+// process's) the copy runs as before.
+inline void prefault(void *p, size_t bytes) {
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+  static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+  if (!p || bytes < (128u << 10)) return;
+  const uintptr_t a = (uintptr_t)p / page * page;
+  const uintptr_t e = ((uintptr_t)p + bytes + page - 1) / page * page;
+  madvise(reinterpret_cast<void *>(a), e - a, MADV_POPULATE_WRITE);
+}
 
 // Every call that enqueues work on a colony (or rewrites its state) marks the
 // cached state block stale.
