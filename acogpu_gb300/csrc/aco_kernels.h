@@ -92,6 +92,9 @@ cudaError_t launch_construct_cluster(const ColonyDev &c, int grid, int warps, in
 // aging, launch_construct_rows runs the aging plan first (two launches).
 constexpr int kRowsMaxCities = 8192;
 constexpr int kRowsMaxAnts = 11;
+// Rows that the long-row kernel sums in city order (full rows longer than one
+// chunk of 128); their matrices' pitch is a multiple of 128.
+__host__ __device__ constexpr bool rows_city_order(int n, int K) { return K == n && n > 128; }
 cudaError_t launch_construct_rows(const ColonyDev &c, int grid, int ants, cudaStream_t s);
 // max_n: the batch's largest instance (it picks the visited mask's size).
 int batch_rows_blocks_per_sm(int ants, int max_n, bool aging);

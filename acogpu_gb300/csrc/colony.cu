@@ -230,7 +230,7 @@ int create_common(const aco_params *params, int32_t n, aco_colony **out, aco_col
   c->n = n;
   c->m = params->num_ants;
   c->K = (params->cand_k <= 0 || params->cand_k >= n) ? n : params->cand_k;
-  c->ld = round_up(n, 32);
+  c->ld = round_up(n, rows_city_order(n, c->K) && n <= kRowsMaxCities ? 128 : 32);
   c->ldk = c->K <= 32 ? staged_pitch(c->K) : round_up(c->K, 32);
   c->ldm = round_up(c->m + 1, 32);
   c->apb = params->ants_per_block > 0 ? params->ants_per_block : 4;

@@ -28,30 +28,35 @@
 //     2^-24), and the other way round for i - 1; sequential sums never
 //     decrease, so the crossing is unique).  The 1.02 covers the products of
 //     errors (E < 2.1e-3 at c = 8192) and the 8 the roundings of u S' and of
-//     the bounds; a 1e-44 is added for thresholds in the subnormal range;
+//     the bounds; 1e-37 is added for thresholds in the subnormal range;
 //  4. otherwise -- u S' within the bound of a prefix, or a sum that is not
 //     finite -- forms the reference's running sums themselves (rows_exact).
 //     u falls into such a window in 0.1 to 3 % of the steps at n = 1000 (the
 //     most with fresh pheromone on uniform instances, fewer later, when most
-//     weights are smaller than the window) and in 5 to 8 % at n = 2392.
+//     weights are smaller than the window) and in 5 to 8 % at n = 2392.  The
+//     walk in 256-entry chunks with a scan in each took 2392 cities from 4.4
+//     ms an iteration (128-entry chunks) to 4.0.
 //
 // Full rows without a learned prior are summed in city order, straight from
 // the choice matrix: city 128 j + 4 l + t belongs to lane l, whose open
-// (unvisited) cities are the bits 4 j + t of one register, so masking a
-// weight is one predicated add with no lookup and no city ids, and a lane's
-// four cities are not loaded once all are visited.  Other rows (k < n, the
-// candidate heuristic carrying a prior, at most one chunk) are summed in row
-// order.  Only the prefixes need ids, and usually one chunk of 128: the
-// weights fall off with the distance (97 % of the steps at n = 1000).
+// (unvisited) cities are the bits 4 j + t of one word, so masking needs no
+// lookup and no city ids.  Other rows (k < n, the candidate heuristic carrying
+// a prior, at most one chunk) are summed in row order.  Only the prefixes need
+// ids, and usually one chunk of 128: the weights fall off with the distance
+// (97 % of the steps at n = 1000).  hi and lo, u S' (1 +- E) +- 1e-37, are
+// compared with all prefixes; one warp minimum over (lane, city) keys finds
+// the first past lo, with no city in it if it is not past hi.
 //
-// What bounds it: one ant's step is a chain of an L2 round trip and some
-// fifteen shuffles; a batch keeps 32 independent warps an SM in flight and
-// is bound by issue (about 320 instructions a step).  No warp waits for
-// another.  The former kernel compacted every row into shared memory for a
-// warp of the CTA that ran the sequential sums of all its ants in lockstep:
-// a pass of 5 iterations of 8 x n = 1000 (m = 1000, setup included) took 95.7
-// ms with it and 24.6 with this one, 10 iterations at n = 1501, k = 64 42.4
-// and 12.6 ms, 2 iterations at n = 2392, m = 512 35.3 and 22.6 ms.
+// What bounds it: one ant's step is a chain of an L2 round trip (365 cycles,
+// 740 for the ten 512-byte loads at n = 1000: beyond about 24 lines of a warp
+// the next wait for the first) and some ten shuffles; a batch keeps 32
+// independent warps an SM in flight, two thirds of its issue slots taken.  No
+// warp waits for another.  The former kernel compacted every row into shared
+// memory for a warp of the CTA that ran the sequential sums of all its ants in
+// lockstep.  Construction per iteration, before and now: n = m = 100 214 and
+// 57 us, n = m = 1000 3019 and 784, n = 2392, m = 512 14.98 and 4.00 ms, n =
+// 1501, k = 64, m = 500 about 3.9 ms and 0.88, the batch of 8 x n = 1000 17.8
+// and 3.6 ms.
 #include "k_construct_steps.cuh"
 
 namespace aco {
@@ -96,20 +101,6 @@ struct RowsChunk {
   uint2 id;
 };
 
-template <bool BLEND>
-__device__ __forceinline__ void rows_load(const ColonyDev &c, int cur, int ch, float4 &w,
-                                          float4 &e, uint2 &id, int lane) {
-  const int p0 = ch * 128 + lane * 4;
-  const size_t off = (size_t)cur * c.ldk + p0;
-  const bool in = p0 < c.K;  // ldk % 4 == 0: the four entries are in the row
-  id = in ? __ldg(reinterpret_cast<const uint2 *>(c.nn16 + off)) : make_uint2(0u, 0u);
-  w = in ? __ldcg(reinterpret_cast<const float4 *>((BLEND ? c.tau_nn : c.choice_nn) + off))
-         : make_float4(0.f, 0.f, 0.f, 0.f);
-  if (BLEND)
-    e = in ? __ldg(reinterpret_cast<const float4 *>(c.eta_nn + off))
-           : make_float4(0.f, 0.f, 0.f, 0.f);
-}
-
 // Padding entries (positions K .. ldk - 1) have choice 0 in the table, and
 // positions past the row load zeros, so their weight is 0 whatever their id;
 // a blended weight is formed inside the row only (p0: the lane's position).
@@ -133,100 +124,217 @@ __device__ __forceinline__ RowsChunk rows_mask(const ColonyDev &c, const uint32_
   return r;
 }
 
-// The open cities of one round (1024 cities) of the choice row at offset
-// `row` (a blending ant: their blended weights): chunks h .. h + JB - 1 of
-// 128 cities, all loads first.  A set bit of `open` lies inside the instance,
-// so a load that is made stays inside the row's pitch.
-template <bool BLEND, int JB>
-__device__ __forceinline__ void rows_round_load(const ColonyDev &c, size_t row, uint32_t open,
-                                                int h, const AntCtx &a, float4 (&q)[JB]) {
+// Packed pairs of floats: two additions or FMAs an instruction, each rounded
+// on its own.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float sum2(f32x2 a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+  return x + y;
+}
+
+// 0/1 masks of the four cities of a nibble of the open-city word, in shared
+// memory.
+struct RowsLut {
+  float4 m[16];
+};
+
+__device__ __forceinline__ void rows_lut_init(RowsLut &lut) {
+  for (int i = threadIdx.x; i < 16; i += blockDim.x)
+    lut.m[i] = make_float4((i & 1) ? 1.f : 0.f, (i & 2) ? 1.f : 0.f, (i & 4) ? 1.f : 0.f,
+                           (i & 8) ? 1.f : 0.f);
+  __syncthreads();
+}
+
+// A lane's masked running sums.  LUT (a single colony, bound by one ant's
+// latency): the mask as four floats from the table, two packed FMAs a chunk
+// -- a predicate would cost a compare, and 13 cycles until its use, for each
+// city: n = m = 1000 844 us an iteration against 1287.  A masked infinity
+// turns into a NaN, and a sum that is not finite goes to the exact path.
+// Otherwise (batches, whose many warps would queue for shared memory)
+// predicated adds, the tests on constant bits of one register: 8 x n = 1000
+// 3.6 ms against 4.0.
+template <bool LUT>
+struct RowsSum;
+
+template <>
+struct RowsSum<true> {
+  f32x2 s[4] = {0ull, 0ull, 0ull, 0ull};
+  // Chunks j0 .. j0 + N - 1 (0 .. 7) of the round that `open` stands for.
+  template <int N>
+  __device__ __forceinline__ void add(const ulonglong2 (&q)[N], uint32_t open, int j0,
+                                      const RowsLut &lut) {
 #pragma unroll
-  for (int j = 0; j < JB; j++) {
-    const size_t off = row + (h + j) * 128;
-    const bool need = (open >> (4 * (h + j))) & 0xfu;
-    q[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (!BLEND) {
-      if (need) q[j] = __ldcg(reinterpret_cast<const float4 *>(c.choice + off));
-    } else if (need) {
-      const float4 t = __ldcg(reinterpret_cast<const float4 *>(c.tau + off));
-      const float4 e = __ldg(reinterpret_cast<const float4 *>(c.eta + off));
-      q[j].x = blend_fitness(t.x, e.x, a.meanc, a.ratio, c.use_alpha, c.alpha);
-      q[j].y = blend_fitness(t.y, e.y, a.meanc, a.ratio, c.use_alpha, c.alpha);
-      q[j].z = blend_fitness(t.z, e.z, a.meanc, a.ratio, c.use_alpha, c.alpha);
-      q[j].w = blend_fitness(t.w, e.w, a.meanc, a.ratio, c.use_alpha, c.alpha);
+    for (int j = 0; j < N; j++) {
+      const unsigned at = (j0 + j == 0 ? open << 4 : open >> (4 * (j0 + j) - 4)) & 0xf0u;
+      const ulonglong2 m = *reinterpret_cast<const ulonglong2 *>(
+          reinterpret_cast<const char *>(lut.m) + at);
+      s[2 * (j & 1)] = fma2(q[j].x, m.x, s[2 * (j & 1)]);
+      s[2 * (j & 1) + 1] = fma2(q[j].y, m.y, s[2 * (j & 1) + 1]);
     }
+  }
+  __device__ __forceinline__ float total() const {
+    return sum2(add2(add2(s[0], s[1]), add2(s[2], s[3])));
+  }
+};
+
+template <>
+struct RowsSum<false> {
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  template <int N>
+  __device__ __forceinline__ void add(const ulonglong2 (&q)[N], uint32_t open, int j0,
+                                      const RowsLut &) {
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      float x, y, z, w;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(q[j].x));
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(z), "=f"(w) : "l"(q[j].y));
+      const int b = 4 * (j0 + j);
+      if (open & (1u << b)) s[0] = __fadd_rn(s[0], x);
+      if (open & (2u << b)) s[1] = __fadd_rn(s[1], y);
+      if (open & (4u << b)) s[2] = __fadd_rn(s[2], z);
+      if (open & (8u << b)) s[3] = __fadd_rn(s[3], w);
+    }
+  }
+  __device__ __forceinline__ float total() const { return (s[0] + s[1]) + (s[2] + s[3]); }
+};
+
+// The fields of a colony that every step reads, held in registers (a batch's
+// descriptors are in shared memory).
+struct RowsView {
+  const float *choice, *choice_nn;
+  const int16_t *nn16;
+  int n, K, ld, ldk;
+};
+
+// The choice values of chunks t0 .. t0 + N - 1 of a row (pointer at this
+// lane's city of chunk 0; the pitch of a colony whose rows are summed in city
+// order is a multiple of 128, so a chunk that holds a city is read whole).
+template <int N>
+__device__ __forceinline__ void rows_fetch(const float *row, int t0, int n, ulonglong2 (&q)[N]) {
+#pragma unroll
+  for (int j = 0; j < N; j++) {
+    q[j] = make_ulonglong2(0ull, 0ull);
+    if ((t0 + j) * 128 < n)  // the same for every lane
+      q[j] = __ldcg(reinterpret_cast<const ulonglong2 *>(row + (t0 + j) * 128));
   }
 }
 
-// Adds them to four running sums, one per float4 component (predicated adds).
-template <int JB>
-__device__ __forceinline__ void rows_round_add(const float4 (&q)[JB], uint32_t open, int h,
-                                               float (&s)[4]) {
-#pragma unroll
-  for (int j = 0; j < JB; j++) {
-    const uint32_t b = open >> (4 * (h + j));
-    if (b & 1u) s[0] = __fadd_rn(s[0], q[j].x);
-    if (b & 2u) s[1] = __fadd_rn(s[1], q[j].y);
-    if (b & 4u) s[2] = __fadd_rn(s[2], q[j].z);
-    if (b & 8u) s[3] = __fadd_rn(s[3], q[j].w);
-  }
+template <bool BLEND>
+__device__ __forceinline__ void rows_load(const ColonyDev &c, const RowsView &v, int cur, int ch,
+                                          float4 &w, float4 &e, uint2 &id, int lane) {
+  const int p0 = ch * 128 + lane * 4;
+  const size_t off = (size_t)cur * v.ldk + p0;
+  const bool in = p0 < v.K;  // ldk % 4 == 0: the four entries are in the row
+  id = in ? __ldg(reinterpret_cast<const uint2 *>(v.nn16 + off)) : make_uint2(0u, 0u);
+  w = in ? __ldcg(reinterpret_cast<const float4 *>((BLEND ? c.tau_nn : v.choice_nn) + off))
+         : make_float4(0.f, 0.f, 0.f, 0.f);
+  if (BLEND)
+    e = in ? __ldg(reinterpret_cast<const float4 *>(c.eta_nn + off))
+           : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+__device__ __forceinline__ RowsView rows_view(const ColonyDev &c) {
+  return RowsView{c.choice, c.choice_nn, c.nn16, c.n, c.K, c.ld, c.ldk};
 }
 
 // This lane's part of the sum over the open cities of `cur`'s row, in city
-// order (d_S: 8 adds a round, then the tree).  PIPE (several rounds, few
-// warps an SM): the next round's loads are issued before this round's adds.
-template <bool R1, bool BLEND, bool PIPE>
-__device__ __forceinline__ float rows_city_sum(const ColonyDev &c, int cur, const uint32_t *mask,
-                                               uint32_t own, const AntCtx &a, int lane) {
-  float s[4] = {0.f, 0.f, 0.f, 0.f};
-  const size_t row = (size_t)cur * c.ld + lane * 4;
-  if constexpr (BLEND) {  // few ants blend: two chunks at a time, fewer registers
+// order (d_S: 4 additions a round, then the tree).  Above one round the loads
+// of the next 512 cities are issued before this 512's additions.
+template <bool R1, bool BLEND, bool LUT>
+__device__ __forceinline__ float rows_city_sum(const ColonyDev &c, const RowsView &v, int cur,
+                                               const uint32_t *mask, uint32_t own,
+                                               const RowsLut &lut, const AntCtx &a, int lane) {
+  const size_t row = (size_t)cur * v.ld + lane * 4;
+  if constexpr (BLEND) {  // few ants blend: one chunk at a time, predicated
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-    for (int r = 0; r * 1024 < c.n; r++) {
-      const uint32_t open = R1 ? own : mask[32 * r + lane];
+    for (int t = 0; t * 128 < c.n; t++) {
+      const uint32_t b = (R1 ? own : mask[32 * (t >> 3) + lane]) >> (4 * (t & 7));
+      if (!(b & 0xfu)) continue;
+      const float4 x = __ldcg(reinterpret_cast<const float4 *>(c.tau + row + t * 128));
+      const float4 e = __ldg(reinterpret_cast<const float4 *>(c.eta + row + t * 128));
+      const float v[4] = {blend_fitness(x.x, e.x, a.meanc, a.ratio, c.use_alpha, c.alpha),
+                          blend_fitness(x.y, e.y, a.meanc, a.ratio, c.use_alpha, c.alpha),
+                          blend_fitness(x.z, e.z, a.meanc, a.ratio, c.use_alpha, c.alpha),
+                          blend_fitness(x.w, e.w, a.meanc, a.ratio, c.use_alpha, c.alpha)};
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if ((b >> q) & 1u) s[q] = __fadd_rn(s[q], v[q]);
+    }
+    return (s[0] + s[1]) + (s[2] + s[3]);
+  } else {
+    const float *p = v.choice + row;
+    RowsSum<LUT> sum;
+    if constexpr (R1) {
+      ulonglong2 q[8];
+      rows_fetch<8>(p, 0, v.n, q);
+      sum.template add<8>(q, own, 0, lut);
+    } else {
+      ulonglong2 q0[4], q1[4];
+      rows_fetch<4>(p, 0, v.n, q0);
 #pragma unroll 1
-      for (int h = 0; h < 8; h += 2) {
-        float4 q[2];
-        const uint32_t o2 = open >> (4 * h);
-        rows_round_load<true, 2>(c, row + (size_t)r * 1024 + h * 128, o2, 0, a, q);
-        rows_round_add<2>(q, o2, 0, s);
+      for (int r = 0; r * 1024 < v.n; r++) {
+        const uint32_t open = mask[32 * r + lane];
+        rows_fetch<4>(p, 8 * r + 4, v.n, q1);
+        sum.template add<4>(q0, open, 0, lut);
+        rows_fetch<4>(p, 8 * r + 8, v.n, q0);
+        sum.template add<4>(q1, open, 4, lut);
       }
     }
-  } else if constexpr (R1) {
-    float4 q[8];
-    rows_round_load<false, 8>(c, row, own, 0, a, q);
-    rows_round_add<8>(q, own, 0, s);
-  } else if constexpr (!PIPE) {
-#pragma unroll 1
-    for (int r = 0; r * 1024 < c.n; r++) {
-      float4 q[8];
-      const uint32_t open = mask[32 * r + lane];
-      rows_round_load<false, 8>(c, row + (size_t)r * 1024, open, 0, a, q);
-      rows_round_add<8>(q, open, 0, s);
-    }
-  } else {
-    const int R = (c.n + 1023) >> 10;
-    float4 q0[8], q1[8];
-    uint32_t o0 = mask[lane], o1 = 0u;
-    rows_round_load<false, 8>(c, row, o0, 0, a, q0);
-#pragma unroll 1
-    for (int r = 0; r < R; r += 2) {
-      o1 = r + 1 < R ? mask[32 * (r + 1) + lane] : 0u;
-      rows_round_load<false, 8>(c, row + (size_t)(r + 1) * 1024, o1, 0, a, q1);
-      rows_round_add<8>(q0, o0, 0, s);
-      o0 = r + 2 < R ? mask[32 * (r + 2) + lane] : 0u;
-      rows_round_load<false, 8>(c, row + (size_t)(r + 2) * 1024, o0, 0, a, q0);
-      rows_round_add<8>(q1, o1, 0, s);
-    }
+    return sum.total();
   }
-  return (s[0] + s[1]) + (s[2] + s[3]);
 }
 
 // ---- the rare paths -------------------------------------------------------------
 
-// The reference's running sums over one chunk of 128 entries (four a lane, in
-// order; visited ones 0): from the sum `s` before it to the sum after it, and
-// in `pos` the first entry whose running sum exceeds `thr`, or -1.
+// One chunk of 256 entries for the exact path, eight a lane in row order.
+template <bool R1, bool BLEND>
+__device__ __forceinline__ void rows_load8(const ColonyDev &c, const RowsView &v, int cur, int ch,
+                                           float4 (&w)[2], float4 (&e)[2], uint4 &id, int lane) {
+  const int p0 = ch * 256 + lane * 8;
+  const size_t off = (size_t)cur * v.ldk + p0;
+  const bool in = p0 < v.K;  // ldk % 8 == 0: the eight entries are in the row
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 *wp = reinterpret_cast<const float4 *>((BLEND ? c.tau_nn : v.choice_nn) + off);
+  id = in ? __ldg(reinterpret_cast<const uint4 *>(v.nn16 + off)) : make_uint4(0u, 0u, 0u, 0u);
+  w[0] = in ? __ldcg(wp) : zero;
+  w[1] = in ? __ldcg(wp + 1) : zero;
+  if (BLEND) {
+    const float4 *ep = reinterpret_cast<const float4 *>(c.eta_nn + off);
+    e[0] = in ? __ldg(ep) : zero;
+    e[1] = in ? __ldg(ep + 1) : zero;
+  }
+}
+
+template <bool R1, bool BLEND>
+__device__ __forceinline__ void rows_mask8(const ColonyDev &c, const uint32_t *mask,
+                                           const float4 (&w)[2], const float4 (&e)[2],
+                                           const uint4 &id, int p0, const AntCtx &a,
+                                           float (&x)[8]) {
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const RowsChunk r = rows_mask<R1, BLEND>(
+        c, mask, w[h], e[h], h ? make_uint2(id.z, id.w) : make_uint2(id.x, id.y), p0 + 4 * h, a);
+#pragma unroll
+    for (int t = 0; t < 4; t++) x[4 * h + t] = r.x[t];
+  }
+}
+
+// The reference's running sums over one such chunk (visited entries 0), from
+// entry `start` on: from the sum `s` before it to the sum after the chunk; THR:
+// only up to the first entry whose running sum exceeds `thr`, in `pos` (-1 if
+// there is none).
 //
 // While the sum stays in one binade, with ulp 2^(e-23), adding w rounds to
 // s + RN(w / ulp) ulp unless w / ulp lies halfway between two integers (then
@@ -237,70 +345,99 @@ __device__ __forceinline__ float rows_city_sum(const ColonyDev &c, int cur, cons
 // time: those that would leave the binade (the scan shows the first), large
 // ones, halfway cases; so is every non-zero entry while s is 0, outside
 // 2^-90 .. 2^100 or not finite.  Each trip ends the chunk or adds one such
-// entry, so there are at most 129.  A row has few of them: about log2(S / the
-// first weight) binade changes, and a halfway case needs a weight within a
-// few bits of the sum.
-__device__ __forceinline__ float rows_walk(const float (&x)[4], float s, float thr, int lane,
-                                           int &pos) {
+// entry, so there are at most 257; most chunks take one, which looks at the
+// chunk's total only.
+template <bool THR>
+__device__ __forceinline__ float rows_walk(const float (&x)[8], int start, float s, float thr,
+                                           int lane, int &pos) {
   pos = -1;
-  int start = 0;
-  for (;;) {
+  float v[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) v[q] = 8 * lane + q >= start ? x[q] : 0.0f;
+#pragma unroll 1
+  for (int trip = 0; trip < 258; trip++) {
     const uint32_t eb = __float_as_uint(s) & 0x7f800000u;
     const bool one = !(s >= 0x1p-90f && s <= 0x1p100f);
-    const float M = __uint_as_float(eb | 0x00400000u);
+    // One entry at a time: every non-zero entry counts as large.
+    const float M = one ? 0.0f : __uint_as_float(eb | 0x00400000u);
+    const float half_base = one ? 0.0f : 0.5f * __uint_as_float(eb);
+    const float half_ulp = one ? -1.0f : __uint_as_float(eb - (24u << 23));
     const float lim = __uint_as_float(eb + 0x00800000u);
-    const float half_base = 0.5f * __uint_as_float(eb);
-    const float half_ulp = __uint_as_float(one ? 0u : eb - (24u << 23));
-    float v[4], t[4];
+    float t[8];
     unsigned ev = 0u;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      v[q] = 4 * lane + q >= start ? x[q] : 0.0f;
-      t[q] = one ? 0.0f : __fsub_rn(__fadd_rn(v[q], M), M);
-      const bool special = one ? v[q] != 0.0f
-                               : !(v[q] < half_base) || fabsf(__fsub_rn(v[q], t[q])) == half_ulp;
-      if (special) {
+    for (int q = 0; q < 8; q++) {
+      t[q] = __fsub_rn(__fadd_rn(v[q], M), M);
+      if (!(v[q] < half_base || v[q] == 0.0f) || fabsf(__fsub_rn(v[q], t[q])) == half_ulp)
         ev |= 1u << q;
-        t[q] = 0.0f;  // only entries before the first special one are used
-      }
     }
-    const float t1 = t[0] + t[1], t2 = t1 + t[2], t3 = t2 + t[3];
-    float incl = t3;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float y = __shfl_up_sync(kFull, incl, o);
-      if (lane >= o) incl += y;
-    }
+    for (int q = 1; q < 8; q++) t[q] += t[q - 1];  // now this lane's running terms
+    float incl = t[7];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) incl = scan_level<32>(incl, o);
+    const float end = s + __shfl_sync(kFull, incl, 31);
+    const bool any = __any_sync(kFull, ev != 0u);
+    if (!any && (one || end < lim) && !(THR && end > thr)) return end;
+    // The first special entry, the first that leaves the binade, the first
+    // past thr.  Terms from a special entry on are not used: they may be
+    // wrong or not finite, and so may what the scan made of them, in later
+    // lanes and later entries only.
     float ex = __shfl_up_sync(kFull, incl, 1);
     if (lane == 0) ex = 0.0f;
-    // Running sums after each entry (before the first special one).
-    const float r[4] = {s + (ex + t[0]), s + (ex + t1), s + (ex + t2), s + (ex + t3)};
     unsigned over = 0u;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      if (!one && r[q] >= lim) ev |= 1u << q;
-      if (r[q] > thr) over |= 1u << q;
+    for (int q = 0; q < 8; q++) {
+      const float r = s + (ex + t[q]);
+      if (!one && r >= lim) ev |= 1u << q;
+      if (THR && r > thr) over |= 1u << q;
     }
-    const unsigned mev = __ballot_sync(kFull, ev != 0u), mov = __ballot_sync(kFull, over != 0u);
-    int ie = 128, io = 128;  // first special entry, first entry past thr
-    if (mev) ie = 4 * (__ffs(mev) - 1) + __ffs(__shfl_sync(kFull, ev, __ffs(mev) - 1)) - 1;
-    if (mov) io = 4 * (__ffs(mov) - 1) + __ffs(__shfl_sync(kFull, over, __ffs(mov) - 1)) - 1;
-    if (io < ie) {
-      pos = io;
-      return s;
+    const int ie = (int)__reduce_min_sync(kFull, ev ? 8 * lane + __ffs(ev) - 1 : 256);
+    if (THR) {
+      const int io = (int)__reduce_min_sync(kFull, over ? 8 * lane + __ffs(over) - 1 : 256);
+      if (io < ie) {
+        pos = io;
+        return s;
+      }
     }
-    if (ie >= 128) return s + __shfl_sync(kFull, incl, 31);
-    const int l = ie >> 2, q = ie & 3;
-    const float before = s + (q == 0 ? ex : ex + (q == 1 ? t[0] : q == 2 ? t1 : t2));
-    const float w = q == 0 ? v[0] : q == 1 ? v[1] : q == 2 ? v[2] : v[3];
-    s = __fadd_rn(__shfl_sync(kFull, before, l), __shfl_sync(kFull, w, l));
-    if (s > thr) {
+    if (ie >= 256) return end;
+    const int l = ie >> 3, q = ie & 7;
+    float before = ex, w = v[0];
+#pragma unroll
+    for (int i = 1; i < 8; i++)
+      if (q == i) {
+        before = ex + t[i - 1];
+        w = v[i];
+      }
+    s = __fadd_rn(s + __shfl_sync(kFull, before, l), __shfl_sync(kFull, w, l));
+    if (THR && s > thr) {
       pos = ie;
       return s;
     }
-    start = ie + 1;
-    if (start >= 128) return s;
+    if (ie == 255) return s;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      if (8 * lane + i <= ie) v[i] = 0.0f;
   }
+  return s;  // not reached: every trip consumes an entry
+}
+
+// The first 64 entries of a row, lanes 0 .. 7, added one after another (most
+// of a row's binade changes and halfway cases are there): all lanes run the
+// same chain on broadcast values.
+template <bool THR>
+__device__ __forceinline__ float rows_head(const float (&x)[8], float thr, int &pos) {
+  float s = 0.0f;
+  pos = -1;
+#pragma unroll
+  for (int l = 0; l < 8; l++) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      s = __fadd_rn(s, __shfl_sync(kFull, x[q], l));
+      if (THR && s > thr && pos < 0) pos = 8 * l + q;
+    }
+  }
+  return s;
 }
 
 // The reference's walk (header): the sum over the row with the running sum at
@@ -312,46 +449,46 @@ __device__ __forceinline__ float rows_walk(const float (&x)[4], float s, float t
 template <bool R1, bool BLEND>
 __device__ __noinline__ int rows_exact(const ColonyDev &c, int cur, const uint32_t *mask, float u,
                                        AntCtx a, int lane) {
-  const int nch = (c.K + 127) >> 7;  // at most 64
-  float s = 0.0f, end0 = 0.0f, end1 = 0.0f;
-  float4 w, e;
-  uint2 id;
+  const RowsView v = rows_view(c);
+  const int nch = (c.K + 255) >> 8;  // at most 32
+  float s = 0.0f, end = 0.0f, x[8];
+  float4 w[2], e[2];
+  uint4 id;
   int pos;
-  rows_load<BLEND>(c, cur, 0, w, e, id, lane);
+  rows_load8<R1, BLEND>(c, v, cur, 0, w, e, id, lane);
 #pragma unroll 1
   for (int ch = 0; ch < nch; ch++) {
-    const RowsChunk r = rows_mask<R1, BLEND>(c, mask, w, e, id, ch * 128 + lane * 4, a);
-    rows_load<BLEND>(c, cur, ch + 1, w, e, id, lane);  // zeros past the row
-    s = rows_walk(r.x, s, INFINITY, lane, pos);
-    if (lane == (ch & 31)) (ch < 32 ? end0 : end1) = s;
+    rows_mask8<R1, BLEND>(c, mask, w, e, id, ch * 256 + lane * 8, a, x);
+    rows_load8<R1, BLEND>(c, v, cur, ch + 1, w, e, id, lane);  // zeros past the row
+    if (ch == 0) s = rows_head<false>(x, 0.0f, pos);
+    s = rows_walk<false>(x, ch == 0 ? 64 : 0, s, 0.0f, lane, pos);
+    if (lane == ch) end = s;
   }
   if (s <= 0.0f) return -1;  // chooseBestNext (src/Colony.cu:776-778)
   const float rnd = __fmul_rn(u, s);
   if (rnd != rnd) {
-    for (int ch = 0; ch < nch; ch++) {
-      rows_load<BLEND>(c, cur, ch, w, e, id, lane);
-      const unsigned ids[4] = {id.x & 0xffffu, id.x >> 16, id.y & 0xffffu, id.y >> 16};
-      int first = -1;
-#pragma unroll
-      for (int t = 3; t >= 0; t--)
-        if (ch * 128 + lane * 4 + t < c.K && rows_open<R1>(mask, ids[t])) first = (int)ids[t];
-      const unsigned m = __ballot_sync(kFull, first >= 0);
-      if (m) return __shfl_sync(kFull, first, __ffs(m) - 1);
+    for (int p0 = 0; p0 < c.K; p0 += 32) {
+      const int p = p0 + lane;
+      const unsigned city = p < c.K ? (unsigned)(uint16_t)c.nn16[(size_t)cur * c.ldk + p] : 0u;
+      const unsigned m = __ballot_sync(kFull, p < c.K && rows_open<R1>(mask, city));
+      if (m) return (int)__shfl_sync(kFull, city, __ffs(m) - 1);
     }
     return -1;
   }
-  const unsigned h0 = __ballot_sync(kFull, lane < nch && end0 > rnd);
-  const unsigned h1 = __ballot_sync(kFull, lane + 32 < nch && end1 > rnd);
-  if (!h0 && !h1) return -1;
-  const int ch = h0 ? __ffs(h0) - 1 : 31 + __ffs(h1);
-  s = 0.0f;
-  if (ch > 0) s = __shfl_sync(kFull, ch - 1 < 32 ? end0 : end1, (ch - 1) & 31);
-  rows_load<BLEND>(c, cur, ch, w, e, id, lane);
-  const RowsChunk r = rows_mask<R1, BLEND>(c, mask, w, e, id, ch * 128 + lane * 4, a);
-  rows_walk(r.x, s, rnd, lane, pos);
+  const unsigned h = __ballot_sync(kFull, lane < nch && end > rnd);
+  if (!h) return -1;
+  const int ch = __ffs(h) - 1;
+  rows_load8<R1, BLEND>(c, v, cur, ch, w, e, id, lane);
+  rows_mask8<R1, BLEND>(c, mask, w, e, id, ch * 256 + lane * 8, a, x);
+  if (ch == 0) {
+    s = rows_head<true>(x, rnd, pos);
+    if (pos < 0) rows_walk<true>(x, 64, s, rnd, lane, pos);
+  } else {
+    rows_walk<true>(x, 0, __shfl_sync(kFull, end, ch - 1), rnd, lane, pos);
+  }
   if (pos < 0) return -1;
-  const unsigned v = (pos & 2) ? id.y : id.x;
-  return (int)__shfl_sync(kFull, (pos & 1) ? v >> 16 : v & 0xffffu, pos >> 2);
+  const unsigned ids = (pos & 4) ? ((pos & 2) ? id.w : id.z) : ((pos & 2) ? id.y : id.x);
+  return (int)__shfl_sync(kFull, (pos & 1) ? ids >> 16 : ids & 0xffffu, pos >> 3);
 }
 
 // The fallback (fallback_city's rules on this file's mask): the last
@@ -416,102 +553,116 @@ __device__ __noinline__ int rows_fallback(const ColonyDev &c, int cur, const uin
 
 constexpr int kRowsAmbiguous = -2;
 
-// Inclusive scan over the warp.
-__device__ __forceinline__ float rows_scan(float x, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float y = __shfl_up_sync(kFull, x, o);
-    if (lane >= o) x += y;
-  }
-  return x;
+// One chunk's prefixes: p[t] = base + the sum of the chunk's entries up to
+// this lane's entry t (at most 10 additions each).  A scan within groups of
+// eight lanes, then the groups' totals in every lane; `total` is base plus the
+// whole chunk.
+__device__ __forceinline__ void rows_prefix(const float (&x)[4], float base, int lane,
+                                            float (&p)[4], float &total) {
+  const float c1 = x[0] + x[1], c2 = c1 + x[2], c3 = c2 + x[3];
+  float g = scan_level<8>(c3, 1);
+  g = scan_level<8>(g, 2);
+  g = scan_level<8>(g, 4);
+  const float T0 = __shfl_sync(kFull, g, 7), T1 = __shfl_sync(kFull, g, 15),
+              T2 = __shfl_sync(kFull, g, 23), T3 = __shfl_sync(kFull, g, 31);
+  float e = __shfl_up_sync(kFull, g, 1, 8);  // the group's entries before this lane
+  if ((lane & 7) == 0) e = 0.0f;
+  float before = base;
+  if (lane >= 8) before += T0;
+  if (lane >= 16) before += T1;
+  if (lane >= 24) before += T2;
+  e += before;
+  p[0] = e + x[0];
+  p[1] = e + c1;
+  p[2] = e + c2;
+  p[3] = e + c3;
+  total = base + ((T0 + T1) + (T2 + T3));
+}
+
+// The sum of a value over the warp, in every lane (five additions).
+__device__ __forceinline__ float rows_warp_sum(float x) {
+  x += __shfl_xor_sync(kFull, x, 1);
+  x += __shfl_xor_sync(kFull, x, 2);
+  x += __shfl_xor_sync(kFull, x, 4);
+  const float a = __shfl_sync(kFull, x, 0), b = __shfl_sync(kFull, x, 8),
+              c = __shfl_sync(kFull, x, 16), d = __shfl_sync(kFull, x, 24);
+  return (a + b) + (c + d);
+}
+
+// The first entry of the chunk whose prefix is past lo: its city, or 0xffff if
+// the prefix is not past hi (inside the window); ~0u if there is none.
+__device__ __forceinline__ unsigned rows_first(const float (&p)[4], uint2 id, float lo, float hi,
+                                               int lane) {
+  unsigned city = p[3] > hi ? id.y >> 16 : 0xffffu;
+  if (p[2] > lo) city = p[2] > hi ? id.y & 0xffffu : 0xffffu;
+  if (p[1] > lo) city = p[1] > hi ? id.x >> 16 : 0xffffu;
+  if (p[0] > lo) city = p[0] > hi ? id.x & 0xffffu : 0xffffu;
+  return __reduce_min_sync(kFull, p[3] > lo ? ((unsigned)lane << 16) | city : ~0u);
 }
 
 // The guarded pick of the header at city `cur` with `cnt` open cities or
 // candidates left: the city, -1 (the weights are all zero: no pick), or
 // kRowsAmbiguous.  `own` is this lane's mask word when R1.  Chunk 0 is
-// loaded with the sum's rows and scanned while the sum is reduced, so the
+// loaded with the sum's rows and scanned before they are waited for, so the
 // common step (the crossing in chunk 0: 97 % of the steps at n = 1000) waits
-// for one L2 round trip and one chain of shuffles.
-template <bool R1, bool BLEND, bool PIPE>
-__device__ __forceinline__ int rows_pick(const ColonyDev &c, int cur, const uint32_t *mask,
-                                         uint32_t own, bool natural, int cnt, float u,
-                                         const AntCtx &a, int lane) {
-  const int nch = (c.K + 127) >> 7;
+// for one L2 round trip, the sum and one warp minimum.
+template <bool R1, bool BLEND, bool LUT>
+__device__ __forceinline__ int rows_pick(const ColonyDev &c, const RowsView &v, int cur,
+                                         const uint32_t *mask, uint32_t own, const RowsLut &lut, bool natural, int cnt,
+                                         float u, const AntCtx &a, int lane) {
+  const int nch = (v.K + 127) >> 7;
   float4 w, e;
   uint2 id;
-  rows_load<BLEND>(c, cur, 0, w, e, id, lane);
-  // d_S + d_P + 8 and the entries of both sums: the error terms but for the
-  // chunk of the crossing.
-  int terms = cnt + 28 + nch;
+  rows_load<BLEND>(c, v, cur, 0, w, e, id, lane);
+  // The entries of the sum, d_S + d_P and 8 (a row of 64 chunks adds at most
+  // 64 to either): the window's terms but for the entries up to the crossing.
+  const int terms = cnt + 28 + nch;
+  float p[4], total, S;
   RowsChunk k;
-  float xs, S, incl;
   if (natural) {
-    S = rows_city_sum<R1, BLEND, PIPE>(c, cur, mask, own, a, lane);
-    terms += (c.n + 1023) >> 10 << 3;
+    const float part = rows_city_sum<R1, BLEND, LUT>(c, v, cur, mask, own, lut, a, lane);
     k = rows_mask<R1, BLEND>(c, mask, w, e, id, lane * 4, a);
-    xs = (k.x[0] + k.x[1]) + (k.x[2] + k.x[3]);
-    incl = xs;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float y = __shfl_up_sync(kFull, incl, o);
-      S += __shfl_xor_sync(kFull, S, o);
-      if (lane >= o) incl += y;
-    }
+    rows_prefix(k.x, 0.0f, lane, p, total);
+    S = rows_warp_sum(part);
   } else {
     k = rows_mask<R1, BLEND>(c, mask, w, e, id, lane * 4, a);
-    xs = (k.x[0] + k.x[1]) + (k.x[2] + k.x[3]);
-    incl = rows_scan(xs, lane);
-    S = 0.0f;
-#pragma unroll 1
-    for (int ch = 1; ch < nch; ch++) {
-      rows_load<BLEND>(c, cur, ch, w, e, id, lane);
-      const RowsChunk q = rows_mask<R1, BLEND>(c, mask, w, e, id, ch * 128 + lane * 4, a);
-      S += (q.x[0] + q.x[1]) + (q.x[2] + q.x[3]);
-    }
+    rows_prefix(k.x, 0.0f, lane, p, total);
+    S = total;
     if (nch > 1) {
-#pragma unroll
-      for (int o = 16; o; o >>= 1) S += __shfl_xor_sync(kFull, S, o);
+      float part = 0.0f;
+#pragma unroll 1
+      for (int ch = 1; ch < nch; ch++) {
+        rows_load<BLEND>(c, v, cur, ch, w, e, id, lane);
+        const RowsChunk q = rows_mask<R1, BLEND>(c, mask, w, e, id, ch * 128 + lane * 4, a);
+        part += (q.x[0] + q.x[1]) + (q.x[2] + q.x[3]);
+      }
+      S += rows_warp_sum(part);
     }
-    S += __shfl_sync(kFull, incl, 31);
   }
-  const float rnd = u * S;
-  float base = 0.0f;
 #pragma unroll 1
   for (int ch = 0;;) {
-    float pe = __shfl_up_sync(kFull, incl, 1);  // prefix before this lane's entries
-    if (lane == 0) pe = base;
-    const float c1 = k.x[0] + k.x[1], c2 = c1 + k.x[2], c3 = c2 + k.x[3];
-    const float p0 = pe + k.x[0], p1 = pe + c1, p2 = pe + c2, p3 = pe + c3;
-    const float E = (float)(terms + min(cnt, 128 * (ch + 1))) * 6.08e-8f;  // 1.02 * 2^-24
-    const unsigned hit = __ballot_sync(kFull, p3 > rnd);
-    if (!(S > 0.0f && S < 1e38f)) return S == 0.0f ? -1 : kRowsAmbiguous;
-    if (hit) {
-      const float hi = __fadd_ru(__fmaf_ru(rnd, E, rnd), 1e-44f);
-      const float lo = __fadd_rd(__fmaf_rd(rnd, -E, rnd), -1e-44f);
-      float above = p0, below = pe;
-      unsigned city = k.id.x & 0xffffu;
-      if (!(p0 > rnd)) { above = p1; below = p0; city = k.id.x >> 16; }
-      if (!(p1 > rnd)) { above = p2; below = p1; city = k.id.y & 0xffffu; }
-      if (!(p2 > rnd)) { above = p3; below = p2; city = k.id.y >> 16; }
-      const int mine = above > hi && below <= lo ? (int)city : kRowsAmbiguous;
-      return __shfl_sync(kFull, mine, __ffs(hit) - 1);
-    }
-    if (++ch >= nch) return kRowsAmbiguous;  // u S' close to S'
-    base = __shfl_sync(kFull, incl, 31);
-    rows_load<BLEND>(c, cur, ch, w, e, id, lane);
+    const float E = (float)(terms + min(cnt, 128 * (ch + 1)) + ch) * 6.08e-8f;  // 1.02 * 2^-24
+    const float hi = __fmaf_rn(u * (1.0f + E), S, 1e-37f);
+    const float lo = __fmaf_rn(u * (1.0f - E), S, -1e-37f);
+    const unsigned first = rows_first(p, k.id, lo, hi, lane);
+    if ((int)(first & 0xffffu) < v.n && S <= 3e38f) return (int)(first & 0xffffu);
+    if (S == 0.0f) return -1;
+    // In the window, a sum that is not finite, or u S' close to S'.
+    if (first != ~0u || !(S <= 3e38f) || ++ch >= nch) return kRowsAmbiguous;
+    rows_load<BLEND>(c, v, cur, ch, w, e, id, lane);
     k = rows_mask<R1, BLEND>(c, mask, w, e, id, ch * 128 + lane * 4, a);
-    xs = (k.x[0] + k.x[1]) + (k.x[2] + k.x[3]);
-    incl = rows_scan(xs, lane) + base;
+    rows_prefix(k.x, total, lane, p, total);
   }
 }
 
 // The tour of one valid ant.
-template <bool R1, bool BLEND, bool PIPE>
-__device__ __forceinline__ void rows_tour(const ColonyDev &c, int k, uint32_t *mask, AntCtx a,
-                                          int lane) {
+template <bool R1, bool BLEND, bool LUT>
+__device__ __forceinline__ void rows_tour(const ColonyDev &c, int k, uint32_t *mask,
+                                          const RowsLut &lut, AntCtx a, int lane) {
+  const RowsView v = rows_view(c);
   const int n = c.n;
   int32_t *trow = c.tours + (size_t)k * c.ld;
-  const bool natural = c.K == n && n > 128 && *c.prior_set == 0;
+  const bool natural = rows_city_order(n, c.K) && *c.prior_set == 0;
   uint32_t own = 0u;
   for (int r = 0; r < (R1 ? 1 : kRowsMaskWords / 32); r++) {
     uint32_t open = 0u;
@@ -543,7 +694,8 @@ __device__ __forceinline__ void rows_tour(const ColonyDev &c, int k, uint32_t *m
     for (int x = xb == 0 ? 1 : xb; x < xe; x++) {
       const float u = __shfl_sync(kFull, ublk, x & 31);
       if (BLEND) a.meanc = c.mean[cur];
-      int next = rows_pick<R1, BLEND, PIPE>(c, cur, mask, own, natural, min(c.K, n - x), u, a, lane);
+      int next = rows_pick<R1, BLEND, LUT>(c, v, cur, mask, own, lut, natural, min(v.K, n - x), u, a,
+                                           lane);
       if (next < 0) {
         if (next == kRowsAmbiguous) next = rows_exact<R1, BLEND>(c, cur, mask, u, a, lane);
         if (next < 0) {
@@ -591,8 +743,9 @@ __device__ __forceinline__ void rows_tour(const ColonyDev &c, int k, uint32_t *m
 // ages; blend ants first, then the other valid ones, then the invalid ones),
 // or ant `pos` without aging.  An invalid ant keeps a cleared tour
 // (src/Colony.cu:507-510).
-template <bool R1, bool AGING, bool PIPE>
-__device__ __forceinline__ void rows_ant(const ColonyDev &c, int pos, uint32_t *mask, int lane) {
+template <bool R1, bool AGING, bool LUT>
+__device__ __forceinline__ void rows_ant(const ColonyDev &c, int pos, uint32_t *mask,
+                                         const RowsLut &lut, int lane) {
   AntCtx a;
   a.blend = false;
   a.ratio = 0.0f;
@@ -610,9 +763,9 @@ __device__ __forceinline__ void rows_ant(const ColonyDev &c, int pos, uint32_t *
     if (a.blend) a.ratio = __fdiv_rn(__int2float_rn(age), __int2float_rn(c.min_ret));
   }
   if (AGING && a.blend)
-    rows_tour<R1, true, PIPE>(c, k, mask, a, lane);
+    rows_tour<R1, true, LUT>(c, k, mask, lut, a, lane);
   else
-    rows_tour<R1, false, PIPE>(c, k, mask, a, lane);
+    rows_tour<R1, false, LUT>(c, k, mask, lut, a, lane);
 }
 
 __host__ __device__ constexpr int rows_words(bool r1) { return r1 ? 32 : kRowsMaskWords; }
@@ -623,11 +776,13 @@ __host__ __device__ constexpr int rows_words(bool r1) { return r1 ? 32 : kRowsMa
 // ... so that an aging colony's idle positions (the last ones) spread over
 // the CTAs.
 template <bool R1, bool AGING>
-__global__ void __launch_bounds__(kRowsMaxAnts * 32) k_construct_rows(const __grid_constant__ ColonyDev c) {
+__global__ void __launch_bounds__(kRowsMaxAnts * 32, 1) k_construct_rows(const __grid_constant__ ColonyDev c) {
   __shared__ uint32_t masks[kRowsMaxAnts][rows_words(R1)];
+  __shared__ RowsLut lut;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  rows_lut_init(lut);
   for (int pos = warp * gridDim.x + blockIdx.x; pos < c.m; pos += gridDim.x * warps)
-    rows_ant<R1, AGING, !R1>(c, pos, masks[warp], lane);
+    rows_ant<R1, AGING, true>(c, pos, masks[warp], lut, lane);
 }
 
 cudaError_t launch_construct_rows(const ColonyDev &c, int grid, int ants, cudaStream_t s) {
@@ -649,15 +804,18 @@ cudaError_t launch_construct_rows(const ColonyDev &c, int grid, int ants, cudaSt
 // Batches: every warp takes (instance, position) items from the work queue
 // (largest instances first) until it is empty, with its own copy of the
 // instance's descriptor; no warp waits for another.
-// Three CTAs of 11 warps an SM (56 registers): the pass named in the header
-// took 32.2 ms at 84 to 108 registers, 26.1 at 80 and 24.6 at 56.
+// 64 registers: 32 warps an SM.  A pass of 5 iterations of 8 x n = 1000 took
+// 23.4 ms, 23.8 at 80 registers, 26.2 at 72 (28 warps), 24.5 at 56 and 23.6 at
+// 48 (spills).
 template <bool R1, bool AGING>
-__global__ void __launch_bounds__(kRowsMaxAnts * 32, 3)
+__global__ void __maxnreg__(64)
     k_batch_construct_rows(const ColonyDev *__restrict__ descs, const int4 *__restrict__ items,
                            int num_items, int *queue_head) {
   __shared__ uint32_t masks[kRowsMaxAnts][rows_words(R1)];
+  __shared__ RowsLut lut;
   __shared__ ColonyDev s_desc[kRowsMaxAnts];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  rows_lut_init(lut);
   int have = -1;
   for (;;) {
     int it = 0;
@@ -675,7 +833,7 @@ __global__ void __launch_bounds__(kRowsMaxAnts * 32, 3)
       have = w.x;
     }
     for (int q = 0; q < w.z; q++)
-      rows_ant<R1, AGING, false>(s_desc[warp], w.y + q, masks[warp], lane);
+      rows_ant<R1, AGING, false>(s_desc[warp], w.y + q, masks[warp], lut, lane);
   }
 }
 
