@@ -716,6 +716,7 @@ __device__ __forceinline__ void rows_tour(const ColonyDev &c, int k, uint32_t *m
   __syncwarp();
   // Integer tour length (order-free) and the transposed successor and
   // predecessor lists of the row-owned deposit, one edge per lane.
+  const bool all_deposit = !ranked_by_epilogue(c);
   int64_t len = 0;
 #pragma unroll 8
   for (int i = lane; i < n; i += 32) {
@@ -723,8 +724,10 @@ __device__ __forceinline__ void rows_tour(const ColonyDev &c, int k, uint32_t *m
     const int b0 = trow[i + 1 == n ? 0 : i + 1];
     if ((unsigned)a0 < (unsigned)n && (unsigned)b0 < (unsigned)n) {
       len += c.dist[(size_t)a0 * c.ld + b0];
-      c.succT[(size_t)a0 * c.ldm + k] = b0;
-      c.predT[(size_t)b0 * c.ldm + k] = a0;
+      if (all_deposit) {
+        c.succT[(size_t)a0 * c.ldm + k] = b0;
+        c.predT[(size_t)b0 * c.ldm + k] = a0;
+      }
     } else {
       ok = false;
     }

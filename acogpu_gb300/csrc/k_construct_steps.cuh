@@ -849,6 +849,7 @@ __device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, uint32
   // predecessor of every city for the row-owned deposit, one edge per lane;
   // unrolled so a lane's distance reads (scattered, from HBM when the L2 is
   // cold) are in flight together.
+  const bool all_deposit = !ranked_by_epilogue(c);
   int64_t len = 0;
 #pragma unroll 8
   for (int i = lane; i < n; i += 32) {
@@ -856,8 +857,10 @@ __device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, uint32
     const int b0 = trow[i + 1 == n ? 0 : i + 1];
     if ((unsigned)a0 < (unsigned)n && (unsigned)b0 < (unsigned)n) {
       len += c.dist[(size_t)a0 * c.ld + b0];
-      c.succT[(size_t)a0 * c.ldm + k] = b0;
-      c.predT[(size_t)b0 * c.ldm + k] = a0;
+      if (all_deposit) {
+        c.succT[(size_t)a0 * c.ldm + k] = b0;
+        c.predT[(size_t)b0 * c.ldm + k] = a0;
+      }
     } else {
       atomicOr(&c.st->error, kErrCheck);
     }

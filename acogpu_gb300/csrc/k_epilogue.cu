@@ -30,35 +30,35 @@ __device__ __forceinline__ bool key_less(const MinKey &a, const MinKey &b) {
   return a.v < b.v || (a.v == b.v && a.k < b.k);
 }
 
-// Block-wide minimum of (v, k), ties to the lower k; k < 0 means "none".
-__device__ MinKey block_min(MinKey x, MinKey *scratch) {
+// Warp-wide minimum of (v, k), v >= 0, ties to the lower k; k < 0 means
+// "none": three 32-bit warp minima (a shuffle tree over the 64-bit pairs took
+// ten shuffles and five compares in a chain).
+__device__ __forceinline__ MinKey warp_min(MinKey x) {
+  const bool some = x.k >= 0;
+  const unsigned h = some ? (unsigned)((uint64_t)x.v >> 32) : ~0u, l = (unsigned)x.v;
+  const unsigned mh = __reduce_min_sync(kFull, h);
+  bool in = some && h == mh;
+  const unsigned ml = __reduce_min_sync(kFull, in ? l : ~0u);
+  in = in && l == ml;
+  const unsigned mk = __reduce_min_sync(kFull, in ? (unsigned)x.k : ~0u);
+  return MinKey{(int64_t)(((uint64_t)mh << 32) | ml), mk == ~0u ? -1 : (int)mk};
+}
+
+// Block-wide minimum, in every thread.  `scratch` holds two sets of 32 words,
+// used in turn, so one barrier a call separates the writes from the reads.
+__device__ MinKey block_min(MinKey x, MinKey *scratch, int &turn) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int o = 16; o; o >>= 1) {
-    MinKey y;
-    y.v = __shfl_xor_sync(kFull, x.v, o);
-    y.k = __shfl_xor_sync(kFull, x.k, o);
-    if (key_less(y, x)) x = y;
-  }
-  if (lane == 0) scratch[warp] = x;
+  MinKey *s = scratch + 32 * (turn & 1);
+  turn++;
+  x = warp_min(x);
+  if (lane == 0) s[warp] = x;
   __syncthreads();
-  if (warp == 0) {
-    MinKey y = lane < (int)(blockDim.x >> 5) ? scratch[lane] : MinKey{0, -1};
-    for (int o = 16; o; o >>= 1) {
-      MinKey z;
-      z.v = __shfl_xor_sync(kFull, y.v, o);
-      z.k = __shfl_xor_sync(kFull, y.k, o);
-      if (key_less(z, y)) y = z;
-    }
-    if (lane == 0) scratch[32] = y;
-  }
-  __syncthreads();
-  MinKey r = scratch[32];
-  __syncthreads();
-  return r;
+  return warp_min(lane < (int)(blockDim.x >> 5) ? s[lane] : MinKey{0, -1});
 }
 
 __device__ void epilogue_body(const ColonyDev &c) {
-  __shared__ MinKey scratch[33];
+  __shared__ MinKey scratch[64];
+  int turn = 0;
   __shared__ uint32_t taken[kMaxRankAnts / 32];
   __shared__ int s_improved, s_best_ant;
   const int tid = threadIdx.x, m = c.m, n = c.n;
@@ -74,7 +74,7 @@ __device__ void epilogue_body(const ColonyDev &c) {
     MinKey y{L, k};
     if (key_less(y, best)) best = y;
   }
-  best = block_min(best, scratch);
+  best = block_min(best, scratch, turn);
   if (tid == 0) {
     st->tours_built += c.aging ? st->num_valid : m;
     int ant = -1;
@@ -113,13 +113,16 @@ __device__ void epilogue_body(const ColonyDev &c) {
     int count = 0;
     const int w = c.rank_w;
     for (int r = 0; r < w - 1; r++) {
-      MinKey b{0, -1};
-      for (int k = tid; k < m; k += kEpiThreads) {
-        if ((c.aging && !c.valid[k]) || ((taken[k >> 5] >> (k & 31)) & 1u)) continue;
-        MinKey y{c.len[k], k};
-        if (key_less(y, b)) b = y;
+      MinKey b = best;  // the first rank is the iteration's best
+      if (r > 0) {
+        b = MinKey{0, -1};
+        for (int k = tid; k < m; k += kEpiThreads) {
+          if ((c.aging && !c.valid[k]) || ((taken[k >> 5] >> (k & 31)) & 1u)) continue;
+          MinKey y{c.len[k], k};
+          if (key_less(y, b)) b = y;
+        }
+        b = block_min(b, scratch, turn);
       }
-      b = block_min(b, scratch);
       if (b.k < 0) break;
       if (tid == 0) {
         taken[b.k >> 5] |= 1u << (b.k & 31);
@@ -129,6 +132,16 @@ __device__ void epilogue_body(const ColonyDev &c) {
       count++;
       __syncthreads();
     }
+    // The deposit's successor / predecessor lists, of the ranked ants only.
+    const int listed = ranked_by_epilogue(c) ? count * n : 0;
+    for (int t = tid; t < listed; t += kEpiThreads) {
+      const int q = t / n, i = t - q * n, k = c.dep_col[q];
+      const int32_t *tour = c.tours + (size_t)k * c.ld;
+      const int a = tour[i], b = tour[i + 1 == n ? 0 : i + 1];
+      c.succT[(size_t)a * c.ldm + k] = b;
+      c.predT[(size_t)b * c.ldm + k] = a;
+    }
+    __syncthreads();
     if (tid == 0) {
       if (st->glob_best < ACO_MAX_DISTANCE) {
         c.dep_col[count] = m;
@@ -158,7 +171,7 @@ __device__ void epilogue_body(const ColonyDev &c) {
         r = MinKey{0, i};
         break;
       }
-    r = block_min(r, scratch);
+    r = block_min(r, scratch, turn);
     if (tid == 0 && r.k >= 0) {
       c.valid[r.k] = 0;
       st->num_valid = st->num_valid - 1;
@@ -173,7 +186,7 @@ __device__ void epilogue_body(const ColonyDev &c) {
           q = MinKey{0, i};
           break;
         }
-      q = block_min(q, scratch);
+      q = block_min(q, scratch, turn);
       if (tid == 0 && q.k >= 0) {
         c.valid[q.k] = 1;
         c.age[q.k] = 0;

@@ -450,3 +450,26 @@ def test_fallback_scan_edges_match_oracle(n):
         assert_same_state(g, q, ctx=f"n={n} iteration {it}")
     g.close()
     q.close()
+
+
+@pytest.mark.parametrize("w,m,n,k,aging", [(1, 40, 60, 16, 0), (2, 40, 60, 0, 1), (32, 40, 60, 16, 1),
+                                           (33, 40, 60, 0, 0), (40, 33, 60, 16, 0),
+                                           (60, 7, 60, 16, 1), (6, 1500, 70, 20, 0)])
+def test_ranked_deposit_lists_match_oracle(w, m, n, k, aging):
+    """Ranks around the count above which the construction kernels write the
+    deposit's lists, more ranks than ants, more ants than the epilogue's
+    threads; the pheromone bit for bit."""
+    x, y, d = instance(n, 950 + w)
+    more = FAST_MODE if k else {}
+    p = params(num_ants=m, variant=_abi.ACO_RANK_BASED, rank_w=w, beta=2.0, rho=0.2, cand_k=k,
+               aging=aging, seed=w, **more)
+    g = aco.Colony(d, params=p, num_ants=m)
+    g.initialize()
+    q = oracle.Port(p, d, threads=8)
+    q.initialize()
+    for it in range(4):
+        g.constructSolution()
+        q.iterate()
+        assert_same_state(g, q, aging=bool(aging), ctx=f"w={w} iteration {it}")
+    g.close()
+    q.close()
