@@ -34,8 +34,9 @@ cudaError_t launch_nn_ref_qsort_smem(const int32_t *dist, int n, int ld, int32_t
                                      ColonyState *st, int max_smem, cudaStream_t s);
 cudaError_t launch_gather_nn_f32(const float *src, int n, int ld, const int32_t *nn, int K,
                                  int ldk, float *dst, cudaStream_t s);
+// stable_lists: the candidate lists are in the order of (distance, city).
 cudaError_t launch_greedy_tau0(const ColonyDev &c, int tau0_mode, float tau0_value,
-                               cudaStream_t s);
+                               bool stable_lists, cudaStream_t s);
 cudaError_t launch_init_colony(const ColonyDev &c, cudaStream_t s);
 // Sets *c.prior_set to whether the candidate heuristic differs from the
 // gathered plain heuristic (a learned prior is installed).

@@ -610,7 +610,8 @@ int init_rest(aco_colony *c) {
   if (c->nn16) ACO_CUDA(c, launch_nn_to_i16(c->nn, n, c->K, c->ldk, c->nn16, c->stream), "nn16");
 
   const ColonyDev d = make_dev(c);
-  ACO_CUDA(c, launch_greedy_tau0(d, c->p.tau0_mode, c->p.tau0, c->stream), "tau0");
+  ACO_CUDA(c, launch_greedy_tau0(d, c->p.tau0_mode, c->p.tau0,
+                                 c->p.nn_order == ACO_NN_STABLE, c->stream), "tau0");
   ACO_CUDA(c, launch_init_colony(d, c->stream), "init");
   ACO_CUDA(c, configure_construct(construct_smem_bytes(n, c->K, c->apb)), "configure construct");
   ACO_CUDA(c, configure_pheromone_rows(c->ld), "configure rows");

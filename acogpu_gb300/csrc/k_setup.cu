@@ -434,13 +434,154 @@ cudaError_t launch_nn_to_i16(const int32_t *nn, int n, int K, int ldk, int16_t *
 }
 
 // ---------------------------------------------------------------- tau0
-// Greedy nearest-neighbour tour from city 0 (lowest index on ties); then tau0
-// by the requested rule.  The reference's greedyDistance is a stub returning
-// 0 (src/Colony.cu:1053-1055) and its tau0 is the constant 1e-6
-// (src/AntSystem.cu:200-203).  One CTA of kGreedyThreads: each step reads the
-// current row once (coalesced, n / kGreedyThreads cities per thread) and takes
-// the block-wide minimum of (distance << 32 | city) over unvisited cities, so
-// a step costs one L2 round trip and two barriers.
+// tau0 from the greedy tour's length C_nn (Dorigo's rules).
+__device__ __forceinline__ void greedy_finish(const ColonyDev &c, int64_t len) {
+  const float cnn = __ll2float_rn(len);
+  float t0;
+  if (c.variant == ACO_RANK_BASED) {
+    const float num = __fmul_rn(__fmul_rn(0.5f, (float)c.rank_w), (float)(c.rank_w - 1));
+    t0 = __fdiv_rn(num, __fmul_rn(c.rho, cnn));
+  } else {
+    t0 = __fdiv_rn((float)c.m, cnn);
+  }
+  c.st->tau0 = t0;
+  c.st->greedy_length = len;
+}
+
+// Greedy nearest-neighbour tour from city 0 (lowest index on ties) on stable
+// candidate lists, which hold each row's cities in the order of (distance,
+// city): the next city is the first unvisited one of the list.  Warp 0 walks
+// the lists, one candidate a lane (the first 32): an id load, a lookup in the
+// tabu bits and one warp minimum a step.  The lists are copied to shared
+// memory when they fit (STAGED), else read from L2.  When a list has no
+// unvisited city left the whole CTA takes the minimum over the row.  The tour
+// stays in shared memory; its length is summed at the end, an edge a thread.
+// One CTA runs alone (16 in a batch's setup), so the step's latency is all
+// there is: n = 1000, k = 30 787 -> 113 us, n = 4096, k = 32 (from L2) 5.43 ->
+// 1.50 ms against the whole-row scan of every step below.
+constexpr int kGreedyNnThreads = 256;
+constexpr size_t kGreedyStageBytes = 160 * 1024;
+
+struct GreedyLayout {
+  size_t tour_off, tabu_off, bytes;
+};
+__host__ __device__ inline GreedyLayout greedy_layout(int n, int ldk, bool staged) {
+  GreedyLayout L;
+  L.tour_off = staged ? ((size_t)n * ldk * 2 + 15) / 16 * 16 : 0;
+  L.tabu_off = L.tour_off + ((size_t)n * 2 + 15) / 16 * 16;
+  L.bytes = L.tabu_off + (size_t)((n + 31) / 32) * 4;
+  return L;
+}
+
+template <bool STAGED>
+__global__ void __launch_bounds__(kGreedyNnThreads) k_greedy_tau0_nn(ColonyDev c) {
+  extern __shared__ __align__(16) unsigned char smem_greedy[];
+  __shared__ unsigned red_d[kGreedyNnThreads / 32], red_j[kGreedyNnThreads / 32];
+  __shared__ unsigned long long red_len[kGreedyNnThreads / 32];
+  __shared__ int s_cur, s_pos;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n = c.n, words = (n + 31) >> 5;
+  const GreedyLayout L = greedy_layout(n, c.ldk, STAGED);
+  int16_t *sids = reinterpret_cast<int16_t *>(smem_greedy);
+  int16_t *tour = reinterpret_cast<int16_t *>(smem_greedy + L.tour_off);
+  uint32_t *tabu = reinterpret_cast<uint32_t *>(smem_greedy + L.tabu_off);
+  if (STAGED)
+    for (int t = tid; t < n * c.ldk / 8; t += kGreedyNnThreads)  // ldk % 8 == 0, or its rest below
+      reinterpret_cast<uint4 *>(sids)[t] = __ldg(reinterpret_cast<const uint4 *>(c.nn16) + t);
+  if (STAGED)
+    for (int t = n * c.ldk / 8 * 8 + tid; t < n * c.ldk; t += kGreedyNnThreads)
+      sids[t] = c.nn16[t];
+  for (int w = tid; w < words; w += kGreedyNnThreads) tabu[w] = w == 0 ? 1u : 0u;
+  if (tid == 0) {
+    tour[0] = 0;
+    s_cur = 0;
+    s_pos = 1;
+  }
+  __syncthreads();
+  const int16_t *ids = STAGED ? sids : c.nn16;
+  const bool cand = lane < c.K && lane < c.ldk;
+  for (int rounds = 0; rounds < n; rounds++) {  // one row scan a round: at most n - 1
+    if (warp == 0) {
+      int cur = s_cur, s = s_pos;
+      while (s < n) {
+        const int id = cand ? (int)ids[(size_t)cur * c.ldk + lane] : -1;
+        const bool open = id >= 0 && !((tabu[id >> 5] >> (id & 31)) & 1u);
+        const unsigned m =
+            __reduce_min_sync(kFull, open ? ((unsigned)lane << 16) | (unsigned)id : ~0u);
+        if (m == ~0u) break;
+        cur = (int)(m & 0xffffu);
+        if (lane == 0) {
+          tabu[cur >> 5] |= 1u << (cur & 31);
+          tour[s] = (int16_t)cur;
+        }
+        __syncwarp();
+        s++;
+      }
+      if (lane == 0) {
+        s_cur = cur;
+        s_pos = s;
+      }
+    }
+    __syncthreads();
+    const int cur = s_cur, s = s_pos;
+    if (s >= n) break;
+    // The row's unvisited minimum of (distance, city).
+    const int32_t *row = c.dist + (size_t)cur * c.ld;
+    unsigned bd = ~0u, bj = ~0u;
+    for (int j = tid; j < n; j += kGreedyNnThreads) {
+      if ((tabu[j >> 5] >> (j & 31)) & 1u) continue;
+      const unsigned d = (unsigned)__ldcg(row + j);
+      if (d < bd) {  // j increases: the lowest index of a tie stays
+        bd = d;
+        bj = (unsigned)j;
+      }
+    }
+    const unsigned wd = __reduce_min_sync(kFull, bd);
+    const unsigned wj = __reduce_min_sync(kFull, bd == wd ? bj : ~0u);
+    if (lane == 0) {
+      red_d[warp] = wd;
+      red_j[warp] = wj;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const bool in = lane < kGreedyNnThreads / 32;
+      const unsigned d = in ? red_d[lane] : ~0u, j = in ? red_j[lane] : ~0u;
+      const unsigned md = __reduce_min_sync(kFull, d);
+      const unsigned mj = __reduce_min_sync(kFull, d == md ? j : ~0u);
+      if (lane == 0) {
+        int next = (int)mj;
+        if (mj >= (unsigned)n) {  // cannot happen with n >= 2; recorded
+          atomicOr(&c.st->error, kErrCheck);
+          next = 0;
+        }
+        tabu[next >> 5] |= 1u << (next & 31);
+        tour[s] = (int16_t)next;
+        s_cur = next;
+        s_pos = s + 1;
+      }
+    }
+    __syncthreads();
+  }
+  int64_t len = 0;
+  for (int i = tid; i < n; i += kGreedyNnThreads)
+    len += c.dist[(size_t)tour[i] * c.ld + tour[i + 1 == n ? 0 : i + 1]];
+  for (int o = 16; o; o >>= 1) len += __shfl_xor_sync(kFull, len, o);
+  if (lane == 0) red_len[warp] = (unsigned long long)len;
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < kGreedyNnThreads / 32; w++) len += (int64_t)red_len[w];
+    greedy_finish(c, len);
+  }
+}
+
+// The same tour whatever the candidate lists (none in int16, or another tie
+// order).  The reference's greedyDistance is a stub returning 0
+// (src/Colony.cu:1053-1055) and its tau0 is the constant 1e-6
+// (src/AntSystem.cu:200-203), which this kernel also sets.  One CTA of
+// kGreedyThreads: each step reads the current row once (coalesced, n /
+// kGreedyThreads cities per thread) and takes the block-wide minimum of
+// (distance << 32 | city) over unvisited cities, so a step costs one L2 round
+// trip and two barriers.
 constexpr int kGreedyThreads = 1024;
 
 __global__ void __launch_bounds__(kGreedyThreads)
@@ -497,23 +638,23 @@ __global__ void __launch_bounds__(kGreedyThreads)
     __syncthreads();
     cur = s_next;
   }
-  if (tid == 0) {
-    len += c.dist[(size_t)cur * c.ld + 0];
-    const float cnn = __ll2float_rn(len);
-    float t0;
-    if (c.variant == ACO_RANK_BASED) {
-      const float num = __fmul_rn(__fmul_rn(0.5f, (float)c.rank_w), (float)(c.rank_w - 1));
-      t0 = __fdiv_rn(num, __fmul_rn(c.rho, cnn));
-    } else {
-      t0 = __fdiv_rn((float)c.m, cnn);
-    }
-    c.st->tau0 = t0;
-    c.st->greedy_length = len;
-  }
+  if (tid == 0) greedy_finish(c, len + c.dist[(size_t)cur * c.ld + 0]);
 }
 
 cudaError_t launch_greedy_tau0(const ColonyDev &c, int tau0_mode, float tau0_value,
-                               cudaStream_t s) {
+                               bool stable_lists, cudaStream_t s) {
+  if (tau0_mode == ACO_TAU0_DORIGO && stable_lists && c.nn16 && c.n < 32768) {
+    const bool staged = (size_t)c.n * c.ldk * 2 <= kGreedyStageBytes;
+    const size_t smem = greedy_layout(c.n, c.ldk, staged).bytes;
+    void (*fn)(ColonyDev) = staged ? k_greedy_tau0_nn<true> : k_greedy_tau0_nn<false>;
+    if (smem > 48 * 1024) {
+      const cudaError_t e =
+          cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    fn<<<1, kGreedyNnThreads, smem, s>>>(c);
+    return cudaGetLastError();
+  }
   const size_t smem = (size_t)((c.n + 31) / 32) * 4;
   k_greedy_tau0<<<1, kGreedyThreads, smem, s>>>(c, tau0_mode, tau0_value);
   return cudaGetLastError();

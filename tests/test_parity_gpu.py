@@ -473,3 +473,33 @@ def test_ranked_deposit_lists_match_oracle(w, m, n, k, aging):
         assert_same_state(g, q, aging=bool(aging), ctx=f"w={w} iteration {it}")
     g.close()
     q.close()
+
+
+@pytest.mark.parametrize("n,k,lattice", [(3, 1, 0), (31, 5, 0), (32, 32, 0), (33, 33, 0), (64, 1, 1),
+                                         (257, 2, 0), (400, 16, 1), (1000, 30, 0), (1025, 40, 1),
+                                         (2559, 32, 0), (2561, 32, 0), (4100, 1, 0)])
+@pytest.mark.parametrize("variant", [_abi.ACO_ANT_SYSTEM, _abi.ACO_RANK_BASED])
+def test_greedy_tau0_matches_oracle(n, k, lattice, variant):
+    """tau0 from the greedy tour over candidate lists in shared memory (up to
+    160 KB of them) and in L2, with lists that run out, and distances that tie."""
+    if lattice:
+        side = int(np.ceil(np.sqrt(n)))
+        gx, gy = np.meshgrid(np.arange(side, dtype=np.float32), np.arange(side, dtype=np.float32))
+        d = instances.euc2d_distances(gx.ravel()[:n], gy.ravel()[:n])
+    else:
+        _, _, d = instance(n, 70 + n + k)
+    p = params(num_ants=4, variant=variant, rank_w=6, beta=2.0, rho=0.2, cand_k=k, seed=k,
+               **FAST_MODE)
+    g, q = pair(p, d)
+    assert np.array_equal(bits(g.pheromone()), bits(q.pheromone())), "tau0"
+    cur, seen, length = 0, np.zeros(n, bool), 0
+    seen[0] = True
+    for _ in range(n - 1):
+        row = np.where(seen, np.int64(2**40), d[cur])
+        nxt = int(np.argmin(row))
+        length += int(row[nxt])
+        seen[nxt] = True
+        cur = nxt
+    assert g.stats()["greedy_length"] == length + int(d[cur, 0])
+    g.close()
+    q.close()
