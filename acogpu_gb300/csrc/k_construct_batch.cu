@@ -85,16 +85,16 @@ __global__ void __launch_bounds__(kBatchMaxWarps * 32) k_batch_construct(const C
       if (!s_ok) break;
       if (warp < w.z) {
         if (n <= 1024)
-          construct_ant_staged<AGING, 1, G, TableRows<4 * G>>(
+          construct_ant_staged<AGING, 1, G, TableRows<4 * G>, true, false>(
               c, w.y + warp, c.st->iteration, nullptr, TableRows<4 * G>{sids, scw, smean}, lane);
         else
-          construct_ant_staged<AGING, 2, G, TableRows<4 * G>>(
+          construct_ant_staged<AGING, 2, G, TableRows<4 * G>, true, false>(
               c, w.y + warp, c.st->iteration, nullptr, TableRows<4 * G>{sids, scw, smean}, lane);
       }
     } else if (!MULTI && c.nn16 && c.ldk == 4 * G && c.n <= 2048) {
       // Too large to stage: the same step loop on rows read from L2.
       if (warp < w.z)
-        construct_ant_staged<AGING, 2, G, TableRows<4 * G>>(
+        construct_ant_staged<AGING, 2, G, TableRows<4 * G>, true, false>(
             c, w.y + warp, c.st->iteration, nullptr,
             TableRows<4 * G>{c.nn16, c.choice_nn, c.mean}, lane);
     } else if (warp < w.z) {

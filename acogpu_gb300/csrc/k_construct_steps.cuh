@@ -425,9 +425,13 @@ __device__ __forceinline__ float scan_level(float x, int o) {
 // like they do, and a visited city's are masked to 0: a lane keeps the
 // largest of its cities chunk by chunk (128 cities, four a lane, the chunk's
 // four values kept with it), one warp maximum gives the value and one warp
-// minimum the lowest city that has it.  A group of chunks is loaded ahead of
-// the one being compared: four (n <= 2048; the whole row at n = 1000 takes two
-// groups) or eight (n = 4096: construction 1436 us with four, 1374 with eight).  A row whose largest value is 0 or NaN goes to fallback_rest, which
+// minimum the lowest city that has it.  AHEAD (not in the batch kernel, whose
+// many warps cover the loads and whose registers the buffers would cost: 37.2
+// ms of construction for 512 instances with it, 27 without): a group of chunks
+// is loaded ahead of the one being compared, four (n <= 2048; the whole row at
+// n = 1000 takes two groups) or eight (n = 4096: construction 1436 us with
+// four, 1374 with eight).  A row whose largest value is 0 or NaN goes to
+// fallback_rest, which
 // tells an unvisited zero from a visited city and skips NaNs.
 template <int TW>
 struct TwPack {
@@ -511,18 +515,21 @@ __device__ __forceinline__ uint32_t blend_bits(const ColonyDev &c, uint32_t t, u
                                        c.use_alpha, c.alpha));
 }
 
-template <int TW, bool BL>
+template <int TW, bool BL, bool AHEAD>
 __device__ __forceinline__ int fallback_scan(const ColonyDev &c, int cur, const TwPack<TW> &p,
                                              const AntCtx &a, int lane) {
-  constexpr int GR = TW > 2 && !BL ? 8 : 4;  // chunks a group; the next one loaded ahead
+  constexpr int GR = TW > 2 && !BL && AHEAD ? 8 : 4;  // chunks a group
   const size_t row = (size_t)cur * c.ld;
   unsigned best = 0u;
   int bt = 0;
   uint4 bq = make_uint4(0u, 0u, 0u, 0u), q[GR], e[GR], nq[GR], ne[GR];
-  fallback_group<BL, GR>(c, row, 0, lane, q, e);
+  if (AHEAD) fallback_group<BL, GR>(c, row, 0, lane, q, e);
 #pragma unroll 1
   for (int t0 = 0; t0 * 128 < c.n; t0 += GR) {
-    fallback_group<BL, GR>(c, row, t0 + GR, lane, nq, ne);
+    if (AHEAD)
+      fallback_group<BL, GR>(c, row, t0 + GR, lane, nq, ne);
+    else
+      fallback_group<BL, GR>(c, row, t0, lane, q, e);
     unsigned m[GR];
 #pragma unroll
     for (int t = 0; t < GR; t++) {
@@ -547,10 +554,12 @@ __device__ __forceinline__ int fallback_scan(const ColonyDev &c, int cur, const 
         bt = t0 + t;
         bq = q[t];
       }
+    if (AHEAD) {
 #pragma unroll
-    for (int t = 0; t < GR; t++) {
-      q[t] = nq[t];
-      e[t] = ne[t];
+      for (int t = 0; t < GR; t++) {
+        q[t] = nq[t];
+        e[t] = ne[t];
+      }
     }
   }
   const unsigned m = __reduce_max_sync(kFull, best);
@@ -613,14 +622,14 @@ __device__ __forceinline__ int fallback_tier2(const ColonyDev &c, int cur,
 
 // The whole best-choice fallback, as a called function (the tabu words by
 // value, so they stay in registers): its code stays out of the step loop.
-template <int TW>
+template <int TW, bool AHEAD>
 __device__ __noinline__ int fallback_best(const ColonyDev &c, int cur, TwPack<TW> p, AntCtx a,
                                           int lane, int id, bool vis, bool tier_ok) {
   int next = -1;
   if (tier_ok && c.t2 > 0) next = fallback_tier2<TW>(c, cur, p, id, vis, lane);
   if (next < 0)
-    next = a.blend ? fallback_scan<TW, true>(c, cur, p, a, lane)
-                   : fallback_scan<TW, false>(c, cur, p, a, lane);
+    next = a.blend ? fallback_scan<TW, true, AHEAD>(c, cur, p, a, lane)
+                   : fallback_scan<TW, false, AHEAD>(c, cur, p, a, lane);
   return next;
 }
 
@@ -711,7 +720,7 @@ struct ClusterRows {
 // consecutive steps are computed one per lane and broadcast; the tour
 // positions of the current 32-step block stay in one register per lane and
 // are stored together.
-template <int TW, bool BLEND, int G, class ROWS, bool TIER>
+template <int TW, bool BLEND, int G, class ROWS, bool TIER, bool AHEAD>
 __device__ __forceinline__ void staged_steps(const ColonyDev &c, int k, uint32_t akey, int start,
                                              StepTabu<TW> &tabu, const ROWS &rows, AntCtx a,
                                              int lane, int64_t &fallbacks) {
@@ -796,7 +805,7 @@ __device__ __forceinline__ void staged_steps(const ColonyDev &c, int k, uint32_t
             if (!BLEND && a.blend) a.meanc = rows.row_mean(cur);  // pre-blended table
             TwPack<TW> pk;
             tabu.words_of(pk.w, lane);
-            next = fallback_best<TW>(c, cur, pk, a, lane, id, vis, TIER && !BLEND && !a.blend);
+            next = fallback_best<TW, AHEAD>(c, cur, pk, a, lane, id, vis, TIER && !BLEND && !a.blend);
           } else {  // select_local_best on a full row of at most 32 cities (k == n)
             const unsigned um = __ballot_sync(kFull, lane < c.K && id >= 0 && !vis);
             next = um ? __shfl_sync(kFull, id, 31 - __clz(um)) : -1;
@@ -824,7 +833,7 @@ __device__ __forceinline__ void staged_steps(const ColonyDev &c, int k, uint32_t
 // the step loop (BLEND: the aging fitness blend of every candidate per step;
 // otherwise the weights come blended, or plain, from the table), then the
 // integer length and the transposed successor/predecessor lists.
-template <int TW, int G, bool BLEND, class ROWS, bool TIER = true>
+template <int TW, int G, bool BLEND, class ROWS, bool TIER = true, bool AHEAD = true>
 __device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, uint32_t *words,
                                 const ROWS &rows, AntCtx a, int lane) {
   const int n = c.n;
@@ -843,7 +852,7 @@ __device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, uint32
   tabu.mark(start, lane);
 
   int64_t fallbacks = 0;
-  staged_steps<TW, BLEND, G, ROWS, TIER>(c, k, akey, start, tabu, rows, a, lane, fallbacks);
+  staged_steps<TW, BLEND, G, ROWS, TIER, AHEAD>(c, k, akey, start, tabu, rows, a, lane, fallbacks);
   __syncwarp();
   // Tour length (order-free integer sum) and the transposed successor /
   // predecessor of every city for the row-owned deposit, one edge per lane;
@@ -877,7 +886,7 @@ __device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, uint32
 // One ant with its aging step: updateAntAges (src/Colony.cu:353-364), the
 // cleared tour of an invalid ant (src/Colony.cu:507-510) and the blend
 // decision of compute_fittness (inc/Colony.cuh:21-30).
-template <bool AGING, int TW, int G, class ROWS, bool TIER = true>
+template <bool AGING, int TW, int G, class ROWS, bool TIER = true, bool AHEAD = true>
 __device__ void construct_ant_staged(const ColonyDev &c, int k, uint32_t iter, uint32_t *words,
                                      const ROWS &rows, int lane) {
   AntCtx a;
@@ -900,9 +909,9 @@ __device__ void construct_ant_staged(const ColonyDev &c, int k, uint32_t iter, u
     if (a.blend) a.ratio = __fdiv_rn(__int2float_rn(age), __int2float_rn(c.min_ret));
   }
   if (AGING && a.blend)
-    staged_ant_body<TW, G, true, ROWS, TIER>(c, k, iter, words, rows, a, lane);
+    staged_ant_body<TW, G, true, ROWS, TIER, AHEAD>(c, k, iter, words, rows, a, lane);
   else
-    staged_ant_body<TW, G, false, ROWS, TIER>(c, k, iter, words, rows, a, lane);
+    staged_ant_body<TW, G, false, ROWS, TIER, AHEAD>(c, k, iter, words, rows, a, lane);
 }
 
 }  // namespace aco
