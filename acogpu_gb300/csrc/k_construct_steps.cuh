@@ -431,8 +431,8 @@ __device__ __forceinline__ float scan_level(float x, int o) {
 // is loaded ahead of the one being compared, four (n <= 2048; the whole row at
 // n = 1000 takes two groups) or eight (n = 4096: construction 1436 us with
 // four, 1374 with eight).  A row whose largest value is 0 or NaN goes to
-// fallback_rest, which
-// tells an unvisited zero from a visited city and skips NaNs.
+// fallback_rest, which tells an unvisited zero from a visited city and skips
+// NaNs.
 template <int TW>
 struct TwPack {
   uint32_t w[TW];

@@ -143,11 +143,19 @@ cudaError_t launch_heuristic_table(const int32_t *dist, int n, int ld, const flo
 // shared memory by a TMA bulk copy.  Equal distances keep city order, which
 // is the rank-by-counting order of the reference GPU kernel
 // (inc/Colony.cuh:101-123).
-constexpr int kSortThreads = 1024;
+//
+// Thread t of a stage with partner distance j takes the pair (i, i + j), i =
+// t with a zero bit inserted at j: for j <= 32 a warp's pairs lie in 64
+// consecutive keys of its own, so those stages (six of every merge) need a
+// warp barrier only.  One thread a pair up to 2048 keys, 1024 threads above.
+// With 1024 threads whatever the row and a block barrier a stage the 512
+// instances of a batch (50 to 2000 cities) took 65 us each and n = 4096 1120 us;
+// now 46 and 919.
+constexpr int kSortMaxThreads = 1024;
 constexpr int kMaxSortRow = 16384;
-constexpr int kSortPerThread = kMaxSortRow / kSortThreads;
+constexpr int kSortPerThread = kMaxSortRow / kSortMaxThreads;
 
-__global__ void __launch_bounds__(kSortThreads)
+__global__ void __launch_bounds__(kSortMaxThreads)
     k_nn_sort_stable(const int32_t *__restrict__ dist, int n, int ld, int K, int ldk,
                      int32_t *__restrict__ nn, int32_t *__restrict__ nn2, int t2, int P,
                      ColonyState *st) {
@@ -155,7 +163,7 @@ __global__ void __launch_bounds__(kSortThreads)
   uint64_t *keys = reinterpret_cast<uint64_t *>(smem);
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem + (size_t)P * 8);
   int *flag = reinterpret_cast<int *>(bar + 1);
-  const int row = blockIdx.x, tid = threadIdx.x;
+  const int row = blockIdx.x, tid = threadIdx.x, T = blockDim.x;
   int32_t *drow = reinterpret_cast<int32_t *>(keys);
   if (tid == 0) {
     mbar_init(bar, 1);
@@ -170,40 +178,43 @@ __global__ void __launch_bounds__(kSortThreads)
   }
   __syncthreads();
   if (!*flag) return;
-  uint64_t v[kSortPerThread];
+  uint64_t v[kSortPerThread];  // the launch has P <= kSortPerThread * T
 #pragma unroll
   for (int q = 0; q < kSortPerThread; q++) {
-    const int i = tid + q * kSortThreads;
+    const int i = tid + q * T;
     v[q] = ~0ull;
     if (i < n) v[q] = ((uint64_t)(uint32_t)drow[i] << 32) | (uint32_t)i;
   }
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < kSortPerThread; q++) {
-    const int i = tid + q * kSortThreads;
+    const int i = tid + q * T;
     if (i < P) keys[i] = v[q];
   }
   __syncthreads();
   for (int k = 2; k <= P; k <<= 1) {
     for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = tid; i < P; i += kSortThreads) {
-        const int ixj = i ^ j;
-        if (ixj > i) {
-          const uint64_t a = keys[i], b = keys[ixj];
-          const bool up = (i & k) == 0;
-          if ((a > b) == up) {
-            keys[i] = b;
-            keys[ixj] = a;
-          }
+      for (int t = tid; t < P / 2; t += T) {
+        const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1));
+        const uint64_t a = keys[i], b = keys[i + j];
+        if ((a > b) == ((i & k) == 0)) {
+          keys[i] = b;
+          keys[i + j] = a;
         }
       }
-      __syncthreads();
+      // The next stage's pairs are the warp's own unless it pairs farther
+      // apart: the next merge's first stage has j = k.
+      if (j > 32 || (j == 1 && k > 32))
+        __syncthreads();
+      else
+        __syncwarp();
     }
   }
-  for (int q = tid; q < ldk; q += kSortThreads)
+  __syncthreads();
+  for (int q = tid; q < ldk; q += T)
     nn[(size_t)row * ldk + q] = q < K ? (int32_t)(uint32_t)(keys[q] & 0xffffffffu) : -1;
   if (nn2)  // the fallback's second tier: neighbours K .. K + t2 - 1
-    for (int q = tid; q < kTier2; q += kSortThreads)
+    for (int q = tid; q < kTier2; q += T)
       nn2[(size_t)row * kTier2 + q] =
           q < t2 ? (int32_t)(uint32_t)(keys[K + q] & 0xffffffffu) : -1;
 }
@@ -214,12 +225,15 @@ cudaError_t launch_nn_sort_stable(const int32_t *dist, int n, int ld, int K, int
   if (n > kMaxSortRow) return cudaErrorInvalidValue;
   int P = 1;
   while (P < n) P <<= 1;
-  if (P < 32) P = 32;
+  if (P < 64) P = 64;  // one warp's keys, and the row's pitch fits (ld <= 2 P)
+  const int threads = P / 2 < kSortMaxThreads ? P / 2 : kSortMaxThreads;
   const size_t smem = (size_t)P * 8 + 16;
-  cudaError_t e = cudaFuncSetAttribute(k_nn_sort_stable,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k_nn_sort_stable<<<n, kSortThreads, smem, s>>>(dist, n, ld, K, ldk, nn, nn2, t2, P, st);
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(k_nn_sort_stable,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  k_nn_sort_stable<<<n, threads, smem, s>>>(dist, n, ld, K, ldk, nn, nn2, t2, P, st);
   return cudaGetLastError();
 }
 

@@ -503,3 +503,17 @@ def test_greedy_tau0_matches_oracle(n, k, lattice, variant):
     assert g.stats()["greedy_length"] == length + int(d[cur, 0])
     g.close()
     q.close()
+
+
+@pytest.mark.parametrize("n", [3, 31, 33, 63, 64, 65, 127, 129, 1023, 1025, 2047, 2049, 4097, 8193])
+def test_stable_sort_edges(n):
+    """The stable nn sort around its block sizes, distances with many ties."""
+    g0 = np.random.default_rng(n)
+    x, y = g0.integers(0, 40, (2, n)).astype(np.float32)
+    d = instances.euc2d_distances(x, y)
+    k = min(n - 1, 32)
+    p = params(num_ants=2, beta=1.0, cand_k=k, **FAST_MODE)
+    g = aco.Colony(d, params=p, num_ants=2)
+    g.initialize()
+    assert np.array_equal(g.nn_list(), np.argsort(d, axis=1, kind="stable")[:, :k])
+    g.close()
