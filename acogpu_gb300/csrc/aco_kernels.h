@@ -96,7 +96,12 @@ constexpr int kRowsMaxAnts = 11;
 // Rows that the long-row kernel sums in city order (full rows longer than one
 // chunk of 128); their matrices' pitch is a multiple of 128.
 __host__ __device__ constexpr bool rows_city_order(int n, int K) { return K == n && n > 128; }
-cudaError_t launch_construct_rows(const ColonyDev &c, int grid, int ants, cudaStream_t s);
+// staged: the candidate rows copied to shared memory (n <= 1024, the bytes
+// below configured before).
+size_t construct_rows_staged_bytes(int n, int ldk);
+cudaError_t configure_construct_rows_staged(size_t smem);
+cudaError_t launch_construct_rows(const ColonyDev &c, int grid, int ants, bool staged,
+                                  cudaStream_t s);
 // max_n: the batch's largest instance (it picks the visited mask's size).
 int batch_rows_blocks_per_sm(int ants, int max_n, bool aging);
 cudaError_t launch_batch_construct_rows(const ColonyDev *descs, const int4 *items, int num_items,

@@ -303,7 +303,7 @@ cudaError_t launch_construction(aco_colony *c, const ColonyDev &d) {
     }
     return launch_construct_staged(d, c->nn16, c->staged_grid, c->staged_warps, c->stream);
   }
-  if (c->rows) return launch_construct_rows(d, c->staged_grid, c->staged_warps, c->stream);
+  if (c->rows) return launch_construct_rows(d, c->staged_grid, c->staged_warps, c->rows_staged, c->stream);
   if (c->cluster)
     return launch_construct_cluster(d, c->staged_grid, c->staged_warps, c->cluster, c->stream);
   if (c->direct) return launch_construct_direct(d, c->staged_grid, c->staged_warps, c->stream);
@@ -331,6 +331,16 @@ int plan_construction(aco_colony *c) {
     c->rows = true;
     c->staged_warps = ants;
     c->staged_grid = (c->m + ants - 1) / ants;
+    // Rows in shared memory when they fit (one CTA an SM) and one pass of
+    // such CTAs takes all ants; beyond, more warps an SM on L2 rows are worth
+    // more than the shorter step.  n = m = 100: 57 us from L2, 43 staged; 190
+    // cities 106 staged, 200 from L2 115.
+    const size_t smem = construct_rows_staged_bytes(c->n, c->ldk);
+    c->rows_staged = c->n <= 1024 && smem + 4096 <= (size_t)c->max_smem_optin &&
+                     c->staged_grid <= sms;
+    if (c->rows_staged)
+      ACO_CUDA(c, configure_construct_rows_staged((size_t)c->max_smem_optin - 4096),
+               "configure staged rows");
     return ACO_OK;
   }
   if (c->K > 32 || !c->nn16 || mode == ACO_CONSTRUCT_GLOBAL) return ACO_OK;
@@ -1010,7 +1020,7 @@ struct aco_batch {
   int total_rows = 0, num_items = 0;
   int max_n = 0, max_k = 0, max_ld = 0, num_sms = 1, max_smem_optin = 0;
   int sp = 0;  // row pitch of the staged items: the largest among instances with k <= 32
-  int apb = 8, row_threads = 256, grid = 0;
+  int apb = 8, row_threads = 128, grid = 0;  // rows: 4.4 ms an iteration of 512 instances, 4.75 at 256
   size_t region_bytes = 0;  // shared region of the construction launch
   int staged_count = 0;     // instances built from a staged table
   bool rows = false;        // construction by the long-row batch kernel (every k > 32)

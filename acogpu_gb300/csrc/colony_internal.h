@@ -40,6 +40,7 @@ struct aco_colony {
   bool direct = false;      // construction by the direct (L2-row) kernel
   int cluster = 0;          // construction by the cluster kernel: CTAs per cluster
   bool rows = false;        // construction by the long-row kernel (k > 32)
+  bool rows_staged = false; // ... with the rows in shared memory
   int32_t *nn2 = nullptr;   // fallback second tier (see ColonyDev)
   float *t2v = nullptr;
   float *mout = nullptr;

@@ -230,18 +230,24 @@ __device__ __forceinline__ void rows_fetch(const float *row, int t0, int n, ulon
   }
 }
 
-template <bool BLEND>
+// STG: the view's candidate rows are in shared memory.
+template <bool BLEND, bool STG>
 __device__ __forceinline__ void rows_load(const ColonyDev &c, const RowsView &v, int cur, int ch,
                                           float4 &w, float4 &e, uint2 &id, int lane) {
   const int p0 = ch * 128 + lane * 4;
   const size_t off = (size_t)cur * v.ldk + p0;
   const bool in = p0 < v.K;  // ldk % 4 == 0: the four entries are in the row
-  id = in ? __ldg(reinterpret_cast<const uint2 *>(v.nn16 + off)) : make_uint2(0u, 0u);
-  w = in ? __ldcg(reinterpret_cast<const float4 *>((BLEND ? c.tau_nn : v.choice_nn) + off))
-         : make_float4(0.f, 0.f, 0.f, 0.f);
-  if (BLEND)
-    e = in ? __ldg(reinterpret_cast<const float4 *>(c.eta_nn + off))
-           : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const uint2 *ip = reinterpret_cast<const uint2 *>(v.nn16 + off);
+  const float4 *wp = reinterpret_cast<const float4 *>((BLEND ? c.tau_nn : v.choice_nn) + off);
+  if constexpr (STG) {
+    id = in ? *ip : make_uint2(0u, 0u);
+    w = in ? (BLEND ? __ldcg(wp) : *wp) : zero;
+  } else {
+    id = in ? __ldg(ip) : make_uint2(0u, 0u);
+    w = in ? __ldcg(wp) : zero;
+  }
+  if (BLEND) e = in ? __ldg(reinterpret_cast<const float4 *>(c.eta_nn + off)) : zero;
 }
 
 __device__ __forceinline__ RowsView rows_view(const ColonyDev &c) {
@@ -606,20 +612,20 @@ __device__ __forceinline__ unsigned rows_first(const float (&p)[4], uint2 id, fl
 // loaded with the sum's rows and scanned before they are waited for, so the
 // common step (the crossing in chunk 0: 97 % of the steps at n = 1000) waits
 // for one L2 round trip, the sum and one warp minimum.
-template <bool R1, bool BLEND, bool LUT>
+template <bool R1, bool BLEND, bool LUT, bool STG>
 __device__ __forceinline__ int rows_pick(const ColonyDev &c, const RowsView &v, int cur,
                                          const uint32_t *mask, uint32_t own, const RowsLut &lut, bool natural, int cnt,
                                          float u, const AntCtx &a, int lane) {
   const int nch = (v.K + 127) >> 7;
   float4 w, e;
   uint2 id;
-  rows_load<BLEND>(c, v, cur, 0, w, e, id, lane);
+  rows_load<BLEND, STG>(c, v, cur, 0, w, e, id, lane);
   // The entries of the sum, d_S + d_P and 8 (a row of 64 chunks adds at most
   // 64 to either): the window's terms but for the entries up to the crossing.
   const int terms = cnt + 28 + nch;
   float p[4], total, S;
   RowsChunk k;
-  if (natural) {
+  if (!STG && natural) {
     const float part = rows_city_sum<R1, BLEND, LUT>(c, v, cur, mask, own, lut, a, lane);
     k = rows_mask<R1, BLEND>(c, mask, w, e, id, lane * 4, a);
     rows_prefix(k.x, 0.0f, lane, p, total);
@@ -632,7 +638,7 @@ __device__ __forceinline__ int rows_pick(const ColonyDev &c, const RowsView &v, 
       float part = 0.0f;
 #pragma unroll 1
       for (int ch = 1; ch < nch; ch++) {
-        rows_load<BLEND>(c, v, cur, ch, w, e, id, lane);
+        rows_load<BLEND, STG>(c, v, cur, ch, w, e, id, lane);
         const RowsChunk q = rows_mask<R1, BLEND>(c, mask, w, e, id, ch * 128 + lane * 4, a);
         part += (q.x[0] + q.x[1]) + (q.x[2] + q.x[3]);
       }
@@ -649,17 +655,17 @@ __device__ __forceinline__ int rows_pick(const ColonyDev &c, const RowsView &v, 
     if (S == 0.0f) return -1;
     // In the window, a sum that is not finite, or u S' close to S'.
     if (first != ~0u || !(S <= 3e38f) || ++ch >= nch) return kRowsAmbiguous;
-    rows_load<BLEND>(c, v, cur, ch, w, e, id, lane);
+    rows_load<BLEND, STG>(c, v, cur, ch, w, e, id, lane);
     k = rows_mask<R1, BLEND>(c, mask, w, e, id, ch * 128 + lane * 4, a);
     rows_prefix(k.x, total, lane, p, total);
   }
 }
 
 // The tour of one valid ant.
-template <bool R1, bool BLEND, bool LUT>
-__device__ __forceinline__ void rows_tour(const ColonyDev &c, int k, uint32_t *mask,
-                                          const RowsLut &lut, AntCtx a, int lane) {
-  const RowsView v = rows_view(c);
+template <bool R1, bool BLEND, bool LUT, bool STG>
+__device__ __forceinline__ void rows_tour(const ColonyDev &c, const RowsView &v, int k,
+                                          uint32_t *mask, const RowsLut &lut, AntCtx a,
+                                          int lane) {
   const int n = c.n;
   int32_t *trow = c.tours + (size_t)k * c.ld;
   const bool natural = rows_city_order(n, c.K) && *c.prior_set == 0;
@@ -694,7 +700,7 @@ __device__ __forceinline__ void rows_tour(const ColonyDev &c, int k, uint32_t *m
     for (int x = xb == 0 ? 1 : xb; x < xe; x++) {
       const float u = __shfl_sync(kFull, ublk, x & 31);
       if (BLEND) a.meanc = c.mean[cur];
-      int next = rows_pick<R1, BLEND, LUT>(c, v, cur, mask, own, lut, natural, min(v.K, n - x), u, a,
+      int next = rows_pick<R1, BLEND, LUT, STG>(c, v, cur, mask, own, lut, natural, min(v.K, n - x), u, a,
                                            lane);
       if (next < 0) {
         if (next == kRowsAmbiguous) next = rows_exact<R1, BLEND>(c, cur, mask, u, a, lane);
@@ -746,9 +752,9 @@ __device__ __forceinline__ void rows_tour(const ColonyDev &c, int k, uint32_t *m
 // ages; blend ants first, then the other valid ones, then the invalid ones),
 // or ant `pos` without aging.  An invalid ant keeps a cleared tour
 // (src/Colony.cu:507-510).
-template <bool R1, bool AGING, bool LUT>
-__device__ __forceinline__ void rows_ant(const ColonyDev &c, int pos, uint32_t *mask,
-                                         const RowsLut &lut, int lane) {
+template <bool R1, bool AGING, bool LUT, bool STG>
+__device__ __forceinline__ void rows_ant(const ColonyDev &c, const RowsView &v, int pos,
+                                         uint32_t *mask, const RowsLut &lut, int lane) {
   AntCtx a;
   a.blend = false;
   a.ratio = 0.0f;
@@ -766,9 +772,9 @@ __device__ __forceinline__ void rows_ant(const ColonyDev &c, int pos, uint32_t *
     if (a.blend) a.ratio = __fdiv_rn(__int2float_rn(age), __int2float_rn(c.min_ret));
   }
   if (AGING && a.blend)
-    rows_tour<R1, true, LUT>(c, k, mask, lut, a, lane);
+    rows_tour<R1, true, LUT, STG>(c, v, k, mask, lut, a, lane);
   else
-    rows_tour<R1, false, LUT>(c, k, mask, lut, a, lane);
+    rows_tour<R1, false, LUT, STG>(c, v, k, mask, lut, a, lane);
 }
 
 __host__ __device__ constexpr int rows_words(bool r1) { return r1 ? 32 : kRowsMaskWords; }
@@ -784,22 +790,83 @@ __global__ void __launch_bounds__(kRowsMaxAnts * 32, 1) k_construct_rows(const _
   __shared__ RowsLut lut;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   rows_lut_init(lut);
+  const RowsView v = rows_view(c);
   for (int pos = warp * gridDim.x + blockIdx.x; pos < c.m; pos += gridDim.x * warps)
-    rows_ant<R1, AGING, true>(c, pos, masks[warp], lut, lane);
+    rows_ant<R1, AGING, true, false>(c, v, pos, masks[warp], lut, lane);
 }
 
-cudaError_t launch_construct_rows(const ColonyDev &c, int grid, int ants, cudaStream_t s) {
+// Single colony whose candidate rows fit in shared memory (full rows up to 190
+// cities, n * k up to 36 000): every CTA copies choice values and ids by TMA,
+// and a step waits for shared memory instead of L2 and sums in row order.
+// Layout: [choice n * ldk f32][ids n * ldk int16][mbarrier].
+template <bool AGING>
+__global__ void __launch_bounds__(kRowsMaxAnts * 32, 1)
+    k_construct_rows_staged(const __grid_constant__ ColonyDev c) {
+  extern __shared__ __align__(128) unsigned char smem_rs[];
+  __shared__ uint32_t masks[kRowsMaxAnts][rows_words(true)];
+  __shared__ RowsLut lut;
+  __shared__ int flag;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const uint32_t w_bytes = (uint32_t)c.n * c.ldk * 4u, id_bytes = (uint32_t)c.n * c.ldk * 2u;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem_rs + w_bytes + id_bytes);
+  if (threadIdx.x == 0) {
+    mbar_init(bar, 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    mbar_arrive_expect_tx(bar, w_bytes + id_bytes);
+    constexpr uint32_t kPiece = 32768;
+    const char *g = reinterpret_cast<const char *>(c.choice_nn);
+    for (uint32_t o = 0; o < w_bytes; o += kPiece)
+      tma_load_1d(smem_rs + o, g + o, min(kPiece, w_bytes - o), bar);
+    g = reinterpret_cast<const char *>(c.nn16);
+    for (uint32_t o = 0; o < id_bytes; o += kPiece)
+      tma_load_1d(smem_rs + w_bytes + o, g + o, min(kPiece, id_bytes - o), bar);
+    flag = mbar_wait_bounded(bar, 0, c.st) ? 1 : 0;
+  }
+  __syncthreads();
+  if (!flag) return;
+  RowsView v = rows_view(c);
+  v.choice_nn = reinterpret_cast<const float *>(smem_rs);
+  v.nn16 = reinterpret_cast<const int16_t *>(smem_rs + w_bytes);
+  for (int pos = warp * gridDim.x + blockIdx.x; pos < c.m; pos += gridDim.x * warps)
+    rows_ant<true, AGING, true, true>(c, v, pos, masks[warp], lut, lane);
+}
+
+size_t construct_rows_staged_bytes(int n, int ldk) { return (size_t)n * ldk * 6 + 16; }
+
+cudaError_t configure_construct_rows_staged(size_t smem) {
+  cudaError_t e = cudaFuncSetAttribute(k_construct_rows_staged<false>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_construct_rows_staged<true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return e;
+}
+
+cudaError_t launch_construct_rows(const ColonyDev &c, int grid, int ants, bool staged,
+                                  cudaStream_t s) {
   if (c.aging) {
     cudaError_t e = launch_aging_plan(c, s);
     if (e != cudaSuccess) return e;
-    if (c.n <= 1024)
-      k_construct_rows<true, true><<<grid, ants * 32, 0, s>>>(c);
+  }
+  const int threads = ants * 32;
+  if (staged) {
+    const size_t smem = construct_rows_staged_bytes(c.n, c.ldk);
+    if (c.aging)
+      k_construct_rows_staged<true><<<grid, threads, smem, s>>>(c);
     else
-      k_construct_rows<false, true><<<grid, ants * 32, 0, s>>>(c);
+      k_construct_rows_staged<false><<<grid, threads, smem, s>>>(c);
   } else if (c.n <= 1024) {
-    k_construct_rows<true, false><<<grid, ants * 32, 0, s>>>(c);
+    if (c.aging)
+      k_construct_rows<true, true><<<grid, threads, 0, s>>>(c);
+    else
+      k_construct_rows<true, false><<<grid, threads, 0, s>>>(c);
+  } else if (c.aging) {
+    k_construct_rows<false, true><<<grid, threads, 0, s>>>(c);
   } else {
-    k_construct_rows<false, false><<<grid, ants * 32, 0, s>>>(c);
+    k_construct_rows<false, false><<<grid, threads, 0, s>>>(c);
   }
   return cudaGetLastError();
 }
@@ -835,8 +902,9 @@ __global__ void __maxnreg__(64)
       __syncwarp();
       have = w.x;
     }
+    const RowsView v = rows_view(s_desc[warp]);
     for (int q = 0; q < w.z; q++)
-      rows_ant<R1, AGING, false>(s_desc[warp], w.y + q, masks[warp], lut, lane);
+      rows_ant<R1, AGING, false, false>(s_desc[warp], v, w.y + q, masks[warp], lut, lane);
   }
 }
 
