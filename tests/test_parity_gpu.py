@@ -517,3 +517,29 @@ def test_stable_sort_edges(n):
     g.initialize()
     assert np.array_equal(g.nn_list(), np.argsort(d, axis=1, kind="stable")[:, :k])
     g.close()
+
+
+@pytest.mark.parametrize("n", [3, 32, 33, 34, 64, 65, 97, 303, 1000, 2392])
+@pytest.mark.parametrize("kind", ["ties", "line", "same"])
+def test_reference_sort_edges(n, kind):
+    """The reference's quicksort order by warps: segments around 32 entries,
+    rows full of ties, sorted rows, rows of one value (nothing is smaller than
+    any pivot)."""
+    if kind == "same" and n > 400:
+        n = 400
+    g0 = np.random.default_rng(n)
+    if kind == "ties":
+        x, y = g0.integers(0, 25, (2, n)).astype(np.float32)
+    elif kind == "line":
+        x, y = np.arange(n, dtype=np.float32) * 3, np.zeros(n, np.float32)
+    else:
+        x, y = np.zeros(n, np.float32), np.zeros(n, np.float32)
+    d = instances.euc2d_distances(x, y)
+    p = params(num_ants=2, beta=1.0, cand_k=0)
+    g = aco.Colony(d, params=p, num_ants=2)
+    g.initialize()
+    q = oracle.Port(p, d, threads=8)
+    q.initialize()
+    assert np.array_equal(g.nn_list(), q.nn())
+    g.close()
+    q.close()
