@@ -61,6 +61,10 @@ cudaError_t launch_mlp_reduce(float *part, int G, int ld, bool clear, float *gou
                               bool adam, float *w, float *m1, float *m2, float lr, float b1,
                               float b2, float eps, float bc1, float bc2, __nv_bfloat16 *w1b,
                               __nv_bfloat16 *w2b, __nv_bfloat16 *w2tb, cudaStream_t s);
+cudaError_t launch_pack_examples(const float *f, int E, int B, bool labelled, __nv_bfloat16 *X,
+                                 float *Y, cudaStream_t s);
+cudaError_t launch_refresh_bf16(const float *w, __nv_bfloat16 *w1b, __nv_bfloat16 *w2b,
+                                __nv_bfloat16 *w2tb, cudaStream_t s);
 cudaError_t launch_apply_prior(const ColonyDev &c, const float *prob, float floor_,
                                cudaStream_t s);
 

@@ -52,6 +52,10 @@ struct aco_prior {
   __nv_bfloat16 *ax = nullptr;
   float *aprob = nullptr;
   int64_t a_cap = 0;
+  // examples of the calls on host data: BF16 rows, labels, raw rows, scores
+  __nv_bfloat16 *ux = nullptr;
+  float *uy = nullptr, *uf = nullptr, *uout = nullptr;
+  int64_t u_cap = 0;
   int64_t step = 0;
   int engine = ACO_GEMM_FUSED;  // enum aco_gemm_engine
   std::string err;
@@ -114,22 +118,8 @@ int gemm_status(aco_prior *p) {
 
 // Refreshes the BF16 copies of W1 (padded to 16 inputs) and W2 from the masters.
 int sync_bf16(aco_prior *p) {
-  std::vector<float> w(kParamCount);
-  ACO_PCUDA(p, copy_sync(p, w.data(), p->w, sizeof(float) * kParamCount, cudaMemcpyDeviceToHost),
-            "read weights");
-  std::vector<__nv_bfloat16> w1(kHidden * kFeatPad), w2(kHidden * kHidden), w2t(kHidden * kHidden);
-  for (int o = 0; o < kHidden; o++)
-    for (int f = 0; f < kFeatPad; f++)
-      w1[o * kFeatPad + f] =
-          __float2bfloat16_rn(f < kFeatures ? w[kParamW1 + o * kFeatures + f] : 0.0f);
-  for (int o = 0; o < kHidden; o++)
-    for (int i = 0; i < kHidden; i++) {
-      w2[o * kHidden + i] = __float2bfloat16_rn(w[kParamW2 + o * kHidden + i]);
-      w2t[i * kHidden + o] = w2[o * kHidden + i];
-    }
-  ACO_PCUDA(p, copy_sync(p, p->w1b, w1.data(), w1.size() * 2, cudaMemcpyHostToDevice), "w1");
-  ACO_PCUDA(p, copy_sync(p, p->w2b, w2.data(), w2.size() * 2, cudaMemcpyHostToDevice), "w2");
-  ACO_PCUDA(p, copy_sync(p, p->w2tb, w2t.data(), w2t.size() * 2, cudaMemcpyHostToDevice), "w2t");
+  ACO_PCUDA(p, launch_refresh_bf16(p->w, p->w1b, p->w2b, p->w2tb, p->stream), "bf16 weights");
+  ACO_PCUDA(p, cudaStreamSynchronize(p->stream), "bf16 weights");
   return ACO_OK;
 }
 
@@ -269,20 +259,44 @@ int fused_pass(aco_prior *p, const __nv_bfloat16 *X, const float *Y, int rows, f
   return ACO_OK;
 }
 
-// Uploads host examples (E x 12 FP32 features) into padded BF16 rows.
-int upload_examples(aco_prior *p, const float *feats, const float *labels, int E, int B,
-                    __nv_bfloat16 **Xd, float **Yd) {
-  std::vector<__nv_bfloat16> x((size_t)B * kFeatPad, __float2bfloat16_rn(0.0f));
-  std::vector<float> y((size_t)B, -1.0f);
-  for (int e = 0; e < E; e++) {
-    for (int f = 0; f < kFeatures; f++)
-      x[(size_t)e * kFeatPad + f] = __float2bfloat16_rn(feats[(size_t)e * kFeatures + f]);
-    if (labels) y[e] = labels[e];
+// Buffers of the calls on host examples, kept from call to call (grown as
+// needed, at most kKeepRows rows: larger ones go back at the call's end).
+constexpr int kKeepRows = 1 << 21;
+
+void release_examples(aco_prior *p) {
+  cudaFree(p->ux); cudaFree(p->uy); cudaFree(p->uf); cudaFree(p->uout);
+  p->ux = nullptr;
+  p->uy = p->uf = p->uout = nullptr;
+  p->u_cap = 0;
+}
+
+// Ends a call on host examples: nothing of the caller's is in use any more.
+struct ExamplesGuard {
+  aco_prior *p;
+  ~ExamplesGuard() {
+    cudaStreamSynchronize(p->stream);
+    if (p->u_cap > kKeepRows) release_examples(p);
   }
-  ACO_PCUDA(p, alloc(Xd, x.size()), "alloc");
-  ACO_PCUDA(p, alloc(Yd, y.size()), "alloc");
-  ACO_PCUDA(p, copy_sync(p, *Xd, x.data(), x.size() * 2, cudaMemcpyHostToDevice), "upload x");
-  ACO_PCUDA(p, copy_sync(p, *Yd, y.data(), y.size() * 4, cudaMemcpyHostToDevice), "upload y");
+};
+
+// Uploads host examples (E x 12 FP32 features) and packs them into padded
+// BF16 rows p->ux, labels in p->uy, on the prior's stream.
+int upload_examples(aco_prior *p, const float *feats, const float *labels, int E, int B) {
+  if (B > p->u_cap) {
+    release_examples(p);
+    ACO_PCUDA(p, alloc(&p->ux, (size_t)B * kFeatPad), "alloc");
+    ACO_PCUDA(p, alloc(&p->uy, (size_t)B), "alloc");
+    ACO_PCUDA(p, alloc(&p->uf, (size_t)B * kFeatures), "alloc");
+    ACO_PCUDA(p, alloc(&p->uout, (size_t)B), "alloc");
+    p->u_cap = B;
+  }
+  ACO_PCUDA(p, cudaMemcpyAsync(p->uf, feats, (size_t)E * kFeatures * 4, cudaMemcpyHostToDevice,
+                               p->stream), "upload x");
+  if (labels)
+    ACO_PCUDA(p, cudaMemcpyAsync(p->uy, labels, (size_t)E * 4, cudaMemcpyHostToDevice, p->stream),
+              "upload y");
+  ACO_PCUDA(p, launch_pack_examples(p->uf, E, B, labels != nullptr, p->ux, p->uy, p->stream),
+            "pack examples");
   return ACO_OK;
 }
 
@@ -489,9 +503,10 @@ int aco_prior_loss_and_grads(aco_prior *p, const float *feats, const float *labe
   const int B = round_rows(E);
   const bool fused = p->engine == ACO_GEMM_FUSED;
   if (int s = fused ? ensure_fused(p, E) : ensure_workspace(p, B)) return s;
-  __nv_bfloat16 *X = nullptr;
-  float *Y = nullptr;
-  if (int s = upload_examples(p, feats, labels, E, B, &X, &Y)) return s;
+  ExamplesGuard guard{p};
+  if (int s = upload_examples(p, feats, labels, E, B)) return s;
+  const __nv_bfloat16 *X = p->ux;
+  const float *Y = p->uy;
   int s = ACO_OK;
   if (fused) {
     s = fused_pass(p, X, Y, E, pos_weight, nullptr, p->g, p->loss);
@@ -510,8 +525,6 @@ int aco_prior_loss_and_grads(aco_prior *p, const float *feats, const float *labe
     cudaMemsetAsync(p->g, 0, sizeof(float) * kParamCount, p->stream);
   }
   cudaStreamSynchronize(p->stream);
-  cudaFree(X);
-  cudaFree(Y);
   if (loss) *loss = h;
   return s ? s : gemm_status(p);
 }
@@ -521,24 +534,17 @@ int aco_prior_predict(aco_prior *p, const float *feats, int32_t E, float *probs)
   const int B = round_rows(E);
   const bool fused = p->engine == ACO_GEMM_FUSED;
   if (int s = fused ? ensure_fused(p, E) : ensure_workspace(p, B)) return s;
-  __nv_bfloat16 *X = nullptr;
-  float *Y = nullptr;
-  if (int s = upload_examples(p, feats, nullptr, E, B, &X, &Y)) return s;
-  float *out = p->out;
-  int s = ACO_OK;
-  if (fused && alloc(&out, (size_t)B) != cudaSuccess) s = ACO_ERR_OUT_OF_MEMORY;
-  if (!s)
-    s = fused ? fused_pass(p, X, nullptr, E, 1.0f, out, nullptr, nullptr)
-              : forward_backward(p, X, nullptr, B, E, 1.0f, false, out, nullptr);
+  ExamplesGuard guard{p};
+  if (int s = upload_examples(p, feats, nullptr, E, B)) return s;
+  const __nv_bfloat16 *X = p->ux;
+  float *out = fused ? p->uout : p->out;
+  int s = fused ? fused_pass(p, X, nullptr, E, 1.0f, out, nullptr, nullptr)
+                : forward_backward(p, X, nullptr, B, E, 1.0f, false, out, nullptr);
   if (!s) prefault(probs, (size_t)E * 4);
   if (!s && cudaMemcpyAsync(probs, out, (size_t)E * 4, cudaMemcpyDeviceToHost, p->stream) !=
                 cudaSuccess)
     s = ACO_ERR_CUDA;
   if (!s && cudaStreamSynchronize(p->stream) != cudaSuccess) s = ACO_ERR_CUDA;
-  cudaStreamSynchronize(p->stream);
-  if (fused) cudaFree(out);
-  cudaFree(X);
-  cudaFree(Y);
   return s ? s : gemm_status(p);
 }
 
@@ -663,7 +669,8 @@ void aco_prior_destroy(aco_prior *p) {
   if (p->stream) cudaStreamSynchronize(p->stream);
   void *bufs[] = {p->w, p->g, p->m1, p->m2, p->w1b, p->w2b, p->w2tb, p->X, p->Y, p->Z, p->H1,
                   p->H1t, p->H2, p->dZ2, p->dZ2t, p->dZ1t, p->Xt, p->dlogit, p->out, p->loss,
-                  p->scratch, p->gW1full, p->part, p->slots, p->ax, p->aprob};
+                  p->scratch, p->gW1full, p->part, p->slots, p->ax, p->aprob, p->ux, p->uy, p->uf,
+                  p->uout};
   for (void *b : bufs)
     if (b) cudaFree(b);
   if (p->stream) cudaStreamDestroy(p->stream);

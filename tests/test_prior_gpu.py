@@ -232,3 +232,40 @@ def test_training_learns_and_the_prior_helps():
     plain, learned, spent = _equal_time_runs(test, 30, pr, seed=3)
     assert all(b >= 1 for _, b in spent), spent
     assert learned.mean() < plain.mean(), (learned.mean(), plain.mean(), spent)
+
+
+@ENGINES
+def test_host_examples_after_a_larger_set(engine):
+    """Host examples are packed into kept buffers: padding rows and rows left
+    by a larger set change nothing.  Scores of a prefix equal the prefix of
+    the scores, a set's gradients those of a fresh prior, bit for bit (fixed
+    reduction order, whole set in one pass)."""
+    rng = np.random.default_rng(17)
+    X = rng.uniform(-1.0, 2.0, size=(20_000, 12)).astype(np.float32)
+    X[0, 3], X[1, 5] = 3.0e38, -1.0e-39  # beyond and below the BF16 range
+    y = (rng.random(len(X)) < 0.2).astype(np.float32)
+    pr = EdgePrior(seed=5, engine=engine)
+    whole = pr.predict(X)
+    for E in (1, 127, 128, 129, 255, 257, 4097):
+        assert np.array_equal(pr.predict(X[:E]), whole[:E], equal_nan=True), E
+        loss, g = pr.loss_and_grads(X[2:2 + E], y[2:2 + E], pos_weight=3.0)
+        l1, g1 = EdgePrior(seed=5, engine=engine).loss_and_grads(X[2:2 + E], y[2:2 + E],
+                                                                  pos_weight=3.0)
+        if engine == _abi.ACO_GEMM_FUSED:
+            assert loss == l1 and np.array_equal(g, g1), E
+        else:  # these reduce with atomics: FP32 sums in another order
+            assert abs(loss - l1) <= 1e-5 * abs(l1)
+            assert np.linalg.norm(g - g1) <= 1e-5 * np.linalg.norm(g1), E
+
+
+def test_host_examples_beyond_the_kept_size():
+    """A set above the kept size (2^21 rows) gives its buffers back; its
+    scores and the next call's are those of the small sets."""
+    rng = np.random.default_rng(3)
+    base = rng.uniform(-1.0, 2.0, size=(4096, 12)).astype(np.float32)
+    pr = EdgePrior(seed=5)
+    ref = pr.predict(base)
+    big = np.concatenate([np.tile(base, (512, 1)), base[:1]])
+    out = pr.predict(big)
+    assert np.array_equal(out[:-1].reshape(512, 4096), np.broadcast_to(ref, (512, 4096)))
+    assert out[-1] == ref[0] and np.array_equal(pr.predict(base), ref)
