@@ -49,7 +49,8 @@ cudaError_t launch_transpose_feats(const __nv_bfloat16 *X, int E, __nv_bfloat16 
 // The whole forward (and, with train, loss and backward) pass over `rows`
 // edges in one tcgen05 kernel (k_mlp_fused.cu); grid = mlp_fused_grid().
 // Training writes one partial row per CTA into part (ld >= kParamCount + 1,
-// a multiple of 4): the gradient in packed order, then the loss.
+// a multiple of 4): the gradient, W1 and W2 in the order that k_mlp_reduce
+// takes, then the loss.
 int mlp_fused_grid(int rows, int sms);
 cudaError_t launch_mlp_fused(bool train, const __nv_bfloat16 *X, int rows,
                              const __nv_bfloat16 *w1b, const __nv_bfloat16 *w2b, const float *w,

@@ -210,7 +210,7 @@ __device__ __forceinline__ void mma_rows(uint32_t d, const unsigned char *a, boo
 }  // namespace
 
 template <bool TRAIN>
-__global__ void __launch_bounds__(kThreadsF, 1)
+__global__ void __launch_bounds__(kThreadsF, TRAIN ? 1 : 2)
     k_mlp_fused(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW1,
                 const __grid_constant__ CUtensorMap tmW2,
                 const float *__restrict__ w, const float *__restrict__ labels, int rows,
@@ -525,8 +525,8 @@ __global__ void __launch_bounds__(kThreadsF, 1)
 // masters and refreshes their BF16 copies: W1 into its 16-wide padded rows,
 // W2 row-major and transposed.  `clear` zeroes the rows read (one row only,
 // the layered engines' sums in parameter order); without it W1 and W2 are in
-// k_mlp_fused's order: W1 [feature][unit], W2 [i / 4][o][i % 4].  Ten loads in
-// flight a thread: latency of the L2 bounds it, 5 us for 152 rows.
+// k_mlp_fused's order: W1 [feature][unit], W2 [i / 4][o][i % 4].  Bound by the latency
+// of a launch and of its loads from L2: 5 us for 152 rows.
 __global__ void __launch_bounds__(256)
     k_mlp_reduce(float *__restrict__ part, int G, int ld, int clear, float *__restrict__ gout,
                  float *__restrict__ loss_out, int adam, float *__restrict__ w,
@@ -538,10 +538,8 @@ __global__ void __launch_bounds__(256)
   const int t = blockIdx.x * 32 + tx;
   const bool live = t < kParamCount || (t == kParamCount && loss_out);
   float s = 0.0f;
-  if (live) {
-#pragma unroll 10
+  if (live)
     for (int c = ty; c < G; c += 8) s += part[(size_t)c * ld + t];
-  }
   sh[ty][tx] = s;
   __syncthreads();
   if (ty != 0 || !live) return;

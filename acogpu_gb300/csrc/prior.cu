@@ -247,7 +247,9 @@ int adam_step(aco_prior *p, float lr, float *part, int G, int ld, bool clear, fl
 int fused_pass(aco_prior *p, const __nv_bfloat16 *X, const float *Y, int rows, float pos_weight,
                float *probs, float *gout, float *loss_out) {
   if (int s = ensure_fused(p, rows)) return s;
-  const int G = mlp_fused_grid(rows, p->sms);
+  // Scoring fits twice on an SM: two tiles' chains overlap (18.4 -> 14.8 us for
+  // 100 003 rows); training takes the whole shared memory.
+  const int G = mlp_fused_grid(rows, Y ? p->sms : 2 * p->sms);
   uint32_t *err = reinterpret_cast<uint32_t *>(p->scratch + 2);
   ACO_PCUDA(p, launch_mlp_fused(Y != nullptr, X, rows, p->w1b, p->w2b, p->w, Y,
                                 pos_weight, (float)std::max(1, rows), probs, p->part, kPartLd, G,
