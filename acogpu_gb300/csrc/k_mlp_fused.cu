@@ -102,6 +102,14 @@ __device__ __forceinline__ uint32_t bf2_bits(float lo, float hi) {
   return u;
 }
 
+// The training pass and its reduction are launched so that one may start
+// while the other ends (launch_ordered): nothing that the other writes is
+// touched before grid_wait(), and it is read past L1 (its lines may be old).
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // bf16(relu(x)) of a pair.  The maximum is taken after the rounding (the same
 // value: rounding is monotonic and keeps 0) and drops NaN like fmaxf.
 __device__ __forceinline__ uint32_t relu2_bits(float lo, float hi) {
@@ -254,12 +262,16 @@ __global__ void __launch_bounds__(kThreadsF, TRAIN ? 1 : 2)
     reinterpret_cast<uint4 *>(sDZ)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
     fence_proxy_async();
   }
-  if (threadIdx.x < 128) {
-    b1s[threadIdx.x] = w[kParamB1 + threadIdx.x];
-    b2s[threadIdx.x] = w[kParamB2 + threadIdx.x];
-    w3s[threadIdx.x] = w[kParamW3 + threadIdx.x];
+  if (TRAIN) {
+    grid_wait();
+    grid_release();
   }
-  const float b3 = w[kParamB3];
+  if (threadIdx.x < 128) {
+    b1s[threadIdx.x] = __ldcg(w + kParamB1 + threadIdx.x);
+    b2s[threadIdx.x] = __ldcg(w + kParamB2 + threadIdx.x);
+    w3s[threadIdx.x] = __ldcg(w + kParamW3 + threadIdx.x);
+  }
+  const float b3 = __ldcg(w + kParamB3);
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
@@ -269,6 +281,7 @@ __global__ void __launch_bounds__(kThreadsF, TRAIN ? 1 : 2)
   int tile = blockIdx.x;
   bool x_inflight = false;  // thread 0: a TMA load of X not yet waited for
   if (threadIdx.x == 0 && tile < tiles) {
+    if (TRAIN) asm volatile("fence.proxy.async;" ::: "memory");  // weights of the last step
     mbar_arrive_expect_tx(bar_w, 3u * kKT);
     tma_load_2d(sW1, &tmW1, 0, 0, bar_w);
     tma_load_2d(sW2, &tmW2, 0, 0, bar_w);
@@ -538,8 +551,10 @@ __global__ void __launch_bounds__(256)
   const int t = blockIdx.x * 32 + tx;
   const bool live = t < kParamCount || (t == kParamCount && loss_out);
   float s = 0.0f;
+  grid_wait();
+  grid_release();
   if (live)
-    for (int c = ty; c < G; c += 8) s += part[(size_t)c * ld + t];
+    for (int c = ty; c < G; c += 8) s += __ldcg(part + (size_t)c * ld + t);
   sh[ty][tx] = s;
   __syncthreads();
   if (ty != 0 || !live) return;
@@ -559,11 +574,11 @@ __global__ void __launch_bounds__(256)
         ((t - kParamW2) & 3);
   if (gout) gout[k] = s;
   if (!adam) return;
-  const float a = b1 * m1[k] + (1.0f - b1) * s;
-  const float b = b2 * m2[k] + (1.0f - b2) * s * s;
+  const float a = b1 * __ldcg(m1 + k) + (1.0f - b1) * s;
+  const float b = b2 * __ldcg(m2 + k) + (1.0f - b2) * s * s;
   m1[k] = a;
   m2[k] = b;
-  const float v = w[k] - lr * (a / bc1) / (sqrtf(b / bc2) + eps);
+  const float v = __ldcg(w + k) - lr * (a / bc1) / (sqrtf(b / bc2) + eps);
   w[k] = v;
   const __nv_bfloat16 vb = __float2bfloat16_rn(v);
   if (k < kParamB1) {
@@ -573,6 +588,26 @@ __global__ void __launch_bounds__(256)
     w2b[o * kHidden + i] = vb;
     w2tb[i * kHidden + o] = vb;
   }
+}
+
+// A launch ordered behind the kernel before it in the stream, whose blocks may
+// start as that kernel's leave (each waits in grid_wait for its end): the
+// launch and the set-up of a training step's two kernels are hidden (44 steps
+// of 65536 rows: 1650 us with plain launches, 1555 us).
+template <typename... P, typename... A>
+static cudaError_t launch_ordered(void (*k)(P...), int grid, int threads, size_t smem,
+                                  cudaStream_t s, A... args) {
+  cudaLaunchAttribute a{};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &a;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
 }
 
 int mlp_fused_grid(int rows, int sms) {
@@ -609,11 +644,10 @@ cudaError_t launch_mlp_fused(bool train, const __nv_bfloat16 *X, int rows,
     configured |= 1ull << dev;
   }
   if (train)
-    k_mlp_fused<true><<<grid, kThreadsF, fused_smem<true>(), s>>>(
-        tx, t1, t2, w, labels, rows, pos_weight, norm, out, part, part_ld, err);
-  else
-    k_mlp_fused<false><<<grid, kThreadsF, fused_smem<false>(), s>>>(
-        tx, t1, t2, w, labels, rows, pos_weight, norm, out, part, part_ld, err);
+    return launch_ordered(k_mlp_fused<true>, grid, kThreadsF, fused_smem<true>(), s, tx, t1, t2, w,
+                          labels, rows, pos_weight, norm, out, part, part_ld, err);
+  k_mlp_fused<false><<<grid, kThreadsF, fused_smem<false>(), s>>>(
+      tx, t1, t2, w, labels, rows, pos_weight, norm, out, part, part_ld, err);
   return cudaGetLastError();
 }
 
@@ -623,9 +657,8 @@ cudaError_t launch_mlp_reduce(float *part, int G, int ld, bool clear, float *gou
                               __nv_bfloat16 *w2b, __nv_bfloat16 *w2tb, cudaStream_t s) {
   if (G < 1 || (clear && G != 1)) return cudaErrorInvalidValue;
   const int blocks = (kParamCount + 1 + 31) / 32;
-  k_mlp_reduce<<<blocks, 256, 0, s>>>(part, G, ld, clear ? 1 : 0, gout, loss_out, adam ? 1 : 0,
-                                       w, m1, m2, lr, b1, b2, eps, bc1, bc2, w1b, w2b, w2tb);
-  return cudaGetLastError();
+  return launch_ordered(k_mlp_reduce, blocks, 256, 0, s, part, G, ld, clear ? 1 : 0, gout, loss_out,
+                        adam ? 1 : 0, w, m1, m2, lr, b1, b2, eps, bc1, bc2, w1b, w2b, w2tb);
 }
 
 }  // namespace aco
