@@ -221,10 +221,198 @@ __global__ void __launch_bounds__(kSortMaxThreads)
           q < t2 ? (int32_t)(uint32_t)(keys[K + q] & 0xffffffffu) : -1;
 }
 
+// The same lists when only the first `need` entries of a row's order are
+// wanted (the candidates and the second tier): one warp a row, no block barrier.
+// It looks for a distance bound that between `need` and 32 R entries do not
+// exceed (bisection from the row's largest distance; a few passes over the row
+// in shared memory, as the count may fall anywhere in that range), copies those
+// entries out in city order, and sorts them as 64-bit keys in registers, R a
+// lane.  If no bound gives such a count -- more than 32 R - need equal distances
+// at the bound -- the entries below it are kept and the first of the equal ones
+// in city order, which is the order of their keys.  Rows of at most 32 R
+// entries are sorted whole.
+// Bound by instructions and shared memory, a few thousand cycles a row.  The
+// lists of n = 4096 (k + tier = 160) took 919 us by the whole sort, now 45; those
+// of 512 instances of 50 to 2000 cities (k = 20) 46 us each, now 8.
+constexpr int kSelectWarps = 4;
+constexpr int kMaxSelectRow = 8192;  // 4 x (32 KB + 2 KB)
+
+template <int R>
+__global__ void __launch_bounds__(kSelectWarps * 32)
+    k_nn_select_stable(const int32_t *__restrict__ dist, int n, int ld, int K, int ldk,
+                       int32_t *__restrict__ nn, int32_t *__restrict__ nn2, int t2,
+                       ColonyState *st) {
+  constexpr int CAP = 32 * R;
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row = blockIdx.x * kSelectWarps + warp;
+  if (row >= n) return;
+  const int chunks = (n + 127) >> 7;  // of 128 entries, four a lane
+  unsigned char *mine = smem + (size_t)warp * ((size_t)chunks * 512 + CAP * 8 + 128);
+  uint32_t *d = reinterpret_cast<uint32_t *>(mine);
+  uint64_t *keys = reinterpret_cast<uint64_t *>(mine + (size_t)chunks * 512);
+  uint64_t *bar = keys + CAP;
+  int ok = 0;
+  if (lane == 0) {
+    mbar_init(bar, 1);
+    fence_barrier_init();
+    const uint32_t bytes = (uint32_t)ld * 4u;
+    mbar_arrive_expect_tx(bar, bytes);
+    tma_load_1d(d, dist + (size_t)row * ld, bytes, bar);
+    ok = mbar_wait_bounded(bar, 0, st) ? 1 : 0;
+  }
+  if (!__shfl_sync(kFull, ok, 0)) return;
+  for (int q = n + lane; q < chunks * 128; q += 32) d[q] = ~0u;
+  __syncwarp();
+  const uint4 *d4 = reinterpret_cast<const uint4 *>(d);
+  const int pads = chunks * 128 - n, need = K + (nn2 ? t2 : 0);
+  const unsigned below = (1u << lane) - 1u;
+
+  // Entries up to `bound` are kept; with `ties`, only so many of those equal to it.
+  uint32_t bound = ~0u;
+  int ties = 0;
+  if (n > CAP) {
+    auto count = [&](uint32_t t) {
+      unsigned c = 0;
+      for (int i = 0; i < chunks; i++) {
+        const uint4 v = d4[32 * i + lane];
+        c += (v.x <= t ? 1u : 0u) + (v.y <= t ? 1u : 0u) + (v.z <= t ? 1u : 0u) +
+             (v.w <= t ? 1u : 0u);
+      }
+      return (int)__reduce_add_sync(kFull, c) - (t == ~0u ? pads : 0);
+    };
+    uint32_t lo = 0u, hi = 0u;  // the smallest bound with `need` entries is in [lo, hi]
+    for (int i = 0; i < chunks; i++) {
+      const uint4 v = d4[32 * i + lane];
+      const uint32_t e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const int city = 128 * i + 4 * lane + t;
+        if (city < n && city != row) hi = max(hi, e[t]);  // its own distance may be a sentinel
+      }
+    }
+    hi = __reduce_max_sync(kFull, hi);
+    int c_hi = count(hi), c_lo = 0;  // entries up to hi, and below lo
+    if (c_hi < need) {  // every entry wanted, the row's own among them
+      hi = ~0u;
+      c_hi = n;
+    }
+    while (c_hi > CAP && lo < hi) {
+      const uint32_t mid = lo + ((hi - lo) >> 1);
+      const int c = count(mid);
+      if (c >= need) {
+        hi = mid;
+        c_hi = c;
+      } else {
+        lo = mid + 1u;
+        c_lo = c;
+      }
+    }
+    bound = hi;
+    if (c_hi > CAP) ties = CAP - c_lo;  // lo == hi: the equal ones do not all fit
+  }
+  int kept = 0, seen = 0;
+  for (int i = 0; i < chunks; i++) {
+    const uint4 v = d4[32 * i + lane];
+    const uint32_t e[4] = {v.x, v.y, v.z, v.w};
+    const int city = 128 * i + 4 * lane;
+    bool f[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) f[t] = city + t < n && e[t] <= bound;
+    if (ties > 0) {
+      int r = seen;
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const unsigned b = __ballot_sync(kFull, f[t] && e[t] == bound);
+        r += __popc(b & below);
+        seen += __popc(b);
+      }
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const bool tie = f[t] && e[t] == bound;
+        if (tie && r >= ties) f[t] = false;
+        r += tie ? 1 : 0;
+      }
+    }
+    int pos = kept;
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      const unsigned b = __ballot_sync(kFull, f[t]);
+      pos += __popc(b & below);
+      kept += __popc(b);
+    }
+#pragma unroll
+    for (int t = 0; t < 4; t++)
+      if (f[t] && pos < CAP) keys[pos++] = ((uint64_t)e[t] << 32) | (uint32_t)(city + t);
+  }
+  for (int q = kept + lane; q < CAP; q += 32) keys[q] = ~0ull;
+  __syncwarp();
+  uint64_t x[R];  // the order in which they enter does not matter
+#pragma unroll
+  for (int r = 0; r < R; r++) x[r] = keys[32 * r + lane];
+  __syncwarp();
+  // Bitonic: lane l, register r holds index l R + r.
+#pragma unroll
+  for (int k = 2; k <= CAP; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      if (j >= R) {
+        const bool low = (lane & (j / R)) == 0, up = (lane * R & k) == 0;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          const uint64_t y = __shfl_xor_sync(kFull, x[r], j / R);
+          x[r] = ((x[r] < y) == (low == up)) ? x[r] : y;
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          if (r & j) continue;
+          const bool up = ((lane * R + r) & k) == 0;
+          const uint64_t a = x[r], b = x[r | j];
+          const bool swap = (a > b) == up;
+          x[r] = swap ? b : a;
+          x[r | j] = swap ? a : b;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; r++) keys[lane * R + r] = x[r];
+  __syncwarp();
+  for (int q = lane; q < ldk; q += 32)
+    nn[(size_t)row * ldk + q] = q < K ? (int32_t)(uint32_t)keys[q] : -1;
+  if (nn2)
+    for (int q = lane; q < kTier2; q += 32)
+      nn2[(size_t)row * kTier2 + q] = q < t2 ? (int32_t)(uint32_t)keys[K + q] : -1;
+}
+
+template <int R>
+static cudaError_t launch_select(const int32_t *dist, int n, int ld, int K, int ldk, int32_t *nn,
+                                 ColonyState *st, cudaStream_t s, int32_t *nn2, int t2) {
+  const size_t smem = (size_t)kSelectWarps * ((size_t)((n + 127) / 128) * 512 + 32 * R * 8 + 128);
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(k_nn_select_stable<R>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  k_nn_select_stable<R><<<(n + kSelectWarps - 1) / kSelectWarps, kSelectWarps * 32, smem, s>>>(
+      dist, n, ld, K, ldk, nn, nn2, t2, st);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_nn_sort_stable(const int32_t *dist, int n, int ld, int K, int ldk, int32_t *nn,
                                   ColonyState *st, cudaStream_t s, int32_t *nn2, int t2) {
   if (nn2 && (t2 < 0 || t2 > kTier2 || K + t2 > n - 1)) return cudaErrorInvalidValue;
   if (n > kMaxSortRow) return cudaErrorInvalidValue;
+  // Selection where the wanted entries leave the bisection room below the keys
+  // that a warp sorts, and four rows fit in shared memory.
+  const int need = K + (nn2 ? t2 : 0);
+  if (n <= kMaxSelectRow) {
+    if (n <= 128 || need <= 64)
+      return launch_select<4>(dist, n, ld, K, ldk, nn, st, s, nn2, t2);
+    if (n <= 256 || need <= 192)
+      return launch_select<8>(dist, n, ld, K, ldk, nn, st, s, nn2, t2);
+  }
   int P = 1;
   while (P < n) P <<= 1;
   if (P < 64) P = 64;  // one warp's keys, and the row's pitch fits (ld <= 2 P)

@@ -135,7 +135,7 @@ class ClockSampler:
         try:
             self.proc = subprocess.Popen(
                 ["nvidia-smi", "-i", str(self.device), f"--query-gpu={CLOCK_FIELDS}",
-                 "--format=csv,noheader,nounits", "-lms", "200"],
+                 "--format=csv,noheader,nounits", "-lms", "50"],
                 stdout=open(self.path, "w"), stderr=subprocess.DEVNULL)
         except (OSError, FileNotFoundError):
             self.proc = None
@@ -405,11 +405,19 @@ def parity_check(batch, insts, p, iters):
     return same, compared
 
 
-def rows_bytes(n, tours):
-    """Algorithmic bytes of the long-row construction: per ant-step one
-    candidate row staged (n choice values and n int16 ids) and the tour
-    write."""
-    return tours * (n - 1) * (6 * n + 4)
+def rows_l2_bytes(n, tours):
+    """Bytes that the long-row construction reads from L2: per ant-step the n
+    choice values of the current row, and values and ids of the first 128
+    nearest."""
+    return tours * (n - 1) * (4 * n + 6 * 128)
+
+
+def rows_bytes(n, m, count):
+    """Bytes that one long-row construction of `count` instances cannot do
+    without moving to or from memory: the choice matrix and the ids of the
+    first 128 nearest once, the tours and the successor and predecessor lists
+    out."""
+    return count * (4 * n * n + 256 * n + 12 * m * n)
 
 
 def run_parity(args, rank, world, local):
@@ -472,7 +480,8 @@ def run_parity(args, rank, world, local):
     if rank != 0:
         return None
     hbm = peaks().get("hbm_gbs")
-    per_launch = rows_bytes(PARITY_N, tours / args.steps)
+    per_launch = rows_bytes(PARITY_N, PARITY_N, PARITY_COUNT)
+    l2_launch = rows_l2_bytes(PARITY_N, tours / args.steps)
     construct_s = tune["construct_ms"] / 1e3
     achieved = per_launch / construct_s / 1e9 if construct_s > 0 else None
     return {
@@ -497,7 +506,11 @@ def run_parity(args, rank, world, local):
                      "algorithmic_bytes_per_launch": per_launch,
                      "construct_ms": tune["construct_ms"],
                      "traffic": profiled_traffic("construct_rows_parity_batch8.md"),
-                     "traffic_source": "profiles/construct_rows_parity_batch8.md (ncu)"},
+                     "traffic_source": "profiles/construct_rows_parity_batch8.md (ncu)",
+                     # the rows are read again by every ant, from L2: the kernel
+                     # is bound by issue and latency there, not by memory
+                     "l2_bytes_per_launch": l2_launch,
+                     "l2_read_gbs": l2_launch / construct_s / 1e9 if construct_s > 0 else None},
         "e2e": {"value": e_tours_all / e_wall, "unit": "tours/s",
                 "h2d_bytes_per_step": 8 * PARITY_N * PARITY_COUNT / args.steps,
                 "d2h_bytes_per_step": d2h / args.steps, "create_s": t_create,

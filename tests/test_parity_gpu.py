@@ -543,3 +543,28 @@ def test_reference_sort_edges(n, kind):
     assert np.array_equal(g.nn_list(), q.nn())
     g.close()
     q.close()
+
+
+@pytest.mark.parametrize("n,k", [(256, 200), (257, 64), (257, 65), (257, 192), (257, 193),
+                                 (700, 20), (700, 64), (700, 192), (700, 193), (8192, 32)])
+@pytest.mark.parametrize("kind", ["spread", "same", "far"])
+def test_stable_selection_edges(n, k, kind):
+    """Stable nn lists by selection: around the sizes and list lengths where
+    the rule changes, rows of distinct distances, of one value (no bound
+    separates the entries), and with one city much farther than the others."""
+    if kind != "spread" and n > 700:
+        pytest.skip("one large case is enough")
+    g0 = np.random.default_rng(n + k)
+    x, y = g0.integers(0, 1_000_000, (2, n)).astype(np.float32)
+    if kind == "same":
+        x[:] = 7.0
+        y[:] = 9.0
+    elif kind == "far":
+        x, y = (x // 10_000).astype(np.float32), (y // 10_000).astype(np.float32)
+        x[n // 2] = 40_000_000.0
+    d = instances.euc2d_distances(x, y)
+    p = params(num_ants=2, beta=1.0, cand_k=k, **FAST_MODE)
+    g = aco.Colony(d, params=p, num_ants=2)
+    g.initialize()
+    assert np.array_equal(g.nn_list(), np.argsort(d, axis=1, kind="stable")[:, :k])
+    g.close()
