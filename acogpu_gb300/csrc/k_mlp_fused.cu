@@ -32,7 +32,7 @@
 // The BF16 rounding points are those of the layered kernels in k_mlp.cu.
 //
 // What bounds it: the chain of a tile (three products, each waited for by the
-// epilogue that feeds the next), not bandwidth or the tensor pipe (3 % busy).
+// epilogue that feeds the next), not bandwidth or the tensor pipe (12 % busy).
 // So products that the chain does not need at once run under an epilogue (Z1
 // a tile ahead, dW2 and the sums behind dH1, dW1 behind the next tile), the
 // epilogues work on packed pairs (relu, masks) with 16-byte bias reads, and
