@@ -828,45 +828,54 @@ __device__ __forceinline__ void greedy_finish(const ColonyDev &c, int64_t len) {
 // candidate lists, which hold each row's cities in the order of (distance,
 // city): the next city is the first unvisited one of the list.  Warp 0 walks
 // the lists, one candidate a lane (the first 32): an id load, a lookup in the
-// tabu bits and one warp minimum a step.  The lists are copied to shared
-// memory when they fit (STAGED), else read from L2.  When a list has no
-// unvisited city left the whole CTA takes the minimum over the row.  The tour
+// tabu bits and one warp minimum a step.  The first SK entries of every list are
+// copied to shared memory (STAGED: as many as fit, a multiple of eight, or the
+// whole list), the others are read from L2 when those are visited, then the
+// fallback's second tier where the colony has one.  When no unvisited city is
+// left there either the whole CTA takes the minimum over the row.  The tour
 // stays in shared memory; its length is summed at the end, an edge a thread.
 // One CTA runs alone (16 in a batch's setup), so the step's latency is all
-// there is: n = 1000, k = 30 787 -> 113 us, n = 4096, k = 32 (from L2) 5.43 ->
-// 1.37 ms against the whole-row scan of every step below.
+// there is: n = 1000, k = 30 787 -> 113 us, n = 4096, k = 32 5.43 -> 0.82 ms (1.39
+// with the lists from L2 and no tier) against the whole-row scan of every step
+// below.
 constexpr int kGreedyNnThreads = 256;
-constexpr size_t kGreedyStageBytes = 160 * 1024;
+constexpr size_t kGreedyStageBytes = 200 * 1024;  // with 2 bytes a city more: below 227 KB
+
+// Entries of a list that are staged: 0 if not even eight fit.
+__host__ inline int greedy_staged(int n, int ldk) {
+  if ((size_t)n * ldk * 2 <= kGreedyStageBytes) return ldk;
+  return (int)(kGreedyStageBytes / ((size_t)n * 2)) / 8 * 8;  // below ldk
+}
 
 struct GreedyLayout {
   size_t tour_off, tabu_off, bytes;
 };
-__host__ __device__ inline GreedyLayout greedy_layout(int n, int ldk, bool staged) {
+__host__ __device__ inline GreedyLayout greedy_layout(int n, int sk) {
   GreedyLayout L;
-  L.tour_off = staged ? ((size_t)n * ldk * 2 + 15) / 16 * 16 : 0;
+  L.tour_off = ((size_t)n * sk * 2 + 15) / 16 * 16;
   L.tabu_off = L.tour_off + ((size_t)n * 2 + 15) / 16 * 16;
   L.bytes = L.tabu_off + (size_t)((n + 31) / 32) * 4;
   return L;
 }
 
 template <bool STAGED>
-__global__ void __launch_bounds__(kGreedyNnThreads) k_greedy_tau0_nn(ColonyDev c) {
+__global__ void __launch_bounds__(kGreedyNnThreads) k_greedy_tau0_nn(ColonyDev c, int sk) {
   extern __shared__ __align__(16) unsigned char smem_greedy[];
   __shared__ unsigned red_d[kGreedyNnThreads / 32], red_j[kGreedyNnThreads / 32];
   __shared__ unsigned long long red_len[kGreedyNnThreads / 32];
   __shared__ int s_cur, s_pos;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = c.n, words = (n + 31) >> 5;
-  const GreedyLayout L = greedy_layout(n, c.ldk, STAGED);
+  const GreedyLayout L = greedy_layout(n, STAGED ? sk : 0);
   int16_t *sids = reinterpret_cast<int16_t *>(smem_greedy);
   int16_t *tour = reinterpret_cast<int16_t *>(smem_greedy + L.tour_off);
   uint32_t *tabu = reinterpret_cast<uint32_t *>(smem_greedy + L.tabu_off);
-  if (STAGED)
-    for (int t = tid; t < n * c.ldk / 8; t += kGreedyNnThreads)  // ldk % 8 == 0, or its rest below
-      reinterpret_cast<uint4 *>(sids)[t] = __ldg(reinterpret_cast<const uint4 *>(c.nn16) + t);
-  if (STAGED)
-    for (int t = n * c.ldk / 8 * 8 + tid; t < n * c.ldk; t += kGreedyNnThreads)
-      sids[t] = c.nn16[t];
+  if (STAGED) {  // four entries a thread: ldk and sk are multiples of four
+    const int q = sk >> 2;
+    for (int t = tid; t < n * q; t += kGreedyNnThreads)
+      reinterpret_cast<uint2 *>(sids)[t] =
+          __ldg(reinterpret_cast<const uint2 *>(c.nn16 + (size_t)(t / q) * c.ldk) + t % q);
+  }
   for (int w = tid; w < words; w += kGreedyNnThreads) tabu[w] = w == 0 ? 1u : 0u;
   if (tid == 0) {
     tour[0] = 0;
@@ -874,17 +883,34 @@ __global__ void __launch_bounds__(kGreedyNnThreads) k_greedy_tau0_nn(ColonyDev c
     s_pos = 1;
   }
   __syncthreads();
-  const int16_t *ids = STAGED ? sids : c.nn16;
   const bool cand = lane < c.K && lane < c.ldk;
+  const bool near = cand && STAGED && lane < sk, far = cand && !near;
   for (int rounds = 0; rounds < n; rounds++) {  // one row scan a round: at most n - 1
     if (warp == 0) {
       int cur = s_cur, s = s_pos;
       while (s < n) {
-        const int id = cand ? (int)ids[(size_t)cur * c.ldk + lane] : -1;
-        const bool open = id >= 0 && !((tabu[id >> 5] >> (id & 31)) & 1u);
-        const unsigned m =
-            __reduce_min_sync(kFull, open ? ((unsigned)lane << 16) | (unsigned)id : ~0u);
-        if (m == ~0u) break;
+        auto open = [&](int id) { return id >= 0 && !((tabu[id >> 5] >> (id & 31)) & 1u); };
+        unsigned m = ~0u;
+        if (STAGED) {
+          const int id = near ? (int)sids[cur * sk + lane] : -1;
+          m = __reduce_min_sync(kFull, open(id) ? ((unsigned)lane << 16) | (unsigned)id : ~0u);
+        }
+        if (m == ~0u) {
+          if (!STAGED || sk < c.K) {
+            const int id = far ? (int)c.nn16[(size_t)cur * c.ldk + lane] : -1;
+            m = __reduce_min_sync(kFull, open(id) ? ((unsigned)lane << 16) | (unsigned)id : ~0u);
+          }
+          if (m == ~0u && c.t2 > 0 && c.K <= 32) {  // the next t2 of the order, -1 past them
+            const int4 v =
+                __ldg(reinterpret_cast<const int4 *>(c.nn2 + (size_t)cur * kTier2) + lane);
+            unsigned k = open(v.w) ? (unsigned)v.w : ~0u;
+            if (open(v.z)) k = (unsigned)v.z;
+            if (open(v.y)) k = (unsigned)v.y;
+            if (open(v.x)) k = (unsigned)v.x;
+            m = __reduce_min_sync(kFull, k != ~0u ? ((unsigned)lane << 16) | k : ~0u);
+          }
+          if (m == ~0u) break;
+        }
         cur = (int)(m & 0xffffu);
         if (lane == 0) {
           tabu[cur >> 5] |= 1u << (cur & 31);
@@ -1020,15 +1046,15 @@ __global__ void __launch_bounds__(kGreedyThreads)
 cudaError_t launch_greedy_tau0(const ColonyDev &c, int tau0_mode, float tau0_value,
                                bool stable_lists, cudaStream_t s) {
   if (tau0_mode == ACO_TAU0_DORIGO && stable_lists && c.nn16 && c.n < 32768) {
-    const bool staged = (size_t)c.n * c.ldk * 2 <= kGreedyStageBytes;
-    const size_t smem = greedy_layout(c.n, c.ldk, staged).bytes;
-    void (*fn)(ColonyDev) = staged ? k_greedy_tau0_nn<true> : k_greedy_tau0_nn<false>;
+    const int sk = greedy_staged(c.n, c.ldk);
+    const size_t smem = greedy_layout(c.n, sk).bytes;
+    void (*fn)(ColonyDev, int) = sk > 0 ? k_greedy_tau0_nn<true> : k_greedy_tau0_nn<false>;
     if (smem > 48 * 1024) {
       const cudaError_t e =
           cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
     }
-    fn<<<1, kGreedyNnThreads, smem, s>>>(c);
+    fn<<<1, kGreedyNnThreads, smem, s>>>(c, sk);
     return cudaGetLastError();
   }
   const size_t smem = (size_t)((c.n + 31) / 32) * 4;

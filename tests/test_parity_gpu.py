@@ -568,3 +568,33 @@ def test_stable_selection_edges(n, k, kind):
     g.initialize()
     assert np.array_equal(g.nn_list(), np.argsort(d, axis=1, kind="stable")[:, :k])
     g.close()
+
+
+@pytest.mark.parametrize("n,k,lattice", [(4096, 32, 0), (4100, 32, 1), (6500, 32, 0), (7000, 20, 1),
+                                         (12801, 16, 0)])
+@pytest.mark.parametrize("variant", [_abi.ACO_ANT_SYSTEM, _abi.ACO_RANK_BASED])
+def test_greedy_tau0_with_part_of_the_lists_staged(n, k, lattice, variant):
+    """Lists too long for shared memory: the first 24 or 8 entries are staged,
+    or none, the rest read from L2, then the second tier (Ant System)."""
+    if variant == _abi.ACO_RANK_BASED and n > 10_000:
+        pytest.skip("one case without staged lists is enough")
+    if lattice:
+        side = int(np.ceil(np.sqrt(n)))
+        gx, gy = np.meshgrid(np.arange(side, dtype=np.float32), np.arange(side, dtype=np.float32))
+        x, y = gx.ravel()[:n], gy.ravel()[:n]
+    else:
+        x, y = instances.uniform_instance(n, seed=n, box=100_000)
+    p = params(num_ants=2, variant=variant, rank_w=6, beta=2.0, rho=0.2, cand_k=k, seed=k,
+               **FAST_MODE)
+    g = aco.Colony(coords=(x, y), params=p, num_ants=2)
+    g.initialize()
+    d = g.distances()
+    cur, length = 0, 0
+    left = np.arange(1, n)
+    for _ in range(n - 1):
+        i = int(np.argmin(d[cur, left]))  # `left` stays in city order: the lowest of a tie
+        length += int(d[cur, left[i]])
+        cur = int(left[i])
+        left = np.delete(left, i)
+    assert g.stats()["greedy_length"] == length + int(d[cur, 0])
+    g.close()
