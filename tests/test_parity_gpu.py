@@ -598,3 +598,33 @@ def test_greedy_tau0_with_part_of_the_lists_staged(n, k, lattice, variant):
         left = np.delete(left, i)
     assert g.stats()["greedy_length"] == length + int(d[cur, 0])
     g.close()
+
+
+@pytest.mark.parametrize("kind", ["dense", "half", "limit", "fraction", "mixed", "huge"])
+def test_distances_on_both_paths(kind):
+    """Rounded distances by whole numbers and by the double root: many equal
+    and neighbouring values, sums of squares at k^2 + k and next to it,
+    differences at and past 2^22, fractions, both kinds in one instance, and
+    differences far beyond the whole-number path."""
+    g0 = np.random.default_rng(len(kind))
+    n = 600
+    if kind == "dense":
+        x, y = g0.integers(-20, 20, (2, n))
+    elif kind == "half":
+        k = g0.integers(1, 1 << 20, n)
+        x, y = k, np.sqrt(k).astype(np.int64)
+        x[0] = y[0] = 0
+    elif kind == "limit":
+        e = 1 << 22
+        x = g0.choice([-e, -e + 1, -1, 0, 1, 2, e - 1, e, e + 1, e + 2], n)
+        y = g0.choice([-2, 0, 1, 2047, 2048, e, e + 1], n)
+    elif kind == "fraction":
+        x, y = g0.random((2, n)) * 1000
+    elif kind == "mixed":
+        x, y = g0.integers(0, 10_000, (2, n)) * g0.choice([1.0, 0.5, 0.1], n)
+    else:
+        x, y = g0.random((2, n)) * 1e9
+    x, y = np.asarray(x, np.float32), np.asarray(y, np.float32)
+    g = aco.Colony(coords=(x, y), params=params(num_ants=2, cand_k=8, **FAST_MODE), num_ants=2)
+    assert np.array_equal(g.distances(), instances.euc2d_distances(x, y))
+    g.close()
