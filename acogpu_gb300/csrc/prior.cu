@@ -12,6 +12,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <mutex>
 #include <new>
 #include <random>
 #include <string>
@@ -53,6 +54,8 @@ struct aco_prior {
   float *aprob = nullptr;
   int64_t a_cap = 0;
   // examples of the calls on host data: BF16 rows, labels, raw rows, scores
+  // (one such call at a time: `examples` is held from the upload to the read)
+  std::mutex examples;
   __nv_bfloat16 *ux = nullptr;
   float *uy = nullptr, *uf = nullptr, *uout = nullptr;
   int64_t u_cap = 0;
@@ -272,9 +275,12 @@ void release_examples(aco_prior *p) {
   p->u_cap = 0;
 }
 
-// Ends a call on host examples: nothing of the caller's is in use any more.
+// A call on host examples: alone in the kept buffers from its upload to its
+// end, when nothing of the caller's is in use any more.
 struct ExamplesGuard {
   aco_prior *p;
+  std::lock_guard<std::mutex> alone;
+  explicit ExamplesGuard(aco_prior *q) : p(q), alone(q->examples) {}
   ~ExamplesGuard() {
     cudaStreamSynchronize(p->stream);
     if (p->u_cap > kKeepRows) release_examples(p);
@@ -504,8 +510,8 @@ int aco_prior_loss_and_grads(aco_prior *p, const float *feats, const float *labe
   if (!p || !feats || !labels || E < 1 || !grads) return ACO_ERR_INVALID_ARGUMENT;
   const int B = round_rows(E);
   const bool fused = p->engine == ACO_GEMM_FUSED;
+  ExamplesGuard guard(p);
   if (int s = fused ? ensure_fused(p, E) : ensure_workspace(p, B)) return s;
-  ExamplesGuard guard{p};
   if (int s = upload_examples(p, feats, labels, E, B)) return s;
   const __nv_bfloat16 *X = p->ux;
   const float *Y = p->uy;
@@ -535,8 +541,8 @@ int aco_prior_predict(aco_prior *p, const float *feats, int32_t E, float *probs)
   if (!p || !feats || E < 1 || !probs) return ACO_ERR_INVALID_ARGUMENT;
   const int B = round_rows(E);
   const bool fused = p->engine == ACO_GEMM_FUSED;
+  ExamplesGuard guard(p);
   if (int s = fused ? ensure_fused(p, E) : ensure_workspace(p, B)) return s;
-  ExamplesGuard guard{p};
   if (int s = upload_examples(p, feats, nullptr, E, B)) return s;
   const __nv_bfloat16 *X = p->ux;
   float *out = fused ? p->uout : p->out;

@@ -393,6 +393,9 @@ ACO_API int aco_prior_train(aco_prior *p, int32_t epochs, int32_t batch, float l
 /* Loss and packed gradient of a batch given on the host (E x 12 features). */
 ACO_API int aco_prior_loss_and_grads(aco_prior *p, const float *feats, const float *labels,
                                      int32_t E, float pos_weight, float *loss, float *grads);
+/* Several threads may call aco_prior_predict and aco_prior_loss_and_grads with
+ * one prior at once (they take turns); any other call on it needs the prior
+ * to itself. */
 ACO_API int aco_prior_predict(aco_prior *p, const float *feats, int32_t E, float *probs);
 /* Scores the colony's candidate edges and installs the prior. */
 ACO_API int aco_prior_apply(aco_prior *p, aco_colony *c, float floor);

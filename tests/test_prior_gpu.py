@@ -1,6 +1,7 @@
 """GPU tests of the learned heuristic prior: features, the MLP's forward and
 backward kernels against the CPU oracle, parity of a colony that uses the
 prior, and what training buys over the plain method."""
+import threading
 import time
 
 import numpy as np
@@ -269,3 +270,41 @@ def test_host_examples_beyond_the_kept_size():
     out = pr.predict(big)
     assert np.array_equal(out[:-1].reshape(512, 4096), np.broadcast_to(ref, (512, 4096)))
     assert out[-1] == ref[0] and np.array_equal(pr.predict(base), ref)
+
+
+@ENGINES
+def test_threads_score_with_one_prior(engine):
+    """Host examples of several threads share the prior's kept buffers: every
+    thread gets its own rows' scores and gradients, also while another thread's
+    larger set makes the buffers grow or go back."""
+    rng = np.random.default_rng(29)
+    sizes = (5, 130, 4097, 20_000, (1 << 21) + 1)
+    sets = []
+    for E in sizes:
+        X = rng.uniform(-1.0, 2.0, size=(E, 12)).astype(np.float32)
+        sets.append((X, (rng.random(E) < 0.2).astype(np.float32)))
+    pr = EdgePrior(seed=5, engine=engine)
+    alone = [(pr.predict(X), pr.loss_and_grads(X, y, pos_weight=3.0)) for X, y in sets]
+    wrong, start = [], threading.Barrier(len(sets))
+
+    def score(i):
+        (X, y), (probs, (loss, grads)) = sets[i], alone[i]
+        try:
+            start.wait()
+            for _ in range(4 if len(X) > 1 << 20 else 40):
+                if not np.array_equal(pr.predict(X), probs):
+                    wrong.append((len(X), "scores"))
+                l1, g1 = pr.loss_and_grads(X, y, pos_weight=3.0)
+                # the layered engines reduce with atomics, in any order
+                if engine == _abi.ACO_GEMM_FUSED and not (l1 == loss and np.array_equal(g1, grads)):
+                    wrong.append((len(X), "gradients"))
+        except Exception as e:  # a thread's failure is the test's
+            wrong.append((len(X), repr(e)))
+
+    threads = [threading.Thread(target=score, args=(i,)) for i in range(len(sets))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong[:5]
+    pr.close()
