@@ -9,6 +9,21 @@
 
 namespace aco {
 
+// Lets `fn` be launched with `need` bytes of dynamic shared memory beside its
+// `fixed` static ones.  The limit belongs to the kernel, for every colony and
+// host thread, so it is always set to the most that the device allows: set to
+// one colony's need, it made the launches of a larger colony fail.
+inline cudaError_t open_smem(const void *fn, size_t need, int fixed = 0) {
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e != cudaSuccess) return e;
+  most -= fixed;
+  if (most < 0 || need > (size_t)most) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 // ---- setup (k_setup.cu) ----
 cudaError_t launch_distances_from_coords(const float *x, const float *y, int n, int ld,
                                          int32_t *dist, cudaStream_t s);

@@ -314,36 +314,30 @@ size_t construct_staged_smem_bytes(int n, int ld, int sp, bool aging) {
 }
 
 cudaError_t configure_construct(size_t smem) {
-  const int v = (int)smem;
-  cudaError_t e = cudaFuncSetAttribute(k_construct<true, true>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, v);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_construct<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_construct<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_construct<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
+  cudaError_t e = open_smem((const void *)k_construct<true, true>, smem);
+  if (e == cudaSuccess) e = open_smem((const void *)k_construct<true, false>, smem);
+  if (e == cudaSuccess) e = open_smem((const void *)k_construct<false, true>, smem);
+  if (e == cudaSuccess) e = open_smem((const void *)k_construct<false, false>, smem);
   return e;
 }
 
 namespace {
 template <bool AGING, int TW, int G, bool TIER>
-cudaError_t staged_attr(int v) {
-  return cudaFuncSetAttribute(k_construct_staged<AGING, TW, G, TIER>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, v);
+cudaError_t staged_attr(size_t smem) {
+  return open_smem((const void *)k_construct_staged<AGING, TW, G, TIER>, smem, 128);
 }
 template <int G, bool TIER>
-cudaError_t staged_attr_tier(int v) {
-  cudaError_t e = staged_attr<true, 1, G, TIER>(v);
-  if (e == cudaSuccess) e = staged_attr<false, 1, G, TIER>(v);
-  if (e == cudaSuccess) e = staged_attr<true, 2, G, TIER>(v);
-  if (e == cudaSuccess) e = staged_attr<false, 2, G, TIER>(v);
+cudaError_t staged_attr_tier(size_t smem) {
+  cudaError_t e = staged_attr<true, 1, G, TIER>(smem);
+  if (e == cudaSuccess) e = staged_attr<false, 1, G, TIER>(smem);
+  if (e == cudaSuccess) e = staged_attr<true, 2, G, TIER>(smem);
+  if (e == cudaSuccess) e = staged_attr<false, 2, G, TIER>(smem);
   return e;
 }
 template <int G>
-cudaError_t staged_attr_all(int v) {
-  cudaError_t e = staged_attr_tier<G, false>(v);
-  if (e == cudaSuccess) e = staged_attr_tier<G, true>(v);
+cudaError_t staged_attr_all(size_t smem) {
+  cudaError_t e = staged_attr_tier<G, false>(smem);
+  if (e == cudaSuccess) e = staged_attr_tier<G, true>(smem);
   return e;
 }
 template <int G, bool TIER>
@@ -372,11 +366,10 @@ cudaError_t staged_launch(const ColonyDev &c, const int16_t *nn16, int grid, int
 }  // namespace
 
 cudaError_t configure_construct_staged(size_t smem) {
-  const int v = (int)smem;
-  cudaError_t e = staged_attr_all<4>(v);
-  if (e == cudaSuccess) e = staged_attr_all<5>(v);
-  if (e == cudaSuccess) e = staged_attr_all<6>(v);
-  if (e == cudaSuccess) e = staged_attr_all<8>(v);
+  cudaError_t e = staged_attr_all<4>(smem);
+  if (e == cudaSuccess) e = staged_attr_all<5>(smem);
+  if (e == cudaSuccess) e = staged_attr_all<6>(smem);
+  if (e == cudaSuccess) e = staged_attr_all<8>(smem);
   return e;
 }
 

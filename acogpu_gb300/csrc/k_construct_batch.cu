@@ -123,9 +123,9 @@ size_t batch_staged_table_bytes(int n, int ld, int sp, bool aging) {
 
 namespace {
 template <bool MULTI, bool AGING, int G>
-cudaError_t batch_attr(int v) {
-  return cudaFuncSetAttribute(k_batch_construct<MULTI, AGING, G>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, v);
+cudaError_t batch_attr(size_t smem) {
+  return open_smem((const void *)k_batch_construct<MULTI, AGING, G>, smem,
+                   (sizeof(ColonyDev) + 8 + 127) / 128 * 128);
 }
 template <bool MULTI, bool AGING, int G>
 cudaError_t batch_launch(const ColonyDev *descs, const int4 *items, int num_items, int *queue_head,
@@ -151,17 +151,16 @@ const void *batch_fn_for(bool multi, int sp, bool aging) {
 }  // namespace
 
 cudaError_t configure_batch_construct(size_t smem) {
-  const int v = (int)smem;
-  cudaError_t e = batch_attr<true, true, 8>(v);
-  if (e == cudaSuccess) e = batch_attr<true, false, 8>(v);
-  if (e == cudaSuccess) e = batch_attr<false, true, 4>(v);
-  if (e == cudaSuccess) e = batch_attr<false, false, 4>(v);
-  if (e == cudaSuccess) e = batch_attr<false, true, 5>(v);
-  if (e == cudaSuccess) e = batch_attr<false, false, 5>(v);
-  if (e == cudaSuccess) e = batch_attr<false, true, 6>(v);
-  if (e == cudaSuccess) e = batch_attr<false, false, 6>(v);
-  if (e == cudaSuccess) e = batch_attr<false, true, 8>(v);
-  if (e == cudaSuccess) e = batch_attr<false, false, 8>(v);
+  cudaError_t e = batch_attr<true, true, 8>(smem);
+  if (e == cudaSuccess) e = batch_attr<true, false, 8>(smem);
+  if (e == cudaSuccess) e = batch_attr<false, true, 4>(smem);
+  if (e == cudaSuccess) e = batch_attr<false, false, 4>(smem);
+  if (e == cudaSuccess) e = batch_attr<false, true, 5>(smem);
+  if (e == cudaSuccess) e = batch_attr<false, false, 5>(smem);
+  if (e == cudaSuccess) e = batch_attr<false, true, 6>(smem);
+  if (e == cudaSuccess) e = batch_attr<false, false, 6>(smem);
+  if (e == cudaSuccess) e = batch_attr<false, true, 8>(smem);
+  if (e == cudaSuccess) e = batch_attr<false, false, 8>(smem);
   return e;
 }
 

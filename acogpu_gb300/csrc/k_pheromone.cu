@@ -273,12 +273,10 @@ static cudaError_t launch_rows_t(const ColonyDev &c, int threads, cudaStream_t s
 
 template <bool EVAP, bool DEPOSIT, bool WRITE_TAU>
 static cudaError_t configure_t(int ld) {
-  const int v = (int)rows_smem(ld, DEPOSIT);
-  cudaError_t e = cudaFuncSetAttribute(k_pheromone_rows<EVAP, DEPOSIT, WRITE_TAU>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, v);
+  const size_t smem = rows_smem(ld, DEPOSIT);
+  cudaError_t e = open_smem((const void *)k_pheromone_rows<EVAP, DEPOSIT, WRITE_TAU>, smem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_batch_pheromone_rows<EVAP, DEPOSIT, WRITE_TAU>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, v);
+    e = open_smem((const void *)k_batch_pheromone_rows<EVAP, DEPOSIT, WRITE_TAU>, smem);
   return e;
 }
 
