@@ -42,7 +42,11 @@ int fail(aco_colony *c, int status, const std::string &msg) {
   return status;
 }
 
+// The runtime keeps a failed call's error until it is read, and a launch
+// reports whatever it finds there: every error returned is read here, so that
+// the next call on another colony does not fail for it.
 int cuda_fail(aco_colony *c, cudaError_t e, const char *what) {
+  cudaGetLastError();
   std::string msg = std::string(what) + ": " + cudaGetErrorString(e);
   if (e == cudaErrorMemoryAllocation) return fail(c, ACO_ERR_OUT_OF_MEMORY, msg);
   return fail(c, ACO_ERR_CUDA, msg);
@@ -486,6 +490,7 @@ int aco_colony_create(const aco_params *params, const int32_t *dist, int32_t n,
   if (e == cudaSuccess) e = launch_fill_padding_int(c->dist, n, c->ld, ACO_MAX_DISTANCE, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
+    cudaGetLastError();
     aco_colony_destroy(c);
     return ACO_ERR_CUDA;
   }
@@ -511,6 +516,7 @@ int aco_colony_create_coords(const aco_params *params, const float *x, const flo
   if (e == cudaSuccess) e = launch_distances_from_coords(dxy, dxy + n, n, c->ld, c->dist, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
+    cudaGetLastError();
     aco_colony_destroy(c);
     return ACO_ERR_CUDA;
   }
@@ -720,6 +726,7 @@ int aco_colony_run(aco_colony *c, int32_t iterations) {
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (s) {
       if (g) cudaGraphDestroy(g);
+      cudaGetLastError();
       return s;
     }
     if (e != cudaSuccess) return cuda_fail(c, e, "end capture");
@@ -1043,9 +1050,11 @@ int bfail(aco_batch *b, int status, const std::string &msg) {
 #define ACO_BCUDA(b, call, what)                                                         \
   do {                                                                                   \
     cudaError_t e_ = (call);                                                             \
-    if (e_ != cudaSuccess)                                                               \
+    if (e_ != cudaSuccess) {                                                             \
+      cudaGetLastError(); /* as in cuda_fail */                                          \
       return bfail(b, e_ == cudaErrorMemoryAllocation ? ACO_ERR_OUT_OF_MEMORY : ACO_ERR_CUDA, \
                    std::string(what) + ": " + cudaGetErrorString(e_));                   \
+    }                                                                                    \
   } while (0)
 
 void batch_drop_graph(aco_batch *b) {

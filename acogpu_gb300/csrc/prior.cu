@@ -74,9 +74,11 @@ int pfail(aco_prior *p, int status, const std::string &msg) {
 #define ACO_PCUDA(p, call, what)                                                           \
   do {                                                                                     \
     cudaError_t e_ = (call);                                                               \
-    if (e_ != cudaSuccess)                                                                 \
+    if (e_ != cudaSuccess) {                                                               \
+      cudaGetLastError(); /* read, or the next launch would report it */                   \
       return pfail(p, e_ == cudaErrorMemoryAllocation ? ACO_ERR_OUT_OF_MEMORY : ACO_ERR_CUDA, \
                    std::string(what) + ": " + cudaGetErrorString(e_));                    \
+    }                                                                                      \
   } while (0)
 
 template <class T>

@@ -8,6 +8,7 @@ import pytest
 import acogpu_gb300 as aco
 from acogpu_gb300 import _abi
 from acogpu_gb300.colony import AcoError, lib
+from acogpu_gb300.prior import EdgePrior
 from helpers import instance, params
 
 pytestmark = pytest.mark.gpu
@@ -60,3 +61,35 @@ def test_injected_allocation_failure_is_clean(after):
     assert abs(torch.cuda.mem_get_info()[0] - free0) < (4 << 20)  # nothing left behind
     (b0, t0), (b1, t1) = run_twice_same()
     assert b0 == b1 and np.array_equal(t0, t1)
+
+
+def test_a_refused_allocation_does_not_fail_the_next_calls():
+    """A colony far larger than the device's memory is refused; what exists and
+    what is created next works as if it had not been asked for."""
+    import torch
+    x, y, _ = instance(80, 3)
+    p = params(num_ants=16, beta=2.0, rho=0.2, cand_k=10, seed=3, **FAST)
+    q = params(num_ants=16, cand_k=10, **{**FAST, "nn_order": _abi.ACO_NN_REFERENCE_QSORT})
+    far = np.arange(1 << 20, dtype=np.float32)  # matrices of 4 TB
+
+    def refuse():
+        with pytest.raises(AcoError) as err:
+            aco.Colony(coords=(far, far), params=q, num_ants=16)
+        assert err.value.status == _abi.ACO_ERR_OUT_OF_MEMORY
+
+    refuse()
+    c = aco.Colony(coords=(x, y), params=p, num_ants=16)
+    c.initialize()
+    refuse()
+    c.run(2)
+    c.synchronize()
+    b = aco.Batch([(x, y)], params=p, num_ants=16)
+    refuse()
+    b.initialize()
+    refuse()
+    b.run(1)
+    b.synchronize()
+    pr = EdgePrior(seed=1)
+    refuse()
+    pr.predict(np.zeros((5, 12), np.float32))
+    torch.cuda.synchronize()
