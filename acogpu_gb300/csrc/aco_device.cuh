@@ -47,7 +47,7 @@ struct ColonyState {
   uint32_t error;
   int32_t error_info;
   float tau0;
-  int32_t greedy_pad;
+  int32_t signed_weights;  // a pheromone or heuristic value is negative (or was, since the reset)
   int64_t greedy_length;   // C_nn
   int64_t fallbacks;       // steps resolved by the fallback rule
   int64_t tours_built;     // valid ants that built a tour, summed over iterations
@@ -86,6 +86,7 @@ struct ColonyDev {
   float *t2v;
   float *mout;
   int t2;
+  int is_signed;  // weights may be negative (the general kernel's case)
   ColonyState *st;
   float rho, alpha;
   int use_alpha;

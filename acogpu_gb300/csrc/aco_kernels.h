@@ -28,6 +28,9 @@ inline cudaError_t open_smem(const void *fn, size_t need, int fixed = 0) {
 cudaError_t launch_distances_from_coords(const float *x, const float *y, int n, int ld,
                                          int32_t *dist, cudaStream_t s);
 cudaError_t launch_fill_padding_int(int32_t *mat, int n, int ld, int32_t value, cudaStream_t s);
+// Sets *out to 1 if a distance is negative (*out cleared before).
+cudaError_t launch_negative_distance(const int32_t *dist, int n, int ld, int32_t *out,
+                                     cudaStream_t s);
 cudaError_t launch_max_distance(const int32_t *dist, int n, int ld, int32_t *out, cudaStream_t s);
 cudaError_t launch_heuristic_device(const int32_t *dist, int n, int ld, float beta, float *eta,
                                     cudaStream_t s);

@@ -202,7 +202,7 @@ int aco_colony_load(aco_colony *c, const char *path) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_status(c, e, "restore colony state");
   c->optimum = h.optimum;
-  return ACO_OK;
+  return colony_check_signs(c, false);
 }
 
 }  // extern "C"

@@ -131,6 +131,7 @@ ColonyDev make_dev(const aco_colony *c) {
   d.min_pop = c->p.min_population_limit;
   d.variant = c->p.variant; d.rank_w = c->p.rank_w; d.fallback = c->p.fallback;
   d.seed = c->p.seed;
+  d.is_signed = c->is_signed;
   return d;
 }
 
@@ -266,14 +267,34 @@ int aco::colony_fail(aco_colony *c, int status, const std::string &msg) {
 
 namespace {
 
-int device_error(aco_colony *c) {
-  ColonyState h;
-  ACO_CUDA(c, cudaMemcpyAsync(&h, c->st, sizeof(h), cudaMemcpyDeviceToHost, c->stream),
-           "read state");
-  ACO_CUDA(c, cudaStreamSynchronize(c->stream), "synchronize");
+int plan_construction(aco_colony *c);
+
+// Takes in whether weights may be negative; a change re-plans construction.
+int take_signs(aco_colony *c, const ColonyState &h) {
+  const bool now = c->neg_dist || h.signed_weights != 0;
+  if (now == c->is_signed) return ACO_OK;
+  c->is_signed = now;
+  drop_graph(c);
+  return plan_construction(c);
+}
+
+int error_of(aco_colony *c, const ColonyState &h) {
   if (h.error & kErrTimeout) return fail(c, ACO_ERR_DEVICE_TIMEOUT, "a bounded device wait expired");
   if (h.error & kErrCheck) return fail(c, ACO_ERR_DEVICE_CHECK, "a device-side check failed");
   return ACO_OK;
+}
+
+int wait_state(aco_colony *c, ColonyState *h) {
+  ACO_CUDA(c, cudaMemcpyAsync(h, c->st, sizeof(*h), cudaMemcpyDeviceToHost, c->stream),
+           "read state");
+  ACO_CUDA(c, cudaStreamSynchronize(c->stream), "synchronize");
+  return ACO_OK;
+}
+
+int device_error(aco_colony *c) {
+  ColonyState h;
+  if (int s = wait_state(c, &h)) return s;
+  return error_of(c, h);
 }
 
 int read_state(aco_colony *c, ColonyState *h) {
@@ -318,7 +339,8 @@ cudaError_t launch_construction(aco_colony *c, const ColonyDev &d) {
 // candidate table in shared memory, one CTA per SM) when the table fits, else
 // the cluster kernel (the table split over ceil(n/1024) CTAs, n <= 8192),
 // else the direct kernel (the same step loop on rows read from L2); otherwise,
-// and in ACO_CONSTRUCT_GLOBAL mode, the general global-memory kernel.  The
+// in ACO_CONSTRUCT_GLOBAL mode and where weights may be negative, the general
+// global-memory kernel.  The
 // k <= 32 kernels put one ant per warp.  For k > 32 (mode AUTO or ROWS) the
 // long-row kernel: one warp per ant, the ants spread evenly over the SMs.
 int plan_construction(aco_colony *c) {
@@ -328,6 +350,7 @@ int plan_construction(aco_colony *c) {
   c->rows = false;
   const int mode = c->p.construct_mode;
   const int sms = c->num_sms > 0 ? c->num_sms : 1;
+  if (c->is_signed) return ACO_OK;
   if (c->nn16 && c->n <= kRowsMaxCities && c->K > 32 &&
       (mode == ACO_CONSTRUCT_ROWS || mode == ACO_CONSTRUCT_AUTO)) {
     int ants = c->tune_warps > 0 ? c->tune_warps : (c->m + sms - 1) / sms;
@@ -435,6 +458,14 @@ int read_matrix_f32(aco_colony *c, const float *src, int cols, int ldsrc, float 
 
 }  // namespace
 
+int aco::colony_check_signs(aco_colony *c, bool errors) {
+  ColonyState h;
+  if (int s = wait_state(c, &h)) return s;
+  if (errors)
+    if (int s = error_of(c, h)) return s;
+  return take_signs(c, h);
+}
+
 extern "C" {
 
 void aco_debug_fail_allocation(int32_t after) { g_fail_alloc.store(after < 0 ? -1 : after); }
@@ -488,7 +519,12 @@ int aco_colony_create(const aco_params *params, const int32_t *dist, int32_t n,
     e = cudaMemcpy2DAsync(c->dist, (size_t)c->ld * 4, dist, (size_t)n * 4, (size_t)n * 4, n, kind,
                           c->stream);
   if (e == cudaSuccess) e = launch_fill_padding_int(c->dist, n, c->ld, ACO_MAX_DISTANCE, c->stream);
+  int32_t negative = 0;
+  int32_t *word = &c->st->signed_weights;  // 0 until the colony is initialised
+  if (e == cudaSuccess) e = launch_negative_distance(c->dist, n, c->ld, word, c->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&negative, word, 4, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  c->neg_dist = negative != 0;
   if (e != cudaSuccess) {
     cudaGetLastError();
     aco_colony_destroy(c);
@@ -539,6 +575,7 @@ int init_begin(aco_colony *c, int32_t *dmax) {
   state_changed(c);
   drop_graph(c);
   c->initialized = false;
+  c->is_signed = c->neg_dist;
   const int n = c->n;
   // RankBasedAntSystem::computeParameters (src/RankBasedAntSystem.cu:31-36)
   if (c->p.variant == ACO_RANK_BASED && c->p.rank_w > n) c->p.rank_w = n;
@@ -667,7 +704,7 @@ int aco_colony_initialize(aco_colony *c) {
   NvtxRange range("aco_colony_initialize");
   if (!c) return ACO_ERR_INVALID_ARGUMENT;
   if (int s = initialize_enqueue(c)) return s;
-  if (int s = device_error(c)) return s;
+  if (int s = colony_check_signs(c, true)) return s;
   c->initialized = true;
   return ACO_OK;
 }
@@ -875,7 +912,7 @@ int aco_colony_write_pheromone(aco_colony *c, const float *in) {
                                 c->n, cudaMemcpyHostToDevice, c->stream),
            "write pheromone");
   ACO_CUDA(c, launch_pheromone_rows(make_dev(c), false, false, false, c->stream), "choice rows");
-  return device_error(c);
+  return colony_check_signs(c, true);
 }
 
 int aco_colony_read_heuristic(aco_colony *c, float *out) {
@@ -1030,7 +1067,9 @@ struct aco_batch {
   int apb = 8, row_threads = 128, grid = 0;  // rows: 4.4 ms an iteration of 512 instances, 4.75 at 256
   size_t region_bytes = 0;  // shared region of the construction launch
   int staged_count = 0;     // instances built from a staged table
-  bool rows = false;        // construction by the long-row batch kernel (every k > 32)
+  bool rows_fit = false;    // the long-row batch kernel takes every instance (k > 32)
+  bool rows = false;        // ... and is used (no instance with negative weights)
+  std::vector<char> is_signed;  // the instances' flags that the descriptors and items are for
   int min_k = 1 << 30;
   bool initialized = false;
   cudaGraph_t graph = nullptr;
@@ -1086,7 +1125,7 @@ size_t batch_plan_region(const aco_batch *b, int apb, std::vector<char> *staged,
   for (size_t i = 0; i < b->cols.size(); i++) {
     const aco_colony *c = b->cols[i];
     if (b->p.construct_mode == ACO_CONSTRUCT_GLOBAL || c->K > 32 || !c->nn16 || c->n > 2048 ||
-        c->ldk != b->sp)
+        c->ldk != b->sp || c->is_signed)
       continue;
     const size_t t = batch_staged_table_bytes(c->n, c->ld, b->sp, aging);
     if (t > avail) continue;
@@ -1096,6 +1135,23 @@ size_t batch_plan_region(const aco_batch *b, int apb, std::vector<char> *staged,
   }
   if (count) *count = cnt;
   return batch_region_bytes(b->max_n, b->max_k, apb, max_table);
+}
+
+// The instances' descriptors; one whose weights may be negative goes without
+// int16 ids, which sends it to the general kernel.
+int batch_upload_descs(aco_batch *b) {
+  std::vector<ColonyDev> descs;
+  b->is_signed.clear();
+  for (const aco_colony *c : b->cols) {
+    descs.push_back(make_dev(c));
+    if (c->is_signed) descs.back().nn16 = nullptr;
+    b->is_signed.push_back(c->is_signed);
+  }
+  ACO_BCUDA(b, upload_sync(b, b->d_descs, descs.data(), descs.size() * sizeof(ColonyDev)),
+            "upload descs");
+  b->rows = b->rows_fit &&
+            std::find(b->is_signed.begin(), b->is_signed.end(), 1) == b->is_signed.end();
+  return ACO_OK;
 }
 
 // Work items (instance, first ant, ants, staged), largest instances first.
@@ -1164,6 +1220,17 @@ int batch_build_items(aco_batch *b) {
   b->num_items = (int)items.size();
   batch_drop_graph(b);
   return ACO_OK;
+}
+
+// Plans again when an instance's weights became negative, or no longer are,
+// since the plan was made (a caller's pheromone or prior).
+int batch_take_signs(aco_batch *b) {
+  bool same = true;
+  for (size_t i = 0; i < b->cols.size(); i++)
+    same = same && (b->is_signed[i] != 0) == b->cols[i]->is_signed;
+  if (same) return ACO_OK;
+  if (int s = batch_upload_descs(b)) return s;
+  return batch_build_items(b);
 }
 
 int batch_enqueue(aco_batch *b, bool construct, bool epilogue, bool rows, bool update) {
@@ -1288,9 +1355,10 @@ int aco_batch_create(const aco_params *params, int32_t count, const int32_t *siz
   if (b->sp == 0) b->sp = 32;
   // Candidate rows longer than 32 in every instance (full rows included):
   // the long-row batch kernel, when every instance has int16 ids.
-  b->rows = b->min_k > 32 && params->construct_mode != ACO_CONSTRUCT_GLOBAL;
+  b->rows_fit = b->min_k > 32 && params->construct_mode != ACO_CONSTRUCT_GLOBAL;
   for (aco_colony *c : b->cols)
-    if (!c->nn16) b->rows = false;
+    if (!c->nn16) b->rows_fit = false;
+  b->rows = b->rows_fit;
   // Ants per CTA until tuned: the ants spread over the SMs, at most what the
   // kernel's registers allow (20 warps, one CTA an SM; the long-row kernel
   // keeps four CTAs of 8 warps an SM).  512 instances of 50 to 2000 cities:
@@ -1308,7 +1376,6 @@ int aco_batch_initialize(aco_batch *b) {
   if (!b) return ACO_ERR_INVALID_ARGUMENT;
   b->initialized = false;
   batch_drop_graph(b);
-  std::vector<ColonyDev> descs;
   std::vector<int2> rowmap;
   // The instances' setup kernels are small (the greedy tour is one CTA):
   // they run on a pool of streams, ordered after the batch stream, so that
@@ -1376,18 +1443,16 @@ int aco_batch_initialize(aco_batch *b) {
   if (s) return s;
   for (size_t i = 0; i < b->cols.size(); i++) {
     aco_colony *c = b->cols[i];
-    if (int e = device_error(c)) return bfail(b, e, c->err);
+    if (int e = colony_check_signs(c, true)) return bfail(b, e, c->err);
     c->initialized = true;
-    descs.push_back(make_dev(c));
     for (int j = 0; j < c->n; j++) rowmap.push_back(make_int2((int)i, j));
   }
   if (!b->d_descs) {
-    ACO_BCUDA(b, cudaMalloc(&b->d_descs, descs.size() * sizeof(ColonyDev)), "alloc descs");
+    ACO_BCUDA(b, cudaMalloc(&b->d_descs, b->cols.size() * sizeof(ColonyDev)), "alloc descs");
     ACO_BCUDA(b, cudaMalloc(&b->d_rowmap, rowmap.size() * sizeof(int2)), "alloc rowmap");
     ACO_BCUDA(b, cudaMalloc(&b->d_queue, sizeof(int)), "alloc queue");
   }
-  ACO_BCUDA(b, upload_sync(b, b->d_descs, descs.data(), descs.size() * sizeof(ColonyDev)),
-            "upload descs");
+  if (int s = batch_upload_descs(b)) return s;
   ACO_BCUDA(b, upload_sync(b, b->d_rowmap, rowmap.data(), rowmap.size() * sizeof(int2)),
             "upload rowmap");
   ACO_BCUDA(b, configure_pheromone_rows(b->max_ld), "configure rows");
@@ -1400,6 +1465,7 @@ int aco_batch_run(aco_batch *b, int32_t iterations) {
   NvtxRange range("aco_batch_run");
   if (!b || iterations < 0) return ACO_ERR_INVALID_ARGUMENT;
   if (!b->initialized) return bfail(b, ACO_ERR_NOT_INITIALIZED, "batch not initialized");
+  if (int s = batch_take_signs(b)) return s;
   for (aco_colony *c : b->cols) state_changed(c);  // the replays rewrite every state block
   if (!b->graph_exec) {
     const int64_t before = b->launches;
@@ -1527,6 +1593,7 @@ int aco_colony_autotune(aco_colony *c, aco_tuning *out) {
 int aco_batch_autotune(aco_batch *b, aco_tuning *out) {
   if (!b) return ACO_ERR_INVALID_ARGUMENT;
   if (!b->initialized) return bfail(b, ACO_ERR_NOT_INITIALIZED, "batch not initialized");
+  if (int s = batch_take_signs(b)) return s;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);

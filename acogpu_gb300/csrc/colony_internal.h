@@ -41,6 +41,8 @@ struct aco_colony {
   int cluster = 0;          // construction by the cluster kernel: CTAs per cluster
   bool rows = false;        // construction by the long-row kernel (k > 32)
   bool rows_staged = false; // ... with the rows in shared memory
+  bool neg_dist = false;    // a distance is negative: deposits may be
+  bool is_signed = false;   // weights may be negative: the general kernel only
   int32_t *nn2 = nullptr;   // fallback second tier (see ColonyDev)
   float *t2v = nullptr;
   float *mout = nullptr;
@@ -96,4 +98,11 @@ namespace aco {
 ColonyDev colony_dev(const aco_colony *c);
 // Records `msg` as the colony's last error and returns `status`.
 int colony_fail(aco_colony *c, int status, const std::string &msg);
+// After a row pass over weights that a caller brought (initialise, written
+// pheromone, a checkpoint, a prior): reads whether any is negative and, if the
+// answer changed, chooses the construction kernel again.  The fast kernels
+// settle picks by bounds on sums of weights that are not negative; the general
+// kernel adds entry by entry and takes any.  errors: also reports the device's
+// error words.
+int colony_check_signs(aco_colony *c, bool errors);
 }  // namespace aco

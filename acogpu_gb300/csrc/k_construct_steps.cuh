@@ -255,13 +255,24 @@ __device__ void construct_ant(const ColonyDev &c, int k, uint32_t iter, uint32_t
       if (!(S <= 0.0f)) {
         const float rnd = __fmul_rn(u, S);
         int found = -1;
-        for (int base = 0; base < nchunks; base += 32) {
+        for (int base = 0; base < nchunks && !c.is_signed; base += 32) {
           const int q = base + lane;
           const unsigned m = __ballot_sync(kFull, q < nchunks && !(cend[q] <= rnd));
           if (m) {
             found = base + __ffs(m) - 1;
             break;
           }
+        }
+        // Sums of negative weights too may pass rnd inside a chunk and end below
+        // it: every chunk is walked again, up to the first that has the crossing.
+        for (int ch = 0; ch < nchunks && c.is_signed && next < 0; ch++) {
+          int id;
+          float w;
+          candidate<false>(c, cur, ch * 32 + lane, tabu, sids, scw, a, id, w);
+          float p;
+          fold_nonzero(ch > 0 ? cend[ch - 1] : 0.0f, w, lane, wbuf, p);
+          const unsigned hit = __ballot_sync(kFull, w != 0.0f && !(p <= rnd));
+          if (hit) next = __shfl_sync(kFull, id, __ffs(hit) - 1);
         }
         if (found >= 0) {
           const float s0 = found > 0 ? cend[found - 1] : 0.0f;

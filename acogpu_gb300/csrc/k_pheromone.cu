@@ -21,7 +21,9 @@
 // the choice values of the tier's cities and the largest choice value of the
 // row outside the row itself, its candidates and its tier (marked in a
 // shared bitmap before the row lands; NaNs ignored, as the fallback never
-// picks one).
+// picks one).  The form that only writes choice values, which every pheromone
+// or heuristic that a caller brings passes through, records negative ones in
+// the colony's state.
 //
 // Atomic mode: a float4 evaporation pass, then one red.global.add.f32 per
 // directed edge, then the same row pass without evaporation or deposit.
@@ -188,10 +190,16 @@ __device__ __forceinline__ void pheromone_row_body(const ColonyDev &c, const int
   float *trow = c.tau + (size_t)j * ld;
   float *crow = c.choice + (size_t)j * ld;
   float mx = -1.0f;  // tier: largest choice value outside the marked cities
+  constexpr bool kSigns = !EVAP && !DEPOSIT;
+  unsigned signs = 0u;
   for (int h4 = tid; h4 < ld / 4; h4 += nthreads) {
     const float4 t = reinterpret_cast<const float4 *>(row)[h4];
     const float4 e = reinterpret_cast<const float4 *>(erow)[h4];
     if (WRITE_TAU) reinterpret_cast<float4 *>(trow)[h4] = t;
+    if (kSigns)
+      signs |= __float_as_uint(t.x) | __float_as_uint(t.y) | __float_as_uint(t.z) |
+               __float_as_uint(t.w) | __float_as_uint(e.x) | __float_as_uint(e.y) |
+               __float_as_uint(e.z) | __float_as_uint(e.w);
     float4 cv;
     cv.x = choice_of(t.x, e.x, c.use_alpha, c.alpha);
     cv.y = choice_of(t.y, e.y, c.use_alpha, c.alpha);
@@ -231,11 +239,14 @@ __device__ __forceinline__ void pheromone_row_body(const ColonyDev &c, const int
       tv = row[id];
       // eta_nn is eta gathered in candidate order (times the learned prior,
       // when one is installed), so without a prior this is tau * eta.
-      cv = choice_of(tv, c.eta_nn[koff + r], c.use_alpha, c.alpha);
+      const float ev = c.eta_nn[koff + r];
+      if (kSigns) signs |= __float_as_uint(ev);
+      cv = choice_of(tv, ev, c.use_alpha, c.alpha);
     }
     c.choice_nn[koff + r] = cv;
     if (c.aging) c.tau_nn[koff + r] = tv;
   }
+  if (kSigns && (signs >> 31)) atomicOr(&c.st->signed_weights, 1);
   if (c.aging && tid == 0) {
     float s = 0.0f;
     for (int h = 0; h < n; h++) s = __fadd_rn(s, row[h]);

@@ -597,6 +597,9 @@ int aco_prior_apply(aco_prior *p, aco_colony *c, float floor_) {
   if (!s && cudaStreamSynchronize(p->stream) != cudaSuccess) s = ACO_ERR_CUDA;
   if (s) return pfail(p, s, "apply failed");
   if (int g = gemm_status(p)) return g;
+  // eta (floor + p) can only be negative below a floor of 0.
+  if (!(floor_ >= 0.0f))
+    if (int e = colony_check_signs(c, false)) return pfail(p, e, "apply failed");
   // The colony's candidate table changed: a captured iteration graph stays
   // valid (same buffers), the staged copy is reloaded at every launch.
   return ACO_OK;
