@@ -30,18 +30,21 @@ __device__ __forceinline__ bool key_less(const MinKey &a, const MinKey &b) {
   return a.v < b.v || (a.v == b.v && a.k < b.k);
 }
 
-// Warp-wide minimum of (v, k), v >= 0, ties to the lower k; k < 0 means
+// Warp-wide minimum of (v, k), ties to the lower k; k < 0 means
 // "none": three 32-bit warp minima (a shuffle tree over the 64-bit pairs took
 // ten shuffles and five compares in a chain).
 __device__ __forceinline__ MinKey warp_min(MinKey x) {
   const bool some = x.k >= 0;
-  const unsigned h = some ? (unsigned)((uint64_t)x.v >> 32) : ~0u, l = (unsigned)x.v;
+  // The sign bit flipped, so that the halves order like signed lengths (tours
+  // over negative distances; no length reaches the ~0u of none).
+  const uint64_t v = (uint64_t)x.v ^ (1ull << 63);
+  const unsigned h = some ? (unsigned)(v >> 32) : ~0u, l = (unsigned)v;
   const unsigned mh = __reduce_min_sync(kFull, h);
   bool in = some && h == mh;
   const unsigned ml = __reduce_min_sync(kFull, in ? l : ~0u);
   in = in && l == ml;
   const unsigned mk = __reduce_min_sync(kFull, in ? (unsigned)x.k : ~0u);
-  return MinKey{(int64_t)(((uint64_t)mh << 32) | ml), mk == ~0u ? -1 : (int)mk};
+  return MinKey{(int64_t)((((uint64_t)mh << 32) | ml) ^ (1ull << 63)), mk == ~0u ? -1 : (int)mk};
 }
 
 // Block-wide minimum, in every thread.  `scratch` holds two sets of 32 words,

@@ -80,6 +80,24 @@ def test_prior_with_a_negative_floor(n, k, mode):
     pr.close()
 
 
+@pytest.mark.parametrize("n,k,mode", SHAPES)
+def test_negative_distances(n, k, mode):
+    """Tours of negative length: the best is the lowest, and its deposits make
+    pheromone negative between two iterations of one run."""
+    rng = np.random.default_rng(7 * n)
+    d = np.triu(3 * rng.integers(-20, 7, (n, n)), 1)
+    d[d == 0] = 3
+    d = np.triu(d, 1) + np.triu(d, 1).T
+    np.fill_diagonal(d, 0x7FFFFFFF)
+    g, q = pair(n, k, mode, d=d.astype(np.int32), nn_order=_abi.ACO_NN_REFERENCE_QSORT)
+    g.run(3)
+    g.synchronize()
+    for _ in range(3):
+        q.iterate()
+    assert q.glob_best() < 0
+    follow(g, q, 1, 0, f"n={n} k={k} mode={mode}")
+
+
 @pytest.mark.parametrize("sizes,k", [((60, 300, 1100), 0), ((50, 400, 1500), 20)])
 def test_batch_with_one_signed_instance(sizes, k):
     insts = [instance(n, 40 + n)[:2] for n in sizes]
