@@ -1111,14 +1111,25 @@ cudaError_t upload_sync(aco_batch *b, void *dst, const void *src, size_t bytes) 
   return e == cudaSuccess ? cudaStreamSynchronize(b->stream) : e;
 }
 
+// The region's bytes that fit beside the kernel's static shared memory
+// (descriptor, item, flags) plus slack.
+size_t batch_region_limit(int max_smem_optin) {
+  return (size_t)max_smem_optin - batch_construct_smem_bytes(0) - sizeof(ColonyDev) - 256;
+}
+
+// The most ants per CTA, up to `ants`, whose tabu lists fit (one at least).
+int batch_fit_ants(int max_n, int max_k, int ants, int max_smem_optin) {
+  while (ants > 1 && batch_region_bytes(max_n, max_k, ants, 0) > batch_region_limit(max_smem_optin))
+    ants--;
+  return ants;
+}
+
 // Shared memory of the construction launch with `apb` warps per CTA: the
 // largest staged table that fits next to the per-warp buffers, and which
 // instances are staged.
 size_t batch_plan_region(const aco_batch *b, int apb, std::vector<char> *staged, int *count) {
   const bool aging = b->p.aging != 0;
-  // static shared memory of the kernel (descriptor, item, flags) plus slack
-  const size_t fixed = sizeof(ColonyDev) + 256;
-  const size_t avail = (size_t)b->max_smem_optin - batch_construct_smem_bytes(0) - fixed;
+  const size_t avail = batch_region_limit(b->max_smem_optin);
   size_t max_table = 0;
   int cnt = 0;
   if (staged) staged->assign(b->cols.size(), 0);
@@ -1362,13 +1373,21 @@ int aco_batch_create(const aco_params *params, int32_t count, const int32_t *siz
   // Ants per CTA until tuned: the ants spread over the SMs, at most what the
   // kernel's registers allow (20 warps, one CTA an SM; the long-row kernel
   // keeps four CTAs of 8 warps an SM).  512 instances of 50 to 2000 cities:
-  // construction 55.5 ms at the former 8 ants a CTA, 30 at 20.
+  // construction 55.5 ms at the former 8 ants a CTA, 30 at 20.  From 45 000
+  // cities on (full rows; 90 000 with short lists) 20 ants' lists no longer fit.
   int64_t ants = 0;
   for (aco_colony *c : b->cols) ants += c->m;
-  b->apb = (int)std::min<int64_t>(b->rows ? 8 : kBatchMaxWarps,
+  const int most =
+      b->rows ? 8 : batch_fit_ants(b->max_n, b->max_k, kBatchMaxWarps, b->max_smem_optin);
+  b->apb = (int)std::min<int64_t>(most,
                                   std::max<int64_t>(1, (ants + b->num_sms - 1) / b->num_sms));
   *out = b;
   return ACO_OK;
+}
+
+int aco_selftest_batch_ants(int32_t max_n, int32_t max_k, int32_t ants, int32_t max_smem) {
+  if (max_n < 1 || max_k < 1 || ants < 1 || max_smem < 8192) return ACO_ERR_INVALID_ARGUMENT;
+  return batch_fit_ants(max_n, max_k, ants, max_smem);
 }
 
 int aco_batch_initialize(aco_batch *b) {

@@ -531,6 +531,10 @@ ACO_API void aco_tsplib_destroy(aco_tsplib *t);
  * once every request has passed) reports ACO_ERR_OUT_OF_MEMORY without
  * allocating; a negative value switches the injection off.  Process-wide. */
 ACO_API int aco_selftest_bounded_wait(uint32_t polls);
+/* The most ants per CTA, up to `ants`, that the batch kernel's shared memory
+ * holds for instances of max_n cities and max_k candidates on a device that
+ * allows max_smem bytes a CTA. */
+ACO_API int aco_selftest_batch_ants(int32_t max_n, int32_t max_k, int32_t ants, int32_t max_smem);
 ACO_API void aco_debug_fail_allocation(int32_t after);
 
 #ifdef __cplusplus

@@ -122,3 +122,25 @@ def test_tuning_layout_matches_c():
     """aco_tuning: five int/float fields, the construction mode, two reserved."""
     assert ctypes.sizeof(_abi.AcoTuning) == 32
     assert _abi.AcoTuning.construct_mode.offset == 20
+
+
+def test_batch_ants_per_cta_fit_in_shared_memory():
+    """The default ants per CTA of a batch: their tabu lists (one word per 32
+    cities, 32 words, and one per 32 candidates of lists beyond 32) fit beside
+    the kernel's other shared memory, and no fewer ants are taken than fit."""
+    fit, smem = aco.lib().aco_selftest_batch_ants, 232448
+
+    def region(n, k, ants):
+        words = (n + 31) // 32 + 32 + ((k + 31) // 32 if k > 32 else 0)
+        return (ants * words * 4 + 127) // 128 * 128
+
+    for n in (50, 8193, 16384, 30_000, 44_000, 45_500, 46_500, 60_000, 91_000, 120_000, 300_000):
+        for k in (20, n):
+            for ants in (1, 8, 20):
+                got = fit(n, k, ants, smem)
+                assert 1 <= got <= ants
+                assert region(n, k, got) <= smem - 512 or got == 1
+                assert got == ants or region(n, k, got + 1) > smem - 1024, (n, k, ants, got)
+    assert fit(46_500, 46_500, 20, smem) < 20 <= fit(45_000, 20, 20, smem)
+    assert fit(46_500, 46_500, 8, smem) == 8
+    assert fit(0, 1, 1, smem) == _abi.ACO_ERR_INVALID_ARGUMENT
