@@ -14,7 +14,9 @@
 
 #include <algorithm>
 #include <atomic>
+#include <functional>
 #include <new>
+#include <queue>
 #include <string>
 #include <vector>
 
@@ -1165,6 +1167,59 @@ int batch_upload_descs(aco_batch *b) {
   return ACO_OK;
 }
 
+// The ants per CTA until tuned, of the kernels that give a CTA up to 20 ants of
+// one instance at a time (fewer where their lists do not fit: from 45 000 cities
+// on, full rows, 90 000 with short lists).  512 instances of 50 to 2000 cities:
+// construction 55.5 ms at 8 ants a CTA, 30 at 20.  Where there are only a few
+// items for each SM the last ones decide: 64 instances of 30 cities 13.4 us at 8
+// or 16, 22.3 at 12 (192 items for 152 SMs); 48 of 200 to 2000 cities, 64 ants
+// each, 734 us at 20, 612 at 12.  So the items are laid out as the queue will
+// hand them out, largest first to the CTA that is free first, a step counted as
+// 34 units and one more for each warp of an SM (a step takes 0.26 us with 7
+// warps, 0.35 with 20), and the shape that ends first is taken.  The long-row
+// kernel (four CTAs of 8 warps an SM) and the general one for lists beyond 32
+// spread the ants over the SMs: the general one has room for more CTAs, and more
+// of them cost as much as a shorter last round gains (16 instances of 500
+// cities and one of 20: 11.8 ms at 8 and 20, 12.1 to 12.7 between).
+int batch_default_ants(const aco_batch *b) {
+  const int most =
+      b->rows ? 8 : batch_fit_ants(b->max_n, b->max_k, kBatchMaxWarps, b->max_smem_optin);
+  int64_t ants = 0, items = 0;
+  for (const aco_colony *c : b->cols) {
+    ants += c->m;
+    items += (c->m + most - 1) / most;
+  }
+  if (b->rows || b->max_k > 32)
+    return (int)std::min<int64_t>(most,
+                                  std::max<int64_t>(1, (ants + b->num_sms - 1) / b->num_sms));
+  if (most <= 8 || items > 8 * (int64_t)b->num_sms) return most;
+  std::vector<std::pair<int, int>> by_size;  // cities, ants
+  for (const aco_colony *c : b->cols) by_size.emplace_back(c->n, c->m);
+  std::sort(by_size.rbegin(), by_size.rend());
+  int best = most;
+  int64_t best_end = INT64_MAX;
+  for (int per = 8; per <= most; per += 2) {
+    const size_t smem = batch_construct_smem_bytes(batch_plan_region(b, per, nullptr, nullptr));
+    const int blocks =
+        batch_construct_blocks_per_sm(per, smem, false, b->sp, b->p.aging != 0);
+    std::priority_queue<int64_t, std::vector<int64_t>, std::greater<int64_t>> free_at;
+    for (int i = 0; i < b->num_sms * blocks; i++) free_at.push(0);
+    int64_t end = 0;
+    for (const auto &s : by_size)
+      for (int q = 0; q < (s.second + per - 1) / per; q++) {
+        const int64_t t = free_at.top() + (int64_t)s.first * (34 + per * blocks);
+        free_at.pop();
+        free_at.push(t);
+        end = std::max(end, t);
+      }
+    if (end < best_end) {
+      best_end = end;
+      best = per;
+    }
+  }
+  return best;
+}
+
 // Work items (instance, first ant, ants, staged), largest instances first.
 int batch_build_items(aco_batch *b) {
   std::vector<int> order(b->cols.size());
@@ -1370,17 +1425,12 @@ int aco_batch_create(const aco_params *params, int32_t count, const int32_t *siz
   for (aco_colony *c : b->cols)
     if (!c->nn16) b->rows_fit = false;
   b->rows = b->rows_fit;
-  // Ants per CTA until tuned: the ants spread over the SMs, at most what the
-  // kernel's registers allow (20 warps, one CTA an SM; the long-row kernel
-  // keeps four CTAs of 8 warps an SM).  512 instances of 50 to 2000 cities:
-  // construction 55.5 ms at the former 8 ants a CTA, 30 at 20.  From 45 000
-  // cities on (full rows; 90 000 with short lists) 20 ants' lists no longer fit.
-  int64_t ants = 0;
-  for (aco_colony *c : b->cols) ants += c->m;
-  const int most =
-      b->rows ? 8 : batch_fit_ants(b->max_n, b->max_k, kBatchMaxWarps, b->max_smem_optin);
-  b->apb = (int)std::min<int64_t>(most,
-                                  std::max<int64_t>(1, (ants + b->num_sms - 1) / b->num_sms));
+  if (configure_batch_construct(0) != cudaSuccess) {  // for the occupancy query
+    cudaGetLastError();
+    aco_batch_destroy(b);
+    return ACO_ERR_CUDA;
+  }
+  b->apb = batch_default_ants(b);
   *out = b;
   return ACO_OK;
 }
