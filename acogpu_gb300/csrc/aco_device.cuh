@@ -92,19 +92,12 @@ struct ColonyDev {
   int use_alpha;
   int aging, min_ret, max_ret, global_perf, min_pop;
   int variant, rank_w, fallback;
+  // Who writes the successor / predecessor lists of the ordered deposit: the
+  // construction kernels, for every ant, or the epilogue (rank-based system),
+  // for the ranked ants only.
+  int epilogue_lists;
   uint64_t seed;
 };
-
-// Who writes the successor / predecessor lists of the ordered deposit: the
-// construction kernels, for every ant, where every ant deposits (the Ant
-// System) or many do; the epilogue, for the few ranked ants only, in the
-// rank-based system.  At n = m = 1000, w = 6 that takes 23 us out of the
-// construction (three million scattered line accesses) and adds 6 us to the
-// epilogue, whose one SM issues 10 000 of them.
-constexpr int kEpilogueRanks = 32;
-__device__ __forceinline__ bool ranked_by_epilogue(const ColonyDev &c) {
-  return c.variant == ACO_RANK_BASED && c.rank_w <= kEpilogueRanks;
-}
 
 __host__ __device__ inline int round_up(int x, int a) { return (x + a - 1) / a * a; }
 

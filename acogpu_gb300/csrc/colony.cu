@@ -115,6 +115,27 @@ struct Carve {
   }
 };
 
+// Whether the epilogue writes the deposit's lists.  It writes w - 1 ants' lists
+// from one SM, 1.7 ns a city; the construction kernels write all ants' from every
+// SM, 5 ps a city at n = 1000 and more where the lists outgrow the L2 cache (9 at
+// 4096, 21 at 8192).  An iteration with the lists by the construction / by the
+// epilogue, us, m = 1000: n = 1000 w = 2 273 / 271, w = 6 275 / 280, w = 32 295 /
+// 344; n = 4096 w = 6 1664 / 1664, w = 32 1685 / 1864; n = 8192 w = 6 4731 / 4626,
+// w = 16 4758 / 4797; with 32 ants at n = 4096, w = 16 1604 / 1704.  In a batch
+// every instance has an SM for its epilogue, and all wait for the longest: 8 x n
+// = m = 1000 w = 16 1069 / 1060, w = 32 1082 / 1106; 48 instances of 200 to 2000
+// cities, m = 64, w = 6 1098 / 1066, w = 32 1120 / 1180.
+// cities: the sum of m n max(1, n / 2000); longest: the largest n; rounds:
+// instances an SM.
+bool lists_by_epilogue(const aco_params &p, double cities, int longest, int rounds) {
+  return p.variant == ACO_RANK_BASED &&
+         300.0 * (p.rank_w - 1) * longest * rounds <= cities;
+}
+
+double list_cities(const aco_colony *c) {
+  return (double)c->m * c->n * std::max(1.0, c->n / 2000.0);
+}
+
 ColonyDev make_dev(const aco_colony *c) {
   ColonyDev d;
   d.n = c->n; d.m = c->m; d.K = c->K; d.ld = c->ld; d.ldk = c->ldk; d.ldm = c->ldm;
@@ -134,6 +155,7 @@ ColonyDev make_dev(const aco_colony *c) {
   d.variant = c->p.variant; d.rank_w = c->p.rank_w; d.fallback = c->p.fallback;
   d.seed = c->p.seed;
   d.is_signed = c->is_signed;
+  d.epilogue_lists = lists_by_epilogue(c->p, list_cities(c), c->n, 1);
   return d;
 }
 
@@ -1155,8 +1177,12 @@ size_t batch_plan_region(const aco_batch *b, int apb, std::vector<char> *staged,
 int batch_upload_descs(aco_batch *b) {
   std::vector<ColonyDev> descs;
   b->is_signed.clear();
+  double cities = 0.0;
+  for (const aco_colony *c : b->cols) cities += list_cities(c);
+  const int rounds = ((int)b->cols.size() + b->num_sms - 1) / b->num_sms;
   for (const aco_colony *c : b->cols) {
     descs.push_back(make_dev(c));
+    descs.back().epilogue_lists = lists_by_epilogue(c->p, cities, b->max_n, rounds);
     if (c->is_signed) descs.back().nn16 = nullptr;
     b->is_signed.push_back(c->is_signed);
   }

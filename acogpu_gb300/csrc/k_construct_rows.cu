@@ -758,7 +758,7 @@ __device__ __forceinline__ void rows_tour(const ColonyDev &c, const RowsView &v,
   __syncwarp();
   // Integer tour length (order-free) and the transposed successor and
   // predecessor lists of the row-owned deposit, one edge per lane.
-  const bool all_deposit = !ranked_by_epilogue(c);
+  const bool all_deposit = !c.epilogue_lists;
   int64_t len = 0;
 #pragma unroll 8
   for (int i = lane; i < n; i += 32) {

@@ -869,7 +869,7 @@ __device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, uint32
   // predecessor of every city for the row-owned deposit, one edge per lane;
   // unrolled so a lane's distance reads (scattered, from HBM when the L2 is
   // cold) are in flight together.
-  const bool all_deposit = !ranked_by_epilogue(c);
+  const bool all_deposit = !c.epilogue_lists;
   int64_t len = 0;
 #pragma unroll 8
   for (int i = lane; i < n; i += 32) {

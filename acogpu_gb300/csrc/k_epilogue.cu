@@ -136,7 +136,7 @@ __device__ void epilogue_body(const ColonyDev &c) {
       __syncthreads();
     }
     // The deposit's successor / predecessor lists, of the ranked ants only.
-    const int listed = ranked_by_epilogue(c) ? count * n : 0;
+    const int listed = c.epilogue_lists ? count * n : 0;
     for (int t = tid; t < listed; t += kEpiThreads) {
       const int q = t / n, i = t - q * n, k = c.dep_col[q];
       const int32_t *tour = c.tours + (size_t)k * c.ld;

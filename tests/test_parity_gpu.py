@@ -628,3 +628,48 @@ def test_distances_on_both_paths(kind):
     g = aco.Colony(coords=(x, y), params=params(num_ants=2, cand_k=8, **FAST_MODE), num_ants=2)
     assert np.array_equal(g.distances(), instances.euc2d_distances(x, y))
     g.close()
+
+
+@pytest.mark.parametrize("w,m,n,k,aging", [(2, 300, 60, 0, 0), (3, 600, 60, 16, 1), (3, 599, 60, 16, 1),
+                                           (5, 1500, 70, 20, 0), (5, 1500, 70, 0, 1),
+                                           (2, 300, 2400, 16, 0)])
+def test_ranked_lists_by_the_epilogue_match_oracle(w, m, n, k, aging):
+    """The deposit's lists of a few ranks among many ants, which the epilogue
+    writes, and next to the line from which the construction does."""
+    x, y, d = instance(n, 970 + w + m)
+    p = params(num_ants=m, variant=_abi.ACO_RANK_BASED, rank_w=w, beta=2.0, rho=0.2, cand_k=k,
+               aging=aging, seed=w, **(FAST_MODE if k else {}))
+    g = aco.Colony(d, params=p, num_ants=m)
+    g.initialize()
+    q = oracle.Port(p, d, threads=8)
+    q.initialize()
+    for it in range(4 if n < 1000 else 2):
+        g.constructSolution()
+        q.iterate()
+        assert_same_state(g, q, aging=bool(aging), ctx=f"w={w} m={m} iteration {it}")
+    g.close()
+    q.close()
+
+
+@pytest.mark.parametrize("w", [1, 5, 6])
+@pytest.mark.parametrize("k", [0, 16])
+def test_ranked_lists_of_a_batch_match_oracle(w, k):
+    """As above over a batch, where the line depends on all its instances."""
+    insts = [instances.clustered_instance(100, seed=i) for i in range(12)]
+    p = params(num_ants=100, variant=_abi.ACO_RANK_BASED, rank_w=w, beta=2.0, rho=0.2, cand_k=k,
+               seed=w, **(FAST_MODE if k else {}))
+    b = aco.Batch(insts, params=p, num_ants=100)
+    b.initialize()
+    b.run(3)
+    b.synchronize()
+    for i, (x, y) in enumerate(insts):
+        qi = _abi.AcoParams.from_buffer_copy(p)
+        with np.errstate(over="ignore"):
+            qi.seed = int(np.uint64(p.seed) + np.uint64(i) * np.uint64(0x9E3779B97F4A7C15))
+        q = oracle.Port(qi, instances.euc2d_distances(x, y), threads=8)
+        q.initialize()
+        for _ in range(3):
+            q.iterate()
+        assert_same_state(b.colony(i), q, ctx=f"w={w} instance {i}")
+        q.close()
+    b.close()
