@@ -1001,8 +1001,8 @@ __global__ void __launch_bounds__(kGreedyNnThreads) k_greedy_tau0_nn(ColonyDev c
   }
 }
 
-// The same tour whatever the candidate lists (none in int16, or another tie
-// order).  The reference's greedyDistance is a stub returning 0
+// The same tour whatever the candidate lists (none in int16, another tie
+// order, or one city a row).  The reference's greedyDistance is a stub returning 0
 // (src/Colony.cu:1053-1055) and its tau0 is the constant 1e-6
 // (src/AntSystem.cu:200-203), which this kernel also sets.  One CTA of
 // kGreedyThreads: each step reads the current row once (coalesced, n /
@@ -1070,7 +1070,12 @@ __global__ void __launch_bounds__(kGreedyThreads)
 
 cudaError_t launch_greedy_tau0(const ColonyDev &c, int tau0_mode, float tau0_value,
                                bool stable_lists, cudaStream_t s) {
-  if (tau0_mode == ACO_TAU0_DORIGO && stable_lists && c.nn16 && c.n < 32768) {
+  // One candidate a row and no tier: the list is used up at most steps, and then
+  // this kernel's 256 threads scan the row slower than that one's 1024 (n = 4000
+  // 5.23 ms by lists, 5.31 by rows; 8000 25.0 and 23.9; 16000 138 and 81).  With
+  // two candidates the lists win at all sizes (16000 74 and 81).
+  const bool lists = c.K > 1 || c.t2 > 0 || c.n <= 4096;
+  if (tau0_mode == ACO_TAU0_DORIGO && stable_lists && lists && c.nn16 && c.n < 32768) {
     const int sk = greedy_staged(c.n, c.ldk);
     const size_t smem = greedy_layout(c.n, sk).bytes;
     void (*fn)(ColonyDev, int) = sk > 0 ? k_greedy_tau0_nn<true> : k_greedy_tau0_nn<false>;

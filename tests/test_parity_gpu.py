@@ -673,3 +673,25 @@ def test_ranked_lists_of_a_batch_match_oracle(w, k):
         assert_same_state(b.colony(i), q, ctx=f"w={w} instance {i}")
         q.close()
     b.close()
+
+
+@pytest.mark.parametrize("n,k", [(3200, 32), (3201, 32), (4096, 1), (4097, 1), (4266, 32), (4267, 32),
+                                 (6400, 32), (6401, 32), (12800, 2)])
+def test_greedy_tau0_where_the_staged_part_changes(n, k):
+    """Around the sizes where fewer entries of every list are staged (all, 24,
+    16 and 8 of 32), at the largest shared-memory layout, and where lists of
+    one city give way to row scans (rank-based system: no second tier)."""
+    x, y = instances.uniform_instance(n, seed=n, box=100_000)
+    p = params(num_ants=2, variant=_abi.ACO_RANK_BASED, rank_w=6, beta=2.0, rho=0.2, cand_k=k,
+               seed=k, **FAST_MODE)
+    g = aco.Colony(coords=(x, y), params=p, num_ants=2)
+    g.initialize()
+    d = g.distances()
+    cur, length, left = 0, 0, np.arange(1, n)
+    for _ in range(n - 1):
+        i = int(np.argmin(d[cur, left]))  # `left` stays in city order: the lowest of a tie
+        length += int(d[cur, left[i]])
+        cur = int(left[i])
+        left = np.delete(left, i)
+    assert g.stats()["greedy_length"] == length + int(d[cur, 0])
+    g.close()
