@@ -191,3 +191,110 @@ def test_lattice_rows_match_the_port(side, aging):
     d = instances.euc2d_distances(x.ravel(), y.ravel())
     p = _abi.default_params(num_ants=40, aging=aging, cand_k=0, rho=0.5, beta=2.0, seed=side)
     run_vs_port(d, p, 4, f"lattice {side}")
+
+
+@pytest.mark.parametrize("n,aging", [(129, 0), (300, 1), (1100, 0)])
+def test_prior_on_rows_in_city_order_matches_the_port(n, aging):
+    """Full rows of more than 128 cities are summed in city order from the plain
+    choice matrix, but not while a prior is installed: through apply, a second
+    apply, a checkpoint into another colony, and initialising again."""
+    x, y, d = instance(n, 800 + n)
+    p = _abi.default_params(num_ants=40 if n < 1000 else 20, cand_k=0, rho=0.2, beta=2.0, seed=9,
+                            aging=aging)
+    g = aco.Colony(coords=(x, y), params=p, num_ants=p.num_ants)
+    g.initialize()
+    pr = EdgePrior(seed=5)
+    q = oracle.Port(p, d, threads=THREADS)
+    q.initialize()
+    for floor in (0.05, 0.5):
+        pr.apply(g, floor=floor)
+        q.set_candidate_heuristic(candidate_heuristic(g))
+        for it in range(2):
+            g.constructSolution()
+            q.iterate()
+            assert_same_state(g, q, aging=bool(aging), ctx=f"floor {floor} iteration {it}")
+    with tempfile.TemporaryDirectory() as tmp:
+        g.save(os.path.join(tmp, "c"))
+        h = aco.Colony(coords=(x, y), params=p, num_ants=p.num_ants)
+        h.initialize()
+        h.run(1)
+        h.load(os.path.join(tmp, "c"))
+    q.iterate()
+    for col in (g, h):
+        col.run(1)
+        col.synchronize()
+        assert_same_state(col, q, aging=bool(aging), ctx="after the checkpoint")
+    q2 = oracle.Port(p, d, threads=THREADS)
+    q2.initialize()
+    g.initialize()
+    for it in range(2):
+        g.constructSolution()
+        q2.iterate()
+        assert_same_state(g, q2, aging=bool(aging), ctx=f"plain again {it}")
+    # a checkpoint without a prior, into a colony that has one
+    with tempfile.TemporaryDirectory() as tmp:
+        g.save(os.path.join(tmp, "c"))
+        h.load(os.path.join(tmp, "c"))
+    q2.iterate()
+    h.constructSolution()
+    assert_same_state(h, q2, aging=bool(aging), ctx="plain checkpoint")
+    for col in (g, h, q, q2):
+        col.close()
+    pr.close()
+
+
+def coincident(n, seed):
+    x, y = instances.uniform_instance(n, seed=seed)
+    x, y = np.array(x, np.float32), np.array(y, np.float32)
+    for a, b in ((3, n // 3), (7, n // 3 + 1), (n - 30, n - 2), (n // 2, n - 3)):
+        x[b], y[b] = x[a], y[a]
+    return x, y
+
+
+@pytest.mark.parametrize("n,aging", [(200, 0), (700, 1), (1100, 0)])
+def test_coincident_cities_on_rows_in_city_order(n, aging):
+    """Infinite weights where a masked one becomes a NaN in the city-order sum,
+    in one mask word a lane and in more."""
+    x, y = coincident(n, 90 + n)
+    p = _abi.default_params(num_ants=40 if n < 1000 else 16, aging=aging, cand_k=0, rho=0.3,
+                            beta=2.0, seed=n)
+    run_vs_port(instances.euc2d_distances(x, y), p, 4 if n < 1000 else 3, f"coincident n={n}")
+
+
+@pytest.mark.parametrize("sizes", [(200, 300), (200, 1100)])
+def test_batch_with_a_prior_and_coincident_cities(sizes):
+    """The batch kernel's sums of full rows, one mask word a lane (largest
+    instance up to 1024 cities) and more: one instance with a prior, one with
+    infinite weights, then without the prior again."""
+    insts = [instances.uniform_instance(sizes[0], seed=4), coincident(sizes[1], 5),
+             instances.uniform_instance(150, seed=6)]
+    p = _abi.default_params(num_ants=30, cand_k=0, rho=0.2, beta=2.0, seed=77)
+    b = aco.Batch(insts, params=p, num_ants=30)
+    pr = EdgePrior(seed=5)
+
+    def ports():
+        out = []
+        for i, (x, y) in enumerate(insts):
+            qi = _abi.AcoParams.from_buffer_copy(p)
+            with np.errstate(over="ignore"):
+                qi.seed = int(np.uint64(p.seed) + np.uint64(i) * GOLDEN_STEP)
+            out.append(oracle.Port(qi, instances.euc2d_distances(x, y), threads=THREADS))
+            out[-1].initialize()
+        return out
+
+    for prior in (True, False):
+        b.initialize()
+        qs = ports()
+        if prior:
+            pr.apply(b.colony(0), floor=0.1)
+            qs[0].set_candidate_heuristic(candidate_heuristic(b.colony(0)))
+        for it in range(3):
+            b.run(1)
+            b.synchronize()
+            for i, q in enumerate(qs):
+                q.iterate()
+                assert_same_state(b.colony(i), q, ctx=f"prior={prior} instance {i} iteration {it}")
+        for q in qs:
+            q.close()
+    pr.close()
+    b.close()
