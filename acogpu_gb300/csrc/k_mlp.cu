@@ -382,9 +382,11 @@ cudaError_t launch_transpose_feats(const __nv_bfloat16 *X, int E, __nv_bfloat16 
   return cudaGetLastError();
 }
 
-// Candidate heuristic with the prior: eta_nn = eta(gathered) * (floor + p).
+// Candidate heuristic with the prior: eta_nn = eta(gathered) * (floor + p), and
+// *prior_set where that changes an entry.
 __global__ void k_apply_prior(ColonyDev c, const float *__restrict__ prob, float floor_) {
   const int64_t total = (int64_t)c.n * c.ldk;
+  bool differs = false;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = t / c.ldk;
@@ -392,8 +394,11 @@ __global__ void k_apply_prior(ColonyDev c, const float *__restrict__ prob, float
     if (r >= c.K) continue;
     const int j = c.nn[t];
     const float e = c.eta[i * c.ld + j];
-    const_cast<float *>(c.eta_nn)[t] = __fmul_rn(e, __fadd_rn(floor_, prob[i * c.K + r]));
+    const float v = __fmul_rn(e, __fadd_rn(floor_, prob[i * c.K + r]));
+    const_cast<float *>(c.eta_nn)[t] = v;
+    differs |= __float_as_uint(v) != __float_as_uint(e);
   }
+  if (differs && __ldcg(c.prior_set) == 0) *c.prior_set = 1;
 }
 
 cudaError_t launch_apply_prior(const ColonyDev &c, const float *prob, float floor_,

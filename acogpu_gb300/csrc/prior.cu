@@ -591,7 +591,6 @@ int aco_prior_apply(aco_prior *p, aco_colony *c, float floor_) {
     s = fused ? fused_pass(p, X, nullptr, E, 1.0f, prob, nullptr, nullptr)
               : forward_backward(p, X, nullptr, B, E, 1.0f, false, prob, nullptr);
   if (!s && launch_apply_prior(d, prob, floor_, p->stream) != cudaSuccess) s = ACO_ERR_CUDA;
-  if (!s && launch_prior_set(d, p->stream) != cudaSuccess) s = ACO_ERR_CUDA;
   if (!s && launch_pheromone_rows(d, false, false, false, p->stream) != cudaSuccess)
     s = ACO_ERR_CUDA;
   if (!s && cudaStreamSynchronize(p->stream) != cudaSuccess) s = ACO_ERR_CUDA;
