@@ -75,9 +75,12 @@ struct aco_colony {
 // 64 KB page: 64 MB (the pheromone at n = 4096) took 58.6 ms to read, and 2.3
 // ms with the pages populated first; 2.4 MB 2.7 and 0.11 ms.  Buffers below
 // 128 KB mostly come from a heap that is mapped already (malloc maps larger
-// ones afresh), and the call costs about 3 us.  The buffer's contents do not
-// change; where the kernel cannot populate (EINVAL, or memory that is not the
-// process's) the copy runs as before.
+// ones afresh).  On pages that are there already (a kept or pinned buffer) the
+// call walks them for nothing: 0.7 us of a 15 us read of 160 KB, 2 of 36 us for
+// 4 MB, 30 of 392 us for 64 MB.  So from 2 MB on, a buffer whose middle and last
+// pages are there counts as mapped; asking takes 1.1 us.  The buffer's contents
+// do not change; where the kernel cannot populate (EINVAL, or memory that is not
+// the process's) the copy runs as before.
 inline void prefault(void *p, size_t bytes) {
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
@@ -86,6 +89,12 @@ inline void prefault(void *p, size_t bytes) {
   if (!p || bytes < (128u << 10)) return;
   const uintptr_t a = (uintptr_t)p / page * page;
   const uintptr_t e = ((uintptr_t)p + bytes + page - 1) / page * page;
+  auto there = [](uintptr_t at) {
+    unsigned char in = 0;
+    return mincore(reinterpret_cast<void *>(at), 1, &in) == 0 && (in & 1);
+  };
+  const uintptr_t mid = ((uintptr_t)p + bytes / 2) / page * page;
+  if (bytes >= (2u << 20) && there(e - page) && there(mid)) return;
   madvise(reinterpret_cast<void *>(a), e - a, MADV_POPULATE_WRITE);
 }
 
