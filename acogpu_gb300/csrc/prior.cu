@@ -361,7 +361,6 @@ int aco_prior_create(uint64_t seed, aco_prior **out) {
 
 int aco_prior_get_weights(aco_prior *p, float *out) {
   if (!p || !out) return ACO_ERR_INVALID_ARGUMENT;
-  prefault(out, sizeof(float) * kParamCount);
   ACO_PCUDA(p, copy_sync(p, out, p->w, sizeof(float) * kParamCount, cudaMemcpyDeviceToHost),
             "read");
   return ACO_OK;
@@ -528,7 +527,6 @@ int aco_prior_loss_and_grads(aco_prior *p, const float *feats, const float *labe
   }
   float h = 0.0f;
   if (!s) {
-    prefault(grads, sizeof(float) * kParamCount);
     cudaMemcpyAsync(&h, p->loss, 4, cudaMemcpyDeviceToHost, p->stream);
     cudaMemcpyAsync(grads, p->g, sizeof(float) * kParamCount, cudaMemcpyDeviceToHost, p->stream);
     if (cudaStreamSynchronize(p->stream) != cudaSuccess) s = ACO_ERR_CUDA;
