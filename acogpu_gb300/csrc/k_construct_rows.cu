@@ -144,12 +144,15 @@ __device__ __forceinline__ float sum2(f32x2 a) {
 }
 
 // 0/1 masks of the four cities of a nibble of the open-city word, in shared
-// memory.
+// memory (empty where predicates do the masking).
+template <bool LUT>
 struct RowsLut {
   float4 m[16];
 };
+template <>
+struct RowsLut<false> {};
 
-__device__ __forceinline__ void rows_lut_init(RowsLut &lut) {
+__device__ __forceinline__ void rows_lut_init(RowsLut<true> &lut) {
   for (int i = threadIdx.x; i < 16; i += blockDim.x)
     lut.m[i] = make_float4((i & 1) ? 1.f : 0.f, (i & 2) ? 1.f : 0.f, (i & 4) ? 1.f : 0.f,
                            (i & 8) ? 1.f : 0.f);
@@ -173,7 +176,7 @@ struct RowsSum<true> {
   // Chunks j0 .. j0 + N - 1 (0 .. 7) of the round that `open` stands for.
   template <int N>
   __device__ __forceinline__ void add(const ulonglong2 (&q)[N], uint32_t open, int j0,
-                                      const RowsLut &lut) {
+                                      const RowsLut<true> &lut) {
 #pragma unroll
     for (int j = 0; j < N; j++) {
       const unsigned at = (j0 + j == 0 ? open << 4 : open >> (4 * (j0 + j) - 4)) & 0xf0u;
@@ -193,7 +196,7 @@ struct RowsSum<false> {
   float s[4] = {0.f, 0.f, 0.f, 0.f};
   template <int N>
   __device__ __forceinline__ void add(const ulonglong2 (&q)[N], uint32_t open, int j0,
-                                      const RowsLut &) {
+                                      const RowsLut<false> &) {
 #pragma unroll
     for (int j = 0; j < N; j++) {
       float x, y, z, w;
@@ -260,7 +263,8 @@ __device__ __forceinline__ RowsView rows_view(const ColonyDev &c) {
 template <bool R1, bool BLEND, bool LUT>
 __device__ __forceinline__ float rows_city_sum(const ColonyDev &c, const RowsView &v, int cur,
                                                const uint32_t *mask, uint32_t own,
-                                               const RowsLut &lut, const AntCtx &a, int lane) {
+                                               const RowsLut<LUT> &lut, const AntCtx &a,
+                                               int lane) {
   const size_t row = (size_t)cur * v.ld + lane * 4;
   if constexpr (BLEND) {  // few ants blend: one chunk at a time, predicated
     float s[4] = {0.f, 0.f, 0.f, 0.f};
@@ -614,8 +618,9 @@ __device__ __forceinline__ unsigned rows_first(const float (&p)[4], uint2 id, fl
 // for one L2 round trip, the sum and one warp minimum.
 template <bool R1, bool BLEND, bool LUT, bool STG>
 __device__ __forceinline__ int rows_pick(const ColonyDev &c, const RowsView &v, int cur,
-                                         const uint32_t *mask, uint32_t own, const RowsLut &lut, bool natural, int cnt,
-                                         float u, const AntCtx &a, int lane) {
+                                         const uint32_t *mask, uint32_t own,
+                                         const RowsLut<LUT> &lut, bool natural, int cnt, float u,
+                                         const AntCtx &a, int lane) {
   const int nch = (v.K + 127) >> 7;
   float4 w, e;
   uint2 id;
@@ -700,7 +705,7 @@ __device__ __forceinline__ int rows_pick(const ColonyDev &c, const RowsView &v, 
 // The tour of one valid ant.
 template <bool R1, bool BLEND, bool LUT, bool STG>
 __device__ __forceinline__ void rows_tour(const ColonyDev &c, const RowsView &v, int k,
-                                          uint32_t *mask, const RowsLut &lut, AntCtx a,
+                                          uint32_t *mask, const RowsLut<LUT> &lut, AntCtx a,
                                           int lane) {
   const int n = c.n;
   int32_t *trow = c.tours + (size_t)k * c.ld;
@@ -790,7 +795,7 @@ __device__ __forceinline__ void rows_tour(const ColonyDev &c, const RowsView &v,
 // (src/Colony.cu:507-510).
 template <bool R1, bool AGING, bool LUT, bool STG>
 __device__ __forceinline__ void rows_ant(const ColonyDev &c, const RowsView &v, int pos,
-                                         uint32_t *mask, const RowsLut &lut, int lane) {
+                                         uint32_t *mask, const RowsLut<LUT> &lut, int lane) {
   AntCtx a;
   a.blend = false;
   a.ratio = 0.0f;
@@ -823,7 +828,7 @@ __host__ __device__ constexpr int rows_words(bool r1) { return r1 ? 32 : kRowsMa
 template <bool R1, bool AGING>
 __global__ void __launch_bounds__(kRowsMaxAnts * 32, 1) k_construct_rows(const __grid_constant__ ColonyDev c) {
   __shared__ uint32_t masks[kRowsMaxAnts][rows_words(R1)];
-  __shared__ RowsLut lut;
+  __shared__ RowsLut<true> lut;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   rows_lut_init(lut);
   const RowsView v = rows_view(c);
@@ -840,7 +845,7 @@ __global__ void __launch_bounds__(kRowsMaxAnts * 32, 1)
     k_construct_rows_staged(const __grid_constant__ ColonyDev c) {
   extern __shared__ __align__(128) unsigned char smem_rs[];
   __shared__ uint32_t masks[kRowsMaxAnts][rows_words(true)];
-  __shared__ RowsLut lut;
+  __shared__ RowsLut<true> lut;  // for rows in city order only, which are never staged
   __shared__ int flag;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const uint32_t w_bytes = (uint32_t)c.n * c.ldk * 4u, id_bytes = (uint32_t)c.n * c.ldk * 2u;
@@ -910,18 +915,20 @@ cudaError_t launch_construct_rows(const ColonyDev &c, int grid, int ants, bool s
 // Batches: every warp takes (instance, position) items from the work queue
 // (largest instances first) until it is empty, with its own copy of the
 // instance's descriptor; no warp waits for another.
-// 64 registers: 32 warps an SM.  A pass of 5 iterations of 8 x n = 1000 took
-// 23.4 ms, 23.8 at 80 registers, 26.2 at 72 (28 warps), 24.5 at 56 and 23.6 at
-// 48 (spills).
+// 64 registers: 32 warps an SM.  They do not hold everything: the aging form,
+// with both variants of the tour, spills 264 bytes of stores and 500 of loads,
+// the other 116 and 164.  More registers and fewer warps were slower all the
+// same: a pass of 5 iterations of 8 x n = 1000 took 23.4 ms, 23.8 at 80
+// registers, 26.2 at 72 (28 warps), and 24.5 at 56 and 23.6 at 48, which spill
+// more.
 template <bool R1, bool AGING>
 __global__ void __maxnreg__(64)
     k_batch_construct_rows(const ColonyDev *__restrict__ descs, const int4 *__restrict__ items,
                            int num_items, int *queue_head) {
   __shared__ uint32_t masks[kRowsMaxAnts][rows_words(R1)];
-  __shared__ RowsLut lut;
   __shared__ ColonyDev s_desc[kRowsMaxAnts];
+  const RowsLut<false> lut;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  rows_lut_init(lut);
   int have = -1;
   for (;;) {
     int it = 0;
