@@ -49,7 +49,7 @@ cudaError_t launch_nn_ref_qsort(const int32_t *dist, int n, int ld, int32_t *scr
                                 int ldk, ColonyState *st, cudaStream_t s);
 int nn_ref_qsort_smem_rows(int n, int max_smem);
 cudaError_t launch_nn_ref_qsort_smem(const int32_t *dist, int n, int ld, int32_t *nn, int ldk,
-                                     ColonyState *st, int max_smem, cudaStream_t s);
+                                     ColonyState *st, int max_smem, int sms, cudaStream_t s);
 cudaError_t launch_gather_nn_f32(const float *src, int n, int ld, const int32_t *nn, int K,
                                  int ldk, float *dst, cudaStream_t s);
 // stable_lists: the candidate lists are in the order of (distance, city).

@@ -658,7 +658,7 @@ int init_rest(aco_colony *c) {
     }
     if (smem_sort)
       ACO_CUDA(c, launch_nn_ref_qsort_smem(c->dist, n, c->ld, full, c->K == n ? c->ldk : c->ld,
-                                           c->st, c->max_smem_optin, c->stream),
+                                           c->st, c->max_smem_optin, c->num_sms, c->stream),
                "nn quicksort");
     else
       ACO_CUDA(c, launch_nn_ref_qsort(c->dist, n, c->ld, scratch, full,

@@ -757,10 +757,10 @@ static int nn_ref_warp_rows(int n, int max_smem) {
 }
 
 cudaError_t launch_nn_ref_qsort_smem(const int32_t *dist, int n, int ld, int32_t *nn, int ldk,
-                                     ColonyState *st, int max_smem, cudaStream_t s) {
+                                     ColonyState *st, int max_smem, int sms, cudaStream_t s) {
   if (const int wr = nn_ref_warp_rows(n, max_smem)) {
     // Whole rows a CTA, and CTAs for every SM before rows share one.
-    const int rows = std::max(1, std::min(wr, n / 152));
+    const int rows = std::max(1, std::min(wr, n / std::max(1, sms)));
     const size_t smem = (size_t)rows * nn_ref_warp_row_bytes(n);
     const cudaError_t e = open_smem((const void *)k_nn_ref_qsort_warp, smem);
     if (e != cudaSuccess) return e;
