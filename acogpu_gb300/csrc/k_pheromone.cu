@@ -196,10 +196,13 @@ __device__ __forceinline__ void pheromone_row_body(const ColonyDev &c, const int
     const float4 t = reinterpret_cast<const float4 *>(row)[h4];
     const float4 e = reinterpret_cast<const float4 *>(erow)[h4];
     if (WRITE_TAU) reinterpret_cast<float4 *>(trow)[h4] = t;
-    if (kSigns)
-      signs |= __float_as_uint(t.x) | __float_as_uint(t.y) | __float_as_uint(t.z) |
-               __float_as_uint(t.w) | __float_as_uint(e.x) | __float_as_uint(e.y) |
-               __float_as_uint(e.z) | __float_as_uint(e.w);
+    if (kSigns) {  // but the row's own city, whose distance may be any sentinel
+      const int own = j - 4 * h4;
+      signs |= own == 0 ? 0u : __float_as_uint(t.x) | __float_as_uint(e.x);
+      signs |= own == 1 ? 0u : __float_as_uint(t.y) | __float_as_uint(e.y);
+      signs |= own == 2 ? 0u : __float_as_uint(t.z) | __float_as_uint(e.z);
+      signs |= own == 3 ? 0u : __float_as_uint(t.w) | __float_as_uint(e.w);
+    }
     float4 cv;
     cv.x = choice_of(t.x, e.x, c.use_alpha, c.alpha);
     cv.y = choice_of(t.y, e.y, c.use_alpha, c.alpha);
@@ -240,7 +243,7 @@ __device__ __forceinline__ void pheromone_row_body(const ColonyDev &c, const int
       // eta_nn is eta gathered in candidate order (times the learned prior,
       // when one is installed), so without a prior this is tau * eta.
       const float ev = c.eta_nn[koff + r];
-      if (kSigns) signs |= __float_as_uint(ev);
+      if (kSigns && id != j) signs |= __float_as_uint(ev);
       cv = choice_of(tv, ev, c.use_alpha, c.alpha);
     }
     c.choice_nn[koff + r] = cv;

@@ -65,18 +65,19 @@ cudaError_t launch_fill_padding_int(int32_t *mat, int n, int ld, int32_t value, 
   return cudaGetLastError();
 }
 
-__global__ void k_negative_distance(const int32_t *__restrict__ dist, int64_t total,
+// (A city's own distance may be any sentinel.)
+__global__ void k_negative_distance(const int32_t *__restrict__ dist, int64_t total, int ld,
                                     int32_t *out) {
   int32_t signs = 0;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x)
-    signs |= dist[t];
+    if (t % (ld + 1) != 0) signs |= dist[t];
   if (signs < 0) atomicOr(out, 1);
 }
 
 cudaError_t launch_negative_distance(const int32_t *dist, int n, int ld, int32_t *out,
                                      cudaStream_t s) {
-  k_negative_distance<<<608, 256, 0, s>>>(dist, (int64_t)n * ld, out);
+  k_negative_distance<<<608, 256, 0, s>>>(dist, (int64_t)n * ld, ld, out);
   return cudaGetLastError();
 }
 

@@ -127,3 +127,25 @@ def test_batch_with_one_signed_instance(sizes, k):
     for q in ports:
         q.close()
     b.close()
+
+
+@pytest.mark.parametrize("sentinel", [-1, -7])
+def test_a_negative_own_distance_keeps_the_fast_kernel(sentinel):
+    """No tour uses a city's distance to itself, so a negative sentinel there
+    changes neither the tours nor the kernel that builds them."""
+    _, _, d = instance(300, 12)
+    e = d.copy()
+    np.fill_diagonal(e, sentinel)
+    cols = []
+    for m in (d, e):
+        p = _abi.default_params(num_ants=24, cand_k=16, rho=0.2, beta=3.0, seed=4, **FAST)
+        cols.append(aco.Colony(m, params=p, num_ants=24))
+        cols[-1].initialize()
+        cols[-1].run(2)
+        cols[-1].synchronize()
+    a, b = cols
+    assert np.array_equal(b.tours(), a.tours())
+    # the autotuner times the kernels that take the colony: the general one is last
+    assert _abi.ACO_CONSTRUCT_GLOBAL not in [c.autotune()["construct_mode"] for c in cols]
+    for c in cols:
+        c.close()
