@@ -28,7 +28,8 @@
 //     2^-24), and the other way round for i - 1; sequential sums never
 //     decrease, so the crossing is unique).  The 1.02 covers the products of
 //     errors (E < 2.1e-3 at c = 8192) and the 8 the roundings of u S' and of
-//     the bounds; 1e-37 is added for thresholds in the subnormal range;
+//     the bounds; 2^-147 is added for thresholds in the subnormal range, where
+//     products round by up to 2^-150 and sums not at all;
 //  4. otherwise -- u S' within the bound of a prefix, or a sum that is not
 //     finite -- forms the reference's running sums themselves (rows_exact).
 //     u falls into such a window in 0.1 to 3 % of the steps at n = 1000 (the
@@ -43,7 +44,7 @@
 // lookup and no city ids.  Other rows (k < n, the candidate heuristic carrying
 // a prior, at most one chunk) are summed in row order.  Only the prefixes need
 // ids, and usually one chunk of 128: the weights fall off with the distance
-// (97 % of the steps at n = 1000).  hi and lo, u S' (1 +- E) +- 1e-37, are
+// (97 % of the steps at n = 1000).  hi and lo, u S' (1 +- E) +- 2^-147, are
 // compared with all prefixes; one warp minimum over (lane, city) keys finds
 // the first past lo, with no city in it if it is not past hi.
 //
@@ -353,9 +354,10 @@ __device__ __forceinline__ void rows_mask8(const ColonyDev &c, const uint32_t *m
 // running sum.  RN(w / ulp) ulp is (w + M) - M with M = 1.5 2^e, for
 // w < 2^(e-1).  The entries where that does not hold are added one at a
 // time: those that would leave the binade (the scan shows the first), large
-// ones, halfway cases; so is every non-zero entry while s is 0, outside
-// 2^-90 .. 2^100 or not finite.  Each trip ends the chunk or adds one such
-// entry, so there are at most 257; most chunks take one, which looks at the
+// ones, halfway cases; so is every non-zero entry from 2^127 on.  Below 2^-125
+// every term is a multiple of 2^-149 and adds exactly.  A sum that is not finite
+// stays so, but for a NaN among the entries.  Each trip ends the chunk or adds
+// one entry, so there are at most 257; most chunks take one, which looks at the
 // chunk's total only.
 template <bool THR>
 __device__ __forceinline__ float rows_walk(const float (&x)[8], int start, float s, float thr,
@@ -366,13 +368,20 @@ __device__ __forceinline__ float rows_walk(const float (&x)[8], int start, float
   for (int q = 0; q < 8; q++) v[q] = 8 * lane + q >= start ? x[q] : 0.0f;
 #pragma unroll 1
   for (int trip = 0; trip < 258; trip++) {
+    if (__float_as_uint(s) >= 0x7f800000u) {
+      bool nan = false;
+#pragma unroll
+      for (int q = 0; q < 8; q++) nan |= v[q] != v[q];
+      return __any_sync(kFull, nan) ? __uint_as_float(0x7fffffffu) : s;
+    }
     const uint32_t eb = __float_as_uint(s) & 0x7f800000u;
-    const bool one = !(s >= 0x1p-90f && s <= 0x1p100f);
+    const bool tiny = s < 0x1p-125f;
     // One entry at a time: every non-zero entry counts as large.
-    const float M = one ? 0.0f : __uint_as_float(eb | 0x00400000u);
-    const float half_base = one ? 0.0f : 0.5f * __uint_as_float(eb);
-    const float half_ulp = one ? -1.0f : __uint_as_float(eb - (24u << 23));
-    const float lim = __uint_as_float(eb + 0x00800000u);
+    const bool one = s >= 0x1p127f;
+    const float M = one || tiny ? 0.0f : __uint_as_float(eb | 0x00400000u);
+    const float half_base = one ? 0.0f : tiny ? 0x1p-126f : 0.5f * __uint_as_float(eb);
+    const float half_ulp = one || tiny ? -1.0f : 0x1p-23f * half_base;
+    const float lim = tiny ? 0x1p-125f : __uint_as_float(eb + 0x00800000u);
     float t[8];
     unsigned ev = 0u;
 #pragma unroll
@@ -653,8 +662,8 @@ __device__ __forceinline__ int rows_pick(const ColonyDev &c, const RowsView &v, 
   // The first entry of chunk ch past u S' (1 - E) (rows_first).
   auto first_past = [&](const float (&q)[4], const uint2 &ids, int ch) {
     const float E = (float)(terms + min(cnt, 128 * (ch + 1)) + ch) * 6.08e-8f;  // 1.02 * 2^-24
-    const float hi = __fmaf_rn(u * (1.0f + E), S, 1e-37f);
-    const float lo = __fmaf_rn(u * (1.0f - E), S, -1e-37f);
+    const float hi = __fmaf_rn(u * (1.0f + E), S, 0x1p-147f);
+    const float lo = __fmaf_rn(u * (1.0f - E), S, -0x1p-147f);
     return rows_first(q, ids, lo, hi, lane);
   };
   unsigned first = first_past(p, k.id, 0);

@@ -710,9 +710,9 @@ struct ClusterRows {
 //    the place of the three were slower (their selects: 321 us an iteration's
 //    construction at n = m = 1000 against 268), as were the weights through
 //    shared memory and packed FMA chains a lane (310);
-//  * hi, lo = u S' (1 +- E) +- 1e-37, E = 1.02 * 94 * 2^-24 covering both
-//    errors of both sums and the roundings of the bounds (the 1e-37 where
-//    they are not relative any more).  If the first prefix past lo is also
+//  * hi, lo = u S' (1 +- E) +- 2^-147, E = 1.02 * 94 * 2^-24 covering both
+//    errors of both sums and the roundings of the bounds (the 2^-147 where
+//    they are not relative any more: products below 2^-126).  If the first prefix past lo is also
 //    past hi, the reference's sums pass its threshold at that candidate: a
 //    warp minimum of (lane, city) keys finds it and hands over the city;
 //  * otherwise -- a prefix in the window (about 1e-4 of the steps), a sum that
@@ -783,7 +783,7 @@ __device__ __forceinline__ void staged_steps(const ColonyDev &c, int k, uint32_t
       if (g1) p += T0;
       if (g2) p += T1;
       if (NG > 3 && g3) p += T2;
-      const float hi = __fmaf_rn(uhi, S, 1e-37f), lo = __fmaf_rn(ulo, S, -1e-37f);
+      const float hi = __fmaf_rn(uhi, S, 0x1p-147f), lo = __fmaf_rn(ulo, S, -0x1p-147f);
       // The first lane past lo; its city, or 0xffff (as when there is no such
       // lane) if it is inside the window.
       const unsigned city = p > hi ? (unsigned)(id & 0xffff) : 0xffffu;
