@@ -9,19 +9,22 @@
 
 namespace aco {
 
-// Lets `fn` be launched with `need` bytes of dynamic shared memory beside its
-// `fixed` static ones.  The limit belongs to the kernel, for every colony and
-// host thread, so it is always set to the most that the device allows: set to
-// one colony's need, it made the launches of a larger colony fail.
-inline cudaError_t open_smem(const void *fn, size_t need, int fixed = 0) {
+// The most shared memory a CTA of the current device may have (0: no device).
+inline int device_max_smem() {
   int dev = 0, most = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess)
-    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (e != cudaSuccess) return e;
-  most -= fixed;
-  if (most < 0 || need > (size_t)most) return cudaErrorInvalidValue;
-  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+    return 0;
+  return most;
+}
+
+// Lets `fn` be launched with `need` bytes of dynamic shared memory beside its
+// `fixed` static ones, max_smem as above.  The limit belongs to the kernel, for
+// every colony and host thread, so it is always set to the most that the device
+// allows: set to one colony's need, it made the launches of a larger colony fail.
+inline cudaError_t open_smem(const void *fn, size_t need, int max_smem, int fixed = 0) {
+  if (max_smem < fixed || need > (size_t)(max_smem - fixed)) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - fixed);
 }
 
 // ---- setup (k_setup.cu) ----
@@ -64,8 +67,8 @@ cudaError_t launch_prior_set(const ColonyDev &c, cudaStream_t s);
 // ---- iteration ----
 size_t construct_smem_bytes(int n, int K, int ants_per_block);
 // Raise the dynamic shared-memory limits once, outside any stream capture.
-cudaError_t configure_construct(size_t smem);
-cudaError_t configure_pheromone_rows(int ld);
+cudaError_t configure_construct(size_t smem, int max_smem);
+cudaError_t configure_pheromone_rows(int ld, int max_smem);
 cudaError_t launch_construct(const ColonyDev &c, int ants_per_block, cudaStream_t s);
 // Candidate table staged in shared memory (k <= 32, n <= 2048); at most
 // kStagedMaxWarps warps (ants in flight) per CTA.
@@ -92,7 +95,7 @@ __host__ __device__ inline StagedLayout staged_layout(int n, int ld, int sp, boo
   return L;
 }
 size_t construct_staged_smem_bytes(int n, int ld, int sp, bool aging);
-cudaError_t configure_construct_staged(size_t smem);
+cudaError_t configure_construct_staged(size_t smem, int max_smem);
 cudaError_t launch_construct_staged(const ColonyDev &c, const int16_t *nn16, int grid, int warps,
                                     cudaStream_t s);
 // Aging colonies: the age update and the ants' roles that the staged kernel
@@ -141,7 +144,7 @@ cudaError_t launch_batch_pheromone_rows(const ColonyDev *descs, const int2 *rowm
 size_t batch_staged_table_bytes(int n, int ld, int sp, bool aging);
 size_t batch_region_bytes(int max_n, int max_k, int warps, size_t max_table);
 size_t batch_construct_smem_bytes(size_t region_bytes);
-cudaError_t configure_batch_construct(size_t smem);
+cudaError_t configure_batch_construct(size_t smem, int max_smem);
 int batch_construct_blocks_per_sm(int warps, size_t smem, bool multi, int sp, bool aging);
 // sp: the pitch of the staged items (every staged item's ldk equals it).
 cudaError_t launch_batch_construct(const ColonyDev *descs, const int4 *items, int num_items,

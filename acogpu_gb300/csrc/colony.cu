@@ -415,7 +415,7 @@ int plan_construction(aco_colony *c) {
     const size_t smem =
         construct_staged_smem_bytes(c->n, c->ld, c->ldk, c->p.aging != 0);
     if (smem <= (size_t)c->max_smem_optin) {
-      ACO_CUDA(c, configure_construct_staged(smem), "configure staged construct");
+      ACO_CUDA(c, configure_construct_staged(smem, c->max_smem_optin), "configure staged construct");
       c->staged = true;
       return ACO_OK;
     }
@@ -690,8 +690,9 @@ int init_rest(aco_colony *c) {
   ACO_CUDA(c, launch_greedy_tau0(d, c->p.tau0_mode, c->p.tau0,
                                  c->p.nn_order == ACO_NN_STABLE, c->stream), "tau0");
   ACO_CUDA(c, launch_init_colony(d, c->stream), "init");
-  ACO_CUDA(c, configure_construct(construct_smem_bytes(n, c->K, c->apb)), "configure construct");
-  ACO_CUDA(c, configure_pheromone_rows(c->ld), "configure rows");
+  ACO_CUDA(c, configure_construct(construct_smem_bytes(n, c->K, c->apb), c->max_smem_optin),
+           "configure construct");
+  ACO_CUDA(c, configure_pheromone_rows(c->ld, c->max_smem_optin), "configure rows");
   if (int s0 = plan_construction(c)) return s0;
   ACO_CUDA(c, launch_pheromone_rows(d, false, false, false, c->stream), "choice rows");
   return ACO_OK;
@@ -1267,7 +1268,7 @@ int batch_build_items(aco_batch *b) {
     b->grid = b->num_sms * batch_rows_blocks_per_sm(b->apb, b->max_n, b->p.aging != 0);
   } else {
     const size_t smem = batch_construct_smem_bytes(b->region_bytes);
-    ACO_BCUDA(b, configure_batch_construct(smem), "configure batch construct");
+    ACO_BCUDA(b, configure_batch_construct(smem, b->max_smem_optin), "configure batch construct");
     b->grid = b->num_sms * batch_construct_blocks_per_sm(b->apb, smem, b->max_k > 32, b->sp,
                                                          b->p.aging != 0);
   }
@@ -1451,7 +1452,7 @@ int aco_batch_create(const aco_params *params, int32_t count, const int32_t *siz
   for (aco_colony *c : b->cols)
     if (!c->nn16) b->rows_fit = false;
   b->rows = b->rows_fit;
-  if (configure_batch_construct(0) != cudaSuccess) {  // for the occupancy query
+  if (configure_batch_construct(0, b->max_smem_optin) != cudaSuccess) {  // for the occupancy query
     cudaGetLastError();
     aco_batch_destroy(b);
     return ACO_ERR_CUDA;
@@ -1550,7 +1551,7 @@ int aco_batch_initialize(aco_batch *b) {
   if (int s = batch_upload_descs(b)) return s;
   ACO_BCUDA(b, upload_sync(b, b->d_rowmap, rowmap.data(), rowmap.size() * sizeof(int2)),
             "upload rowmap");
-  ACO_BCUDA(b, configure_pheromone_rows(b->max_ld), "configure rows");
+  ACO_BCUDA(b, configure_pheromone_rows(b->max_ld, b->max_smem_optin), "configure rows");
   if (int s = batch_build_items(b)) return s;
   b->initialized = true;
   return ACO_OK;

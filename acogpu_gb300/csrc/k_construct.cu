@@ -313,31 +313,31 @@ size_t construct_staged_smem_bytes(int n, int ld, int sp, bool aging) {
   return staged_layout(n, ld, sp, aging).table + 16;
 }
 
-cudaError_t configure_construct(size_t smem) {
-  cudaError_t e = open_smem((const void *)k_construct<true, true>, smem);
-  if (e == cudaSuccess) e = open_smem((const void *)k_construct<true, false>, smem);
-  if (e == cudaSuccess) e = open_smem((const void *)k_construct<false, true>, smem);
-  if (e == cudaSuccess) e = open_smem((const void *)k_construct<false, false>, smem);
+cudaError_t configure_construct(size_t smem, int max_smem) {
+  cudaError_t e = open_smem((const void *)k_construct<true, true>, smem, max_smem);
+  if (e == cudaSuccess) e = open_smem((const void *)k_construct<true, false>, smem, max_smem);
+  if (e == cudaSuccess) e = open_smem((const void *)k_construct<false, true>, smem, max_smem);
+  if (e == cudaSuccess) e = open_smem((const void *)k_construct<false, false>, smem, max_smem);
   return e;
 }
 
 namespace {
 template <bool AGING, int TW, int G, bool TIER>
-cudaError_t staged_attr(size_t smem) {
-  return open_smem((const void *)k_construct_staged<AGING, TW, G, TIER>, smem, 128);
+cudaError_t staged_attr(size_t smem, int max_smem) {
+  return open_smem((const void *)k_construct_staged<AGING, TW, G, TIER>, smem, max_smem, 128);
 }
 template <int G, bool TIER>
-cudaError_t staged_attr_tier(size_t smem) {
-  cudaError_t e = staged_attr<true, 1, G, TIER>(smem);
-  if (e == cudaSuccess) e = staged_attr<false, 1, G, TIER>(smem);
-  if (e == cudaSuccess) e = staged_attr<true, 2, G, TIER>(smem);
-  if (e == cudaSuccess) e = staged_attr<false, 2, G, TIER>(smem);
+cudaError_t staged_attr_tier(size_t smem, int max_smem) {
+  cudaError_t e = staged_attr<true, 1, G, TIER>(smem, max_smem);
+  if (e == cudaSuccess) e = staged_attr<false, 1, G, TIER>(smem, max_smem);
+  if (e == cudaSuccess) e = staged_attr<true, 2, G, TIER>(smem, max_smem);
+  if (e == cudaSuccess) e = staged_attr<false, 2, G, TIER>(smem, max_smem);
   return e;
 }
 template <int G>
-cudaError_t staged_attr_all(size_t smem) {
-  cudaError_t e = staged_attr_tier<G, false>(smem);
-  if (e == cudaSuccess) e = staged_attr_tier<G, true>(smem);
+cudaError_t staged_attr_all(size_t smem, int max_smem) {
+  cudaError_t e = staged_attr_tier<G, false>(smem, max_smem);
+  if (e == cudaSuccess) e = staged_attr_tier<G, true>(smem, max_smem);
   return e;
 }
 template <int G, bool TIER>
@@ -365,11 +365,11 @@ cudaError_t staged_launch(const ColonyDev &c, const int16_t *nn16, int grid, int
 }
 }  // namespace
 
-cudaError_t configure_construct_staged(size_t smem) {
-  cudaError_t e = staged_attr_all<4>(smem);
-  if (e == cudaSuccess) e = staged_attr_all<5>(smem);
-  if (e == cudaSuccess) e = staged_attr_all<6>(smem);
-  if (e == cudaSuccess) e = staged_attr_all<8>(smem);
+cudaError_t configure_construct_staged(size_t smem, int max_smem) {
+  cudaError_t e = staged_attr_all<4>(smem, max_smem);
+  if (e == cudaSuccess) e = staged_attr_all<5>(smem, max_smem);
+  if (e == cudaSuccess) e = staged_attr_all<6>(smem, max_smem);
+  if (e == cudaSuccess) e = staged_attr_all<8>(smem, max_smem);
   return e;
 }
 

@@ -123,8 +123,8 @@ size_t batch_staged_table_bytes(int n, int ld, int sp, bool aging) {
 
 namespace {
 template <bool MULTI, bool AGING, int G>
-cudaError_t batch_attr(size_t smem) {
-  return open_smem((const void *)k_batch_construct<MULTI, AGING, G>, smem,
+cudaError_t batch_attr(size_t smem, int max_smem) {
+  return open_smem((const void *)k_batch_construct<MULTI, AGING, G>, smem, max_smem,
                    (sizeof(ColonyDev) + 8 + 127) / 128 * 128);
 }
 template <bool MULTI, bool AGING, int G>
@@ -150,17 +150,17 @@ const void *batch_fn_for(bool multi, int sp, bool aging) {
 }
 }  // namespace
 
-cudaError_t configure_batch_construct(size_t smem) {
-  cudaError_t e = batch_attr<true, true, 8>(smem);
-  if (e == cudaSuccess) e = batch_attr<true, false, 8>(smem);
-  if (e == cudaSuccess) e = batch_attr<false, true, 4>(smem);
-  if (e == cudaSuccess) e = batch_attr<false, false, 4>(smem);
-  if (e == cudaSuccess) e = batch_attr<false, true, 5>(smem);
-  if (e == cudaSuccess) e = batch_attr<false, false, 5>(smem);
-  if (e == cudaSuccess) e = batch_attr<false, true, 6>(smem);
-  if (e == cudaSuccess) e = batch_attr<false, false, 6>(smem);
-  if (e == cudaSuccess) e = batch_attr<false, true, 8>(smem);
-  if (e == cudaSuccess) e = batch_attr<false, false, 8>(smem);
+cudaError_t configure_batch_construct(size_t smem, int max_smem) {
+  cudaError_t e = batch_attr<true, true, 8>(smem, max_smem);
+  if (e == cudaSuccess) e = batch_attr<true, false, 8>(smem, max_smem);
+  if (e == cudaSuccess) e = batch_attr<false, true, 4>(smem, max_smem);
+  if (e == cudaSuccess) e = batch_attr<false, false, 4>(smem, max_smem);
+  if (e == cudaSuccess) e = batch_attr<false, true, 5>(smem, max_smem);
+  if (e == cudaSuccess) e = batch_attr<false, false, 5>(smem, max_smem);
+  if (e == cudaSuccess) e = batch_attr<false, true, 6>(smem, max_smem);
+  if (e == cudaSuccess) e = batch_attr<false, false, 6>(smem, max_smem);
+  if (e == cudaSuccess) e = batch_attr<false, true, 8>(smem, max_smem);
+  if (e == cudaSuccess) e = batch_attr<false, false, 8>(smem, max_smem);
   return e;
 }
 

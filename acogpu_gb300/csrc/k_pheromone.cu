@@ -286,20 +286,22 @@ static cudaError_t launch_rows_t(const ColonyDev &c, int threads, cudaStream_t s
 }
 
 template <bool EVAP, bool DEPOSIT, bool WRITE_TAU>
-static cudaError_t configure_t(int ld) {
+static cudaError_t configure_t(int ld, int max_smem) {
   const size_t smem = rows_smem(ld, DEPOSIT);
-  cudaError_t e = open_smem((const void *)k_pheromone_rows<EVAP, DEPOSIT, WRITE_TAU>, smem);
+  cudaError_t e = open_smem((const void *)k_pheromone_rows<EVAP, DEPOSIT, WRITE_TAU>, smem,
+                            max_smem);
   if (e == cudaSuccess)
-    e = open_smem((const void *)k_batch_pheromone_rows<EVAP, DEPOSIT, WRITE_TAU>, smem);
+    e = open_smem((const void *)k_batch_pheromone_rows<EVAP, DEPOSIT, WRITE_TAU>, smem,
+                  max_smem);
   return e;
 }
 
-cudaError_t configure_pheromone_rows(int ld) {
-  cudaError_t e = configure_t<true, true, true>(ld);
-  if (e == cudaSuccess) e = configure_t<false, true, true>(ld);
-  if (e == cudaSuccess) e = configure_t<true, false, true>(ld);
-  if (e == cudaSuccess) e = configure_t<false, false, true>(ld);
-  if (e == cudaSuccess) e = configure_t<false, false, false>(ld);
+cudaError_t configure_pheromone_rows(int ld, int max_smem) {
+  cudaError_t e = configure_t<true, true, true>(ld, max_smem);
+  if (e == cudaSuccess) e = configure_t<false, true, true>(ld, max_smem);
+  if (e == cudaSuccess) e = configure_t<true, false, true>(ld, max_smem);
+  if (e == cudaSuccess) e = configure_t<false, false, true>(ld, max_smem);
+  if (e == cudaSuccess) e = configure_t<false, false, false>(ld, max_smem);
   return e;
 }
 

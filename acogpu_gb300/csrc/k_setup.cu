@@ -421,7 +421,7 @@ static cudaError_t launch_select(const int32_t *dist, int n, int ld, int K, int 
                                  ColonyState *st, cudaStream_t s, int32_t *nn2, int t2) {
   const size_t smem = (size_t)kSelectWarps * ((size_t)((n + 127) / 128) * 512 + 32 * R * 8 + 128);
   if (smem > 48 * 1024) {
-    const cudaError_t e = open_smem((const void *)k_nn_select_stable<R>, smem);
+    const cudaError_t e = open_smem((const void *)k_nn_select_stable<R>, smem, device_max_smem());
     if (e != cudaSuccess) return e;
   }
   k_nn_select_stable<R><<<(n + kSelectWarps - 1) / kSelectWarps, kSelectWarps * 32, smem, s>>>(
@@ -448,7 +448,7 @@ cudaError_t launch_nn_sort_stable(const int32_t *dist, int n, int ld, int K, int
   const int threads = P / 2 < kSortMaxThreads ? P / 2 : kSortMaxThreads;
   const size_t smem = (size_t)P * 8 + 16;
   if (smem > 48 * 1024) {
-    const cudaError_t e = open_smem((const void *)k_nn_sort_stable, smem);
+    const cudaError_t e = open_smem((const void *)k_nn_sort_stable, smem, device_max_smem());
     if (e != cudaSuccess) return e;
   }
   k_nn_sort_stable<<<n, threads, smem, s>>>(dist, n, ld, K, ldk, nn, nn2, t2, P, st);
@@ -763,7 +763,7 @@ cudaError_t launch_nn_ref_qsort_smem(const int32_t *dist, int n, int ld, int32_t
     // Whole rows a CTA, and CTAs for every SM before rows share one.
     const int rows = std::max(1, std::min(wr, n / std::max(1, sms)));
     const size_t smem = (size_t)rows * nn_ref_warp_row_bytes(n);
-    const cudaError_t e = open_smem((const void *)k_nn_ref_qsort_warp, smem);
+    const cudaError_t e = open_smem((const void *)k_nn_ref_qsort_warp, smem, max_smem);
     if (e != cudaSuccess) return e;
     k_nn_ref_qsort_warp<<<(n + rows - 1) / rows, rows * 32, smem, s>>>(dist, n, ld, nn, ldk, st);
     return cudaGetLastError();
@@ -771,7 +771,7 @@ cudaError_t launch_nn_ref_qsort_smem(const int32_t *dist, int n, int ld, int32_t
   const int rows = nn_ref_qsort_smem_rows(n, max_smem);
   if (rows < 1) return cudaErrorInvalidValue;
   const size_t smem = (size_t)rows * n * 8;
-  const cudaError_t e = open_smem((const void *)k_nn_ref_qsort_smem, smem);
+  const cudaError_t e = open_smem((const void *)k_nn_ref_qsort_smem, smem, max_smem);
   if (e != cudaSuccess) return e;
   k_nn_ref_qsort_smem<<<(n + rows - 1) / rows, rows * 32, smem, s>>>(dist, n, ld, nn, ldk, st);
   return cudaGetLastError();
@@ -1083,7 +1083,7 @@ cudaError_t launch_greedy_tau0(const ColonyDev &c, int tau0_mode, float tau0_val
     const size_t smem = greedy_layout(c.n, sk).bytes;
     void (*fn)(ColonyDev, int) = sk > 0 ? k_greedy_tau0_nn<true> : k_greedy_tau0_nn<false>;
     if (smem > 48 * 1024) {
-      const cudaError_t e = open_smem((const void *)fn, smem, 256);
+      const cudaError_t e = open_smem((const void *)fn, smem, device_max_smem(), 256);
       if (e != cudaSuccess) return e;
     }
     fn<<<1, kGreedyNnThreads, smem, s>>>(c, sk);
