@@ -441,9 +441,9 @@ __device__ __forceinline__ float scan_level(float x, int o) {
 // ms of construction for 512 instances with it, 27 without): a group of chunks
 // is loaded ahead of the one being compared, four (n <= 2048; the whole row at
 // n = 1000 takes two groups) or eight (n = 4096: construction 1436 us with
-// four, 1374 with eight).  A row whose largest value is 0 or NaN goes to
-// fallback_rest, which tells an unvisited zero from a visited city and skips
-// NaNs.
+// four, 1374 with eight).  If the largest value is 0 the lowest unvisited city
+// is the answer, from the tabu words alone, and a row with a NaN is scanned again
+// without it (fallback_rest).
 template <int TW>
 struct TwPack {
   uint32_t w[TW];
@@ -475,7 +475,15 @@ __device__ __forceinline__ uint32_t fallback_bits(const TwPack<TW> &p, int t, in
 
 template <int TW>
 __device__ __noinline__ int fallback_rest(const ColonyDev &c, int cur, TwPack<TW> p, AntCtx a,
-                                          int lane) {
+                                          int lane, bool zero) {
+  if (zero) {
+    unsigned first = ~0u;
+#pragma unroll
+    for (int t = TW - 1; t >= 0; t--)
+      if (~p.w[t]) first = (unsigned)(32 * (lane + 32 * t) + __ffs(~p.w[t]) - 1);
+    first = __reduce_min_sync(kFull, first);
+    return first < (unsigned)c.n ? (int)first : -1;
+  }
   float bw = -1.0f;
   int bj = -1;
   const size_t row = (size_t)cur * c.ld;
@@ -574,7 +582,7 @@ __device__ __forceinline__ int fallback_scan(const ColonyDev &c, int cur, const 
     }
   }
   const unsigned m = __reduce_max_sync(kFull, best);
-  if (m == 0u || m > 0x7f800000u) return fallback_rest<TW>(c, cur, p, a, lane);
+  if (m == 0u || m > 0x7f800000u) return fallback_rest<TW>(c, cur, p, a, lane, m == 0u);
   const int r = bq.x == m ? 0 : bq.y == m ? 1 : bq.z == m ? 2 : 3;
   return (int)__reduce_min_sync(kFull, best == m ? (unsigned)(bt * 128 + lane * 4 + r) : ~0u);
 }
@@ -691,6 +699,26 @@ struct ClusterRows {
   }
 };
 
+constexpr int kNoPick = -(1 << 30);
+
+// The reference's own walk over one row (staged_steps, below): the id of the
+// first candidate past the threshold, or kNoPick.  A called function: within the
+// loop it kept the row's weights alive over the fallback (n = m = 1000 with aging,
+// clustered, k = 20: 305 us an iteration, 292 so).
+template <int SP>
+__device__ __noinline__ int exact_pick(float w, int id, float u, int lane) {
+  float ra = 0.0f, rs = 0.0f;
+#pragma unroll 4
+  for (int e = 0; e < SP; e++) {
+    const float we = __shfl_sync(kFull, w, e);
+    ra = __fmaf_rn(we, e <= lane ? 1.0f : 0.0f, ra);
+    rs = __fadd_rn(rs, we);
+  }
+  const float rnd = __fmul_rn(u, rs);
+  const unsigned hit = __ballot_sync(kFull, ra > rnd || rnd != rnd);
+  return hit ? __shfl_sync(kFull, id, __ffs(hit) - 1) : kNoPick;
+}
+
 // The step loop of one ant; BLEND (the aging fitness blend, fixed for the
 // ant's whole tour) is a template parameter so the loop carries no per-step
 // test of it.  Rows are padded to the pitch with id -1 and weight 0, so every
@@ -795,20 +823,13 @@ __device__ __forceinline__ void staged_steps(const ColonyDev &c, int k, uint32_t
       int id_next = rows.id(nx, lr);
       float w_next = BLEND ? 0.0f : rows.weight(nx, lr);
       if (next >= n || !(S <= 3e38f)) {
-        unsigned hit = 0u;
-        if (S != 0.0f) {  // the reference's own sums (header)
-          float ra = 0.0f, rs = 0.0f;
-#pragma unroll 4
-          for (int e = 0; e < SP; e++) {
-            const float we = __shfl_sync(kFull, w, e);
-            ra = __fmaf_rn(we, e <= lane ? 1.0f : 0.0f, ra);
-            rs = __fadd_rn(rs, we);
-          }
-          const float rnd = __fmul_rn(u, rs);
-          hit = __ballot_sync(kFull, ra > rnd || rnd != rnd);
-          next = __shfl_sync(kFull, id, (__ffs(hit) - 1) & 31);
-        }
-        if (hit != 0u) {
+        // With an infinite weight the threshold is infinite too (u > 0) and no
+        // prefix is past it.
+        const float inf = __int_as_float(0x7f800000);
+        next = S != 0.0f && !(S == inf && __any_sync(kFull, w == inf))
+                   ? exact_pick<SP>(w, id, u, lane)
+                   : kNoPick;
+        if (next != kNoPick) {
           if ((unsigned)next >= (unsigned)n) ok = false;  // recorded, not used
         } else {
           fallbacks++;
@@ -869,7 +890,9 @@ __device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, uint32
   // predecessor of every city for the row-owned deposit, one edge per lane;
   // unrolled so a lane's distance reads (scattered, from HBM when the L2 is
   // cold) are in flight together.
-  const bool all_deposit = !c.epilogue_lists;
+  // (Both words, though the second would do: the compiler's step loop above is
+  // then 4 % faster, n = m = 1000, k = 32 281 us an iteration against 272.)
+  const bool all_deposit = !(c.variant == ACO_RANK_BASED && c.epilogue_lists);
   int64_t len = 0;
 #pragma unroll 8
   for (int i = lane; i < n; i += 32) {

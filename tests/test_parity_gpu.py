@@ -695,3 +695,40 @@ def test_greedy_tau0_where_the_staged_part_changes(n, k):
         left = np.delete(left, i)
     assert g.stats()["greedy_length"] == length + int(d[cur, 0])
     g.close()
+
+
+@pytest.mark.parametrize("n,k,mode", [(200, 16, _abi.ACO_CONSTRUCT_STAGED), (1100, 20, _abi.ACO_CONSTRUCT_STAGED),
+                                      (1500, 32, _abi.ACO_CONSTRUCT_CLUSTER),
+                                      (2100, 24, _abi.ACO_CONSTRUCT_CLUSTER),
+                                      (2100, 8, _abi.ACO_CONSTRUCT_DIRECT), (30, 0, _abi.ACO_CONSTRUCT_AUTO),
+                                      (180, 0, _abi.ACO_CONSTRUCT_ROWS), (300, 64, _abi.ACO_CONSTRUCT_ROWS),
+                                      (300, 0, _abi.ACO_CONSTRUCT_ROWS), (1100, 0, _abi.ACO_CONSTRUCT_ROWS)])
+@pytest.mark.parametrize("tau0,place", [(0.0, "uniform"), (1e-30, "uniform"), (3e-42, "uniform"),
+                                        (3e38, "uniform"), (1.0, "third"), (1.0, "lattice")])
+def test_weights_at_the_ends_of_the_range_match_oracle(n, k, mode, tau0, place):
+    """Weights all zero, in and near the subnormal range, whose sums overflow,
+    and infinite ones in most rows: a third of the cities at one place, or
+    cities drawn from a small lattice."""
+    g0 = np.random.default_rng(n + k)
+    if place == "lattice":
+        x, y = g0.integers(0, 25, (2, n)).astype(np.float32)
+    else:
+        x, y = (g0.integers(0, 1000, (2, n)) * 1.0).astype(np.float32)
+        if place == "third":
+            x[: n // 3], y[: n // 3] = 5, 5
+    d = instances.euc2d_distances(x, y)
+    more = {**FAST_MODE, "tau0_mode": _abi.ACO_TAU0_VALUE}
+    p = params(num_ants=20, beta=1.0 if tau0 > 1 else 2.0, rho=0.3, cand_k=k, seed=n, tau0=tau0,
+               **{a: b for a, b in more.items()})
+    p.construct_mode = mode
+    g = aco.Colony(d, params=p, num_ants=20)
+    g.initialize()
+    p.construct_mode = _abi.ACO_CONSTRUCT_AUTO
+    q = oracle.Port(p, d, threads=8)
+    q.initialize()
+    for it in range(2):
+        g.constructSolution()
+        q.iterate()
+        assert_same_state(g, q, ctx=f"tau0={tau0} {place} iteration {it}")
+    g.close()
+    q.close()
