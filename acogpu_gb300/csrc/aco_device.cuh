@@ -45,7 +45,7 @@ struct ColonyState {
   int32_t globalperformance;
   int32_t dep_count;       // entries in the deposit list
   uint32_t error;
-  int32_t error_info;
+  int32_t prior_set;       // eta_nn carries a learned prior (differs from eta's entries)
   float tau0;
   int32_t signed_weights;  // a pheromone or heuristic value is negative (or was, since the reset)
   int64_t greedy_length;   // C_nn
@@ -62,7 +62,6 @@ struct ColonyDev {
   const int32_t *nn;
   const int16_t *nn16;  // n x 32 candidate ids (-1 padded) when k <= 32, else null
   const float *eta_nn;
-  int32_t *prior_set;  // non-zero: eta_nn carries a learned prior (differs from eta's entries)
   float *tau_nn;
   float *choice_nn;
   int32_t *tours;

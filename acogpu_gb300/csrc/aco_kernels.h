@@ -59,7 +59,7 @@ cudaError_t launch_gather_nn_f32(const float *src, int n, int ld, const int32_t 
 cudaError_t launch_greedy_tau0(const ColonyDev &c, int tau0_mode, float tau0_value,
                                bool stable_lists, cudaStream_t s);
 cudaError_t launch_init_colony(const ColonyDev &c, cudaStream_t s);
-// Sets *c.prior_set to whether the candidate heuristic differs from the
+// Sets the state's prior_set to whether the candidate heuristic differs from the
 // gathered plain heuristic (a learned prior is installed): after a checkpoint;
 // launch_apply_prior sets it by itself.
 cudaError_t launch_prior_set(const ColonyDev &c, cudaStream_t s);

@@ -146,7 +146,6 @@ ColonyDev make_dev(const aco_colony *c) {
   d.succT = c->succT; d.predT = c->predT; d.gbtour = c->gbtour;
   d.age = c->age; d.perf = c->perf; d.valid = c->valid; d.mean = c->mean;
   d.dep_col = c->dep_col; d.dep_delta = c->dep_delta; d.plan = c->plan; d.st = c->st;
-  d.prior_set = c->prior_set;
   d.nn2 = c->nn2; d.t2v = c->t2v; d.mout = c->mout; d.t2 = c->t2;
   d.rho = c->p.rho; d.alpha = c->p.alpha; d.use_alpha = c->p.use_alpha;
   d.aging = c->p.aging; d.min_ret = c->p.min_retirement_age;
@@ -239,7 +238,6 @@ int allocate(aco_colony *c) {
   a.add(&c->plan, m + 2);
   a.add(&c->dep_col, m + 1);
   a.add(&c->dep_delta, m + 1);
-  a.add(&c->prior_set, 1);
   a.add(&c->st, 1);
   if ((s = a.commit(c))) return s;
   ACO_CUDA(c, cudaMemsetAsync(c->tours, 0, m * ld * 4, c->stream), "memset tours");
@@ -683,7 +681,6 @@ int init_rest(aco_colony *c) {
   }
   ACO_CUDA(c, launch_gather_nn_f32(c->eta, n, c->ld, c->nn, c->K, c->ldk, c->eta_nn, c->stream),
            "eta_nn");
-  ACO_CUDA(c, cudaMemsetAsync(c->prior_set, 0, sizeof(int32_t), c->stream), "memset prior");
   if (c->nn16) ACO_CUDA(c, launch_nn_to_i16(c->nn, n, c->K, c->ldk, c->nn16, c->stream), "nn16");
 
   const ColonyDev d = make_dev(c);
@@ -1203,23 +1200,31 @@ int batch_upload_descs(aco_batch *b) {
 // each, 734 us at 20, 612 at 12.  So the items are laid out as the queue will
 // hand them out, largest first to the CTA that is free first, a step counted as
 // 34 units and one more for each warp of an SM (a step takes 0.26 us with 7
-// warps, 0.35 with 20), and the shape that ends first is taken.  The long-row
-// kernel (four CTAs of 8 warps an SM) and the general one for lists beyond 32
-// spread the ants over the SMs: the general one has room for more CTAs, and more
-// of them cost as much as a shorter last round gains (16 instances of 500
-// cities and one of 20: 11.8 ms at 8 and 20, 12.1 to 12.7 between).
+// warps, 0.35 with 20), and the shape that ends first is taken.  The general
+// kernel for lists beyond 32 has room for more CTAs an SM, and every ant adds to
+// the SM's time: the ants are spread over the SMs, at least 8 a CTA, more where
+// that leaves no SM a second item.  7 instances of 387 cities, k = 100, aging: 13.1
+// ms at 8, 17.6 at 18 (154 items for 152 SMs); 64 x n = 60, full rows: 211 us at 8,
+// 183 at 20.  The long-row kernel's warps take single ants, 8 warps a CTA.
 int batch_default_ants(const aco_batch *b) {
   const int most =
       b->rows ? 8 : batch_fit_ants(b->max_n, b->max_k, kBatchMaxWarps, b->max_smem_optin);
-  int64_t ants = 0, items = 0;
-  for (const aco_colony *c : b->cols) {
-    ants += c->m;
-    items += (c->m + most - 1) / most;
+  int64_t ants = 0;
+  for (const aco_colony *c : b->cols) ants += c->m;
+  auto items_of = [&](int per) {
+    int64_t items = 0;
+    for (const aco_colony *c : b->cols) items += (c->m + per - 1) / per;
+    return items;
+  };
+  const int spread = (int)std::min<int64_t>(
+      most, std::max<int64_t>(1, (ants + b->num_sms - 1) / b->num_sms));
+  if (b->rows) return spread;
+  if (b->max_k > 32) {
+    int per = std::max(std::min(8, most), spread);
+    while (per < most && items_of(per) > b->num_sms) per++;
+    return per;
   }
-  if (b->rows || b->max_k > 32)
-    return (int)std::min<int64_t>(most,
-                                  std::max<int64_t>(1, (ants + b->num_sms - 1) / b->num_sms));
-  if (most <= 8 || items > 8 * (int64_t)b->num_sms) return most;
+  if (most <= 8 || items_of(most) > 8 * (int64_t)b->num_sms) return most;
   std::vector<std::pair<int, int>> by_size;  // cities, ants
   for (const aco_colony *c : b->cols) by_size.emplace_back(c->n, c->m);
   std::sort(by_size.rbegin(), by_size.rend());

@@ -23,7 +23,6 @@ struct aco_colony {
   float *eta = nullptr, *tau = nullptr, *choice = nullptr;
   int32_t *nn = nullptr;
   float *eta_nn = nullptr, *tau_nn = nullptr, *choice_nn = nullptr;
-  int32_t *prior_set = nullptr;  // device word (see ColonyDev)
   int32_t *tours = nullptr;
   int64_t *newlen = nullptr, *len = nullptr;
   int32_t *succT = nullptr, *predT = nullptr, *gbtour = nullptr;

@@ -718,7 +718,7 @@ __device__ __forceinline__ void rows_tour(const ColonyDev &c, const RowsView &v,
                                           int lane) {
   const int n = c.n;
   int32_t *trow = c.tours + (size_t)k * c.ld;
-  const bool natural = rows_city_order(n, c.K) && *c.prior_set == 0;
+  const bool natural = rows_city_order(n, c.K) && c.st->prior_set == 0;
   uint32_t own = 0u;
   for (int r = 0; r < (R1 ? 1 : kRowsMaskWords / 32); r++) {
     uint32_t open = 0u;

@@ -383,7 +383,7 @@ cudaError_t launch_transpose_feats(const __nv_bfloat16 *X, int E, __nv_bfloat16 
 }
 
 // Candidate heuristic with the prior: eta_nn = eta(gathered) * (floor + p), and
-// *prior_set where that changes an entry.
+// prior_set where that changes an entry.
 __global__ void k_apply_prior(ColonyDev c, const float *__restrict__ prob, float floor_) {
   const int64_t total = (int64_t)c.n * c.ldk;
   bool differs = false;
@@ -398,7 +398,7 @@ __global__ void k_apply_prior(ColonyDev c, const float *__restrict__ prob, float
     const_cast<float *>(c.eta_nn)[t] = v;
     differs |= __float_as_uint(v) != __float_as_uint(e);
   }
-  if (differs && __ldcg(c.prior_set) == 0) *c.prior_set = 1;
+  if (differs && __ldcg(&c.st->prior_set) == 0) c.st->prior_set = 1;
 }
 
 cudaError_t launch_apply_prior(const ColonyDev &c, const float *prob, float floor_,

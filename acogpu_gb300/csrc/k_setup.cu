@@ -810,11 +810,11 @@ __global__ void k_prior_set(ColonyDev c) {
     const float plain = c.eta[j * c.ld + c.nn[j * c.ldk + r]];
     differs |= __float_as_uint(c.eta_nn[j * c.ldk + r]) != __float_as_uint(plain);
   }
-  if (__any_sync(kFull, differs) && (threadIdx.x & 31) == 0) *c.prior_set = 1;
+  if (__any_sync(kFull, differs) && (threadIdx.x & 31) == 0) c.st->prior_set = 1;
 }
 
 cudaError_t launch_prior_set(const ColonyDev &c, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(c.prior_set, 0, sizeof(int32_t), s);
+  cudaError_t e = cudaMemsetAsync(&c.st->prior_set, 0, sizeof(int32_t), s);
   if (e != cudaSuccess) return e;
   k_prior_set<<<608, 256, 0, s>>>(c);
   return cudaGetLastError();
