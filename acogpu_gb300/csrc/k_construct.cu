@@ -5,7 +5,7 @@
 
 namespace aco {
 
-template <bool MULTI, bool AGING>
+template <bool MULTI, bool AGING, bool SIGNED>
 __global__ void __launch_bounds__(512) k_construct(ColonyDev c, int nchunks) {
   extern __shared__ __align__(16) uint32_t smem_construct[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -15,8 +15,8 @@ __global__ void __launch_bounds__(512) k_construct(ColonyDev c, int nchunks) {
   uint32_t *tabu = smem_construct + (size_t)warp * (words + 32 + (MULTI ? nchunks : 0));
   float *wbuf = reinterpret_cast<float *>(tabu + words);
   float *cend = wbuf + 32;
-  construct_ant<MULTI, AGING, false>(c, k, c.st->iteration, tabu, cend, wbuf, nullptr, nullptr,
-                                     nullptr, nchunks, lane);
+  construct_ant<MULTI, AGING, false, SIGNED>(c, k, c.st->iteration, tabu, cend, wbuf, nullptr,
+                                             nullptr, nullptr, nchunks, lane);
 }
 
 // Aging colonies, before the staged construction: updateAntAges
@@ -314,10 +314,14 @@ size_t construct_staged_smem_bytes(int n, int ld, int sp, bool aging) {
 }
 
 cudaError_t configure_construct(size_t smem, int max_smem) {
-  cudaError_t e = open_smem((const void *)k_construct<true, true>, smem, max_smem);
-  if (e == cudaSuccess) e = open_smem((const void *)k_construct<true, false>, smem, max_smem);
-  if (e == cudaSuccess) e = open_smem((const void *)k_construct<false, true>, smem, max_smem);
-  if (e == cudaSuccess) e = open_smem((const void *)k_construct<false, false>, smem, max_smem);
+  if (smem <= 48 * 1024) return cudaSuccess;  // at most 80 000 cities at 4 ants a CTA
+  cudaError_t e = open_smem((const void *)k_construct<true, true, false>, smem, max_smem);
+  if (e == cudaSuccess) e = open_smem((const void *)k_construct<true, false, false>, smem, max_smem);
+  if (e == cudaSuccess) e = open_smem((const void *)k_construct<false, true, false>, smem, max_smem);
+  if (e == cudaSuccess)
+    e = open_smem((const void *)k_construct<false, false, false>, smem, max_smem);
+  if (e == cudaSuccess) e = open_smem((const void *)k_construct<true, true, true>, smem, max_smem);
+  if (e == cudaSuccess) e = open_smem((const void *)k_construct<true, false, true>, smem, max_smem);
   return e;
 }
 
@@ -378,7 +382,10 @@ static cudaError_t launch_construct_t(const ColonyDev &c, int apb, cudaStream_t 
   const int nchunks = (c.K + 31) / 32;
   const size_t smem = construct_smem_bytes(c.n, c.K, apb);
   const int grid = (c.m + apb - 1) / apb;
-  k_construct<MULTI, AGING><<<grid, apb * 32, smem, s>>>(c, nchunks);
+  if (MULTI && c.is_signed)
+    k_construct<MULTI, AGING, MULTI><<<grid, apb * 32, smem, s>>>(c, nchunks);
+  else
+    k_construct<MULTI, AGING, false><<<grid, apb * 32, smem, s>>>(c, nchunks);
   return cudaGetLastError();
 }
 

@@ -97,6 +97,10 @@ __global__ void __launch_bounds__(kBatchMaxWarps * 32) k_batch_construct(const C
         construct_ant_staged<AGING, 2, G, TableRows<4 * G>, true, false>(
             c, w.y + warp, c.st->iteration, nullptr,
             TableRows<4 * G>{c.nn16, c.choice_nn, c.mean}, lane);
+    } else if (MULTI && c.is_signed) {
+      if (warp < w.z)
+        construct_ant<MULTI, AGING, false, MULTI>(c, w.y + warp, c.st->iteration, tabu, cend, wbuf,
+                                                  nullptr, nullptr, nullptr, (c.K + 31) >> 5, lane);
     } else if (warp < w.z) {
       construct_ant<MULTI, AGING, false>(c, w.y + warp, c.st->iteration, tabu, cend, wbuf,
                                          nullptr, nullptr, nullptr, (c.K + 31) >> 5, lane);

@@ -178,7 +178,8 @@ static __device__ int fallback_city(const ColonyDev &c, int cur, const uint32_t 
   return bj;
 }
 
-template <bool MULTI, bool AGING, bool STAGED>
+// SIGNED: weights may be negative.
+template <bool MULTI, bool AGING, bool STAGED, bool SIGNED = false>
 __device__ void construct_ant(const ColonyDev &c, int k, uint32_t iter, uint32_t *tabu,
                               float *cend, float *wbuf, const int16_t *sids, const float *scw,
                               const float *smean, int nchunks, int lane) {
@@ -255,7 +256,7 @@ __device__ void construct_ant(const ColonyDev &c, int k, uint32_t iter, uint32_t
       if (!(S <= 0.0f)) {
         const float rnd = __fmul_rn(u, S);
         int found = -1;
-        for (int base = 0; base < nchunks && !c.is_signed; base += 32) {
+        for (int base = 0; base < nchunks && !SIGNED; base += 32) {
           const int q = base + lane;
           const unsigned m = __ballot_sync(kFull, q < nchunks && !(cend[q] <= rnd));
           if (m) {
@@ -265,7 +266,7 @@ __device__ void construct_ant(const ColonyDev &c, int k, uint32_t iter, uint32_t
         }
         // Sums of negative weights too may pass rnd inside a chunk and end below
         // it: every chunk is walked again, up to the first that has the crossing.
-        for (int ch = 0; ch < nchunks && c.is_signed && next < 0; ch++) {
+        for (int ch = 0; ch < nchunks && SIGNED && next < 0; ch++) {
           int id;
           float w;
           candidate<false>(c, cur, ch * 32 + lane, tabu, sids, scw, a, id, w);
