@@ -15,6 +15,8 @@ namespace aco {
 // reaches both barriers on every path (a copy that timed out only records
 // the error, and the ants run only when every rank staged its slice).  All
 // CTAs share all ants.
+constexpr int kWideClusterWarps = 8;  // the most warps of a launch of the wide form
+
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -34,8 +36,8 @@ __device__ __forceinline__ void cluster_barrier() {
           : "memory");
 }
 
-template <bool AGING, int TW, int G>
-__global__ void __launch_bounds__(kStagedMaxWarps * 32)
+template <bool AGING, int TW, int G, int W>
+__global__ void __launch_bounds__(W * 32)
     k_construct_cluster(ColonyDev c) {
   extern __shared__ __align__(128) unsigned char smem_cl[];
   constexpr int SP = 4 * G;
@@ -95,7 +97,8 @@ __global__ void __launch_bounds__(kStagedMaxWarps * 32)
     const ClusterRows<SP> rows{smem_u32(sids), smem_u32(scw), smem_u32(smean)};
     const uint32_t iter = c.st->iteration;
     for (int k = blockIdx.x * warps + warp; k < c.m; k += gridDim.x * warps)
-      construct_ant_staged<AGING, TW, G, ClusterRows<SP>>(c, k, iter, words, rows, lane);
+      construct_ant_staged<AGING, TW, G, ClusterRows<SP>, true, W == kWideClusterWarps ? 2 : 1>(
+          c, k, iter, words, rows, lane);
   }
   __syncthreads();
   cluster_barrier();  // no slice is released while another CTA may read it
@@ -108,7 +111,7 @@ size_t construct_cluster_smem_bytes(int sp, bool aging, int warps, int tw) {
 }
 
 namespace {
-template <bool AGING, int TW, int G>
+template <bool AGING, int TW, int G, int W>
 cudaError_t cluster_launch_t(const ColonyDev &c, int grid, int warps, int cs, cudaStream_t s,
                              int *max_clusters) {
   const size_t smem = construct_cluster_smem_bytes(4 * G, AGING, warps, TW);
@@ -116,7 +119,7 @@ cudaError_t cluster_launch_t(const ColonyDev &c, int grid, int warps, int cs, cu
     // the query, at planning time, opens the kernel to any warp count, so a
     // launch (possibly under stream capture) sets no attribute
     const size_t most = construct_cluster_smem_bytes(4 * G, AGING, kStagedMaxWarps, TW);
-    cudaError_t e = cudaFuncSetAttribute(k_construct_cluster<AGING, TW, G>,
+    cudaError_t e = cudaFuncSetAttribute(k_construct_cluster<AGING, TW, G, W>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e != cudaSuccess) return e;
   }
@@ -133,15 +136,43 @@ cudaError_t cluster_launch_t(const ColonyDev &c, int grid, int warps, int cs, cu
   cfg.attrs = at;
   cfg.numAttrs = 1;
   if (max_clusters)
-    return cudaOccupancyMaxActiveClusters(max_clusters, k_construct_cluster<AGING, TW, G>, &cfg);
-  return cudaLaunchKernelEx(&cfg, k_construct_cluster<AGING, TW, G>, c);
+    return cudaOccupancyMaxActiveClusters(max_clusters, k_construct_cluster<AGING, TW, G, W>, &cfg);
+  return cudaLaunchKernelEx(&cfg, k_construct_cluster<AGING, TW, G, W>, c);
+}
+// The wide form: at most 8 warps, so that a thread holds up to 255 registers and
+// the fallback scan 32 chunks in flight without spills.  Always with aging (n =
+// 6500, m = 512, k = 32 3509 us an iteration in the narrow form, 3155 in this; n =
+// 2100 769 and 765).  Without aging only where scans are many: no second tier,
+// and short lists or long rows (k = 10: n = 2700 1167 and 1212, 3300 1601 and 1563;
+// k = 20: n = 3300 1403 and 1406, 5000 2337 and 2307; k = 32: n = 4096 1640 and
+// 1650, 6500 3171 and 3134); with a tier the narrow form's smaller loop wins (n =
+// 4096, k = 32 1556 and 1604).
+bool wide_cluster(const ColonyDev &c, int warps) {
+  return warps <= kWideClusterWarps &&
+         (c.aging || (c.t2 == 0 && c.n > (c.K <= 16 ? 3072 : 4096)));
+}
+template <bool AGING, int TW, int G>
+cudaError_t cluster_launch_w(const ColonyDev &c, int grid, int warps, int cs, cudaStream_t s,
+                             int *max_clusters) {
+  constexpr int W = kWideClusterWarps;
+  const bool wide = wide_cluster(c, warps);
+  if (max_clusters) {  // the query opens both forms
+    const cudaError_t e =
+        wide ? cluster_launch_t<AGING, TW, G, kStagedMaxWarps>(c, grid, warps, cs, s, max_clusters)
+             : cluster_launch_t<AGING, TW, G, W>(c, grid, 1, cs, s, max_clusters);
+    if (e != cudaSuccess) return e;
+  }
+  return wide ? cluster_launch_t<AGING, TW, G, W>(c, grid, warps, cs, s, max_clusters)
+              : cluster_launch_t<AGING, TW, G, kStagedMaxWarps>(c, grid, warps, cs, s,
+                                                                max_clusters);
 }
 template <bool AGING, int G>
 cudaError_t cluster_launch_tw(const ColonyDev &c, int grid, int warps, int cs, cudaStream_t s,
                               int *max_clusters) {
-  if (c.n <= 2048) return cluster_launch_t<AGING, 2, G>(c, grid, warps, cs, s, max_clusters);
-  if (c.n <= 4096) return cluster_launch_t<AGING, 4, G>(c, grid, warps, cs, s, max_clusters);
-  return cluster_launch_t<AGING, 8, G>(c, grid, warps, cs, s, max_clusters);
+  if (c.n <= 2048)
+    return cluster_launch_t<AGING, 2, G, kStagedMaxWarps>(c, grid, warps, cs, s, max_clusters);
+  if (c.n <= 4096) return cluster_launch_w<AGING, 4, G>(c, grid, warps, cs, s, max_clusters);
+  return cluster_launch_w<AGING, 8, G>(c, grid, warps, cs, s, max_clusters);
 }
 template <int G>
 cudaError_t cluster_launch_g(const ColonyDev &c, int grid, int warps, int cs, cudaStream_t s,

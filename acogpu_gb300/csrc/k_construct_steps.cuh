@@ -441,8 +441,10 @@ __device__ __forceinline__ float scan_level(float x, int o) {
 // many warps cover the loads and whose registers the buffers would cost: 37.2
 // ms of construction for 512 instances with it, 27 without): a group of chunks
 // is loaded ahead of the one being compared, four (n <= 2048; the whole row at
-// n = 1000 takes two groups) or eight (n = 4096: construction 1436 us with
-// four, 1374 with eight).  If the largest value is 0 the lowest unvisited city
+// n = 1000 takes two groups), eight (n = 4096: construction 1436 us with four,
+// 1374 with eight) or, AHEAD = 2, sixteen (n = 8000, k = 20, rank-based 4562 us an
+// iteration with eight, 4151 with sixteen); of a blending ant, whose chunks take
+// twice the registers, four, and above 2048 cities with AHEAD = 2 only.  If the largest value is 0 the lowest unvisited city
 // is the answer, from the tabu words alone, and a row with a NaN is scanned again
 // without it (fallback_rest).
 template <int TW>
@@ -535,10 +537,10 @@ __device__ __forceinline__ uint32_t blend_bits(const ColonyDev &c, uint32_t t, u
                                        c.use_alpha, c.alpha));
 }
 
-template <int TW, bool BL, bool AHEAD>
+template <int TW, bool BL, int AHEAD>
 __device__ __forceinline__ int fallback_scan(const ColonyDev &c, int cur, const TwPack<TW> &p,
                                              const AntCtx &a, int lane) {
-  constexpr int GR = TW > 2 && !BL && AHEAD ? 8 : 4;  // chunks a group
+  constexpr int GR = TW > 2 && !BL && AHEAD ? 8 * AHEAD : 4;  // chunks a group
   const size_t row = (size_t)cur * c.ld;
   unsigned best = 0u;
   int bt = 0;
@@ -642,14 +644,15 @@ __device__ __forceinline__ int fallback_tier2(const ColonyDev &c, int cur,
 
 // The whole best-choice fallback, as a called function (the tabu words by
 // value, so they stay in registers): its code stays out of the step loop.
-template <int TW, bool AHEAD>
+template <int TW, int AHEAD>
 __device__ __noinline__ int fallback_best(const ColonyDev &c, int cur, TwPack<TW> p, AntCtx a,
                                           int lane, int id, bool vis, bool tier_ok) {
   int next = -1;
   if (tier_ok && c.t2 > 0) next = fallback_tier2<TW>(c, cur, p, id, vis, lane);
   if (next < 0)
-    next = a.blend ? fallback_scan<TW, true, AHEAD>(c, cur, p, a, lane)
-                   : fallback_scan<TW, false, AHEAD>(c, cur, p, a, lane);
+    next = a.blend
+               ? fallback_scan<TW, true, TW <= 2 || AHEAD == 2 ? AHEAD : 0>(c, cur, p, a, lane)
+               : fallback_scan<TW, false, AHEAD>(c, cur, p, a, lane);
   return next;
 }
 
@@ -760,7 +763,7 @@ __device__ __noinline__ int exact_pick(float w, int id, float u, int lane) {
 // consecutive steps are computed one per lane and broadcast; the tour
 // positions of the current 32-step block stay in one register per lane and
 // are stored together.
-template <int TW, bool BLEND, int G, class ROWS, bool TIER, bool AHEAD>
+template <int TW, bool BLEND, int G, class ROWS, bool TIER, int AHEAD>
 __device__ __forceinline__ void staged_steps(const ColonyDev &c, int k, uint32_t akey, int start,
                                              StepTabu<TW> &tabu, const ROWS &rows, AntCtx a,
                                              int lane, int64_t &fallbacks) {
@@ -866,7 +869,7 @@ __device__ __forceinline__ void staged_steps(const ColonyDev &c, int k, uint32_t
 // the step loop (BLEND: the aging fitness blend of every candidate per step;
 // otherwise the weights come blended, or plain, from the table), then the
 // integer length and the transposed successor/predecessor lists.
-template <int TW, int G, bool BLEND, class ROWS, bool TIER = true, bool AHEAD = true>
+template <int TW, int G, bool BLEND, class ROWS, bool TIER = true, int AHEAD = 1>
 __device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, uint32_t *words,
                                 const ROWS &rows, AntCtx a, int lane) {
   const int n = c.n;
@@ -921,7 +924,7 @@ __device__ void staged_ant_body(const ColonyDev &c, int k, uint32_t iter, uint32
 // One ant with its aging step: updateAntAges (src/Colony.cu:353-364), the
 // cleared tour of an invalid ant (src/Colony.cu:507-510) and the blend
 // decision of compute_fittness (inc/Colony.cuh:21-30).
-template <bool AGING, int TW, int G, class ROWS, bool TIER = true, bool AHEAD = true>
+template <bool AGING, int TW, int G, class ROWS, bool TIER = true, int AHEAD = 1>
 __device__ void construct_ant_staged(const ColonyDev &c, int k, uint32_t iter, uint32_t *words,
                                      const ROWS &rows, int lane) {
   AntCtx a;

@@ -732,3 +732,51 @@ def test_weights_at_the_ends_of_the_range_match_oracle(n, k, mode, tau0, place):
         assert_same_state(g, q, ctx=f"tau0={tau0} {place} iteration {it}")
     g.close()
     q.close()
+
+
+@pytest.mark.parametrize("n,m,k,variant,iters", [(2049, 24, 8, _abi.ACO_ANT_SYSTEM, 14),
+                                                 (4097, 24, 10, _abi.ACO_ANT_SYSTEM, 14),
+                                                 (2300, 1300, 6, _abi.ACO_RANK_BASED, 11)])
+def test_cluster_forms_with_blending_ants_match_oracle(n, m, k, variant, iters):
+    """Aging on the cluster kernel's wide form (few ants a CTA) and narrow one
+    (more than 8), through convergence, with few candidates so that blending
+    ants fall back to scans of the row."""
+    x, y, d = instance(n, 40 + n)
+    p = params(num_ants=m, variant=variant, rank_w=4, beta=2.0, rho=0.2, cand_k=k, aging=1, seed=n,
+               **FAST_MODE)
+    (p.min_retirement_age, p.max_retirement_age, p.local_performance, p.global_performance,
+     p.min_population_limit, p.max_population_limit) = (5, 7, 10, 1, 5, 100)
+    p.construct_mode = _abi.ACO_CONSTRUCT_CLUSTER
+    g = aco.Colony(d, params=p, num_ants=m)
+    g.initialize()
+    p.construct_mode = _abi.ACO_CONSTRUCT_AUTO
+    q = oracle.Port(p, d, threads=16)
+    q.initialize()
+    blended = False
+    for it in range(iters):
+        g.constructSolution()
+        q.iterate()
+        a = q.aging()
+        blended = blended or (a["isconverged"] and bool(((a["age"] < 5) & (a["valid"] > 0)).any()))
+        assert_same_state(g, q, aging=True, ctx=f"n={n} iteration {it}")
+    assert blended
+    g.close()
+    q.close()
+
+
+@pytest.mark.parametrize("n,k", [(3072, 16), (3073, 16), (3073, 17), (4096, 17), (4097, 17)])
+def test_cluster_forms_change_over_matches_oracle(n, k):
+    """The rank-based system without aging around the line between the forms."""
+    x, y, d = instance(n, 45 + n)
+    p = params(num_ants=10, variant=_abi.ACO_RANK_BASED, rank_w=4, beta=2.0, rho=0.2, cand_k=k,
+               seed=n + k, **FAST_MODE)
+    g = aco.Colony(d, params=p, num_ants=10)
+    g.initialize()
+    q = oracle.Port(p, d, threads=16)
+    q.initialize()
+    for it in range(2):
+        g.constructSolution()
+        q.iterate()
+        assert_same_state(g, q, ctx=f"n={n} k={k} iteration {it}")
+    g.close()
+    q.close()
