@@ -444,9 +444,9 @@ __device__ __forceinline__ float scan_level(float x, int o) {
 // n = 1000 takes two groups), eight (n = 4096: construction 1436 us with four,
 // 1374 with eight) or, AHEAD = 2, sixteen (n = 8000, k = 20, rank-based 4562 us an
 // iteration with eight, 4151 with sixteen); of a blending ant, whose chunks take
-// twice the registers, four, and above 2048 cities with AHEAD = 2 only.  If the largest value is 0 the lowest unvisited city
-// is the answer, from the tabu words alone, and a row with a NaN is scanned again
-// without it (fallback_rest).
+// twice the registers, four, and above 2048 cities with AHEAD = 2 only.  If the
+// largest value is 0 the lowest unvisited city is the answer, from the tabu words
+// alone, and a row with a NaN is scanned again without it (fallback_rest).
 template <int TW>
 struct TwPack {
   uint32_t w[TW];
